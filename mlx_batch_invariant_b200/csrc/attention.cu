@@ -25,15 +25,38 @@
 // (m' equals m or s) and exp(0) is exactly 1, so one evaluation of
 // exp(-|s - m|) yields both factors with unchanged bits.
 //
-// decode_kernel and prefill_kernel call the same key_update() and merge
-// functions (merge_coeffs / merge_acc for the split fold), which is why a token's bits do not depend on which of the two
-// produced it.
+// The prefill kernel (attn_prefill.cu) performs the same sequence per query, with the same merge functions, which is
+// why a token's bits do not depend on which of the two produced it.
 #include <algorithm>
-#include "bi_common.cuh"
-#include "bi_ptx.cuh"
+#include "attn_common.cuh"
 #include "peer_push.cuh"
 
 namespace bi {
+
+int check_attention(const char* op, const void* q, const void* k, const void* v, const void* out, int64_t B, int64_t Hq,
+                    int64_t Hkv, int64_t Tq, int64_t L, int64_t D, const KvLayout& lay, int split, int dtype) {
+    if (!dtype_ok(dtype)) return fail(BI_ERR_UNSUPPORTED, "%s: dtype %d", op, dtype);
+    if (B < 0 || Hq <= 0 || Hkv <= 0 || Tq <= 0 || L <= 0 || D <= 0 || split <= 0)
+        return fail(BI_ERR_BAD_ARG, "%s: bad sizes B=%lld Hq=%lld Hkv=%lld Tq=%lld L=%lld D=%lld split=%d", op,
+                    (long long)B, (long long)Hq, (long long)Hkv, (long long)Tq, (long long)L, (long long)D, split);
+    if (Hq % Hkv != 0) return fail(BI_ERR_UNSUPPORTED, "%s: Hq=%lld not a multiple of Hkv=%lld", op, (long long)Hq, (long long)Hkv);
+    if (D != 32 && D != 64 && D != 128 && D != 256)
+        return fail(BI_ERR_UNSUPPORTED, "%s: head_dim %lld (supported: 32, 64, 128, 256)", op, (long long)D);
+    if (B == 0) return BI_OK;
+    if (!q || !k || !v || !out) return fail(BI_ERR_BAD_ARG, "%s: null pointer", op);
+    const size_t cb = (size_t)(D / 32) * dtype_size(dtype);  // bytes of one chunk load
+    const size_t al = cb > 16 ? 16 : cb;
+    if (!aligned(q, al) || !aligned(k, al) || !aligned(v, al) || !aligned(out, al))
+        return fail(BI_ERR_MISALIGNED, "%s: pointers must be %zu-byte aligned", op, al);
+    const int64_t se = (int64_t)(al / dtype_size(dtype));
+    if (se > 1 && (lay.sb % se || lay.sh % se || lay.sl % se))
+        return fail(BI_ERR_MISALIGNED, "%s: k/v strides must be multiples of %lld elements", op, (long long)se);
+    if (lay.sl < D) return fail(BI_ERR_BAD_ARG, "%s: key stride %lld < head_dim", op, (long long)lay.sl);
+    if (L > (1 << 30) || B * Hq * Tq > (1LL << 40))
+        return fail(BI_ERR_UNSUPPORTED, "%s: problem too large", op);
+    return BI_OK;
+}
+
 namespace {
 
 constexpr int OCT = 8;        // real lanes per key stream
@@ -91,27 +114,6 @@ __device__ __forceinline__ void key_update(const float (&kf)[NCHUNK * DL], const
         }
     }
 }
-
-// Fold one split's (m, l) into the running (M, L) and return the two factors
-// the accumulators are folded with:  A_d = fma(A_d, c_old, acc_d * c_new).
-__device__ __forceinline__ void merge_coeffs(float& M, float& L, float m, float l, float& c_old, float& c_new) {
-    const float M_new = fmaxf(M, m);
-    c_old = expf_canon(sub_rn(M, M_new));
-    c_new = expf_canon(sub_rn(m, M_new));
-    L = fma_rn(L, c_old, mul_rn(l, c_new));
-    M = M_new;
-}
-__device__ __forceinline__ float merge_acc(float A, float c_old, float acc, float c_new) {
-    return fma_rn(A, c_old, mul_rn(acc, c_new));
-}
-
-struct KvLayout {
-    int64_t sb, sh, sl;  // element strides of k and v: batch (or page, when paged), kv head, key
-    // Paged cache (table != nullptr): k and v are pools of pages [page, kv head, key in page, D]; keys
-    // [i * page_size, (i + 1) * page_size) of sequence b live in page table[b * table_stride + i].
-    const int32_t* table;
-    int page_size, table_stride;
-};
 
 // ---- decode: unit = (batch, kv head, chunk of GU query heads, split) ----------
 template <typename T, int DL, int GU>
@@ -228,14 +230,6 @@ template <typename T, int DL> struct Dec2Cfg {
     static constexpr int WARP_BYTES = DEC2_STAGES * STAGE_BYTES;
     static constexpr int SMEM_BYTES = DEC2_WARPS * WARP_BYTES;
 };
-
-// two T values (consecutive dims) packed in one 32-bit word -> fp32, for 16-bit T
-template <typename T> __device__ __forceinline__ float word_lo(uint32_t w);
-template <typename T> __device__ __forceinline__ float word_hi(uint32_t w);
-template <> __device__ __forceinline__ float word_lo<__nv_bfloat16>(uint32_t w) { return __uint_as_float(w << 16); }
-template <> __device__ __forceinline__ float word_hi<__nv_bfloat16>(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
-template <> __device__ __forceinline__ float word_lo<__half>(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w & 0xFFFFu))); }
-template <> __device__ __forceinline__ float word_hi<__half>(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
 
 // Slice of a row owned by real lane r, as packed pairs: dst[jp][d] = (x[(r + 16 jp) * DL + d], x[(r + 8 + 16 jp) * DL + d])
 template <typename T, int DL>
@@ -888,160 +882,6 @@ int launch_decode_combine(const float* pm, const float* pl, const float* pacc, c
     return check_launch("bi_attn_decode combine");
 }
 
-// ---- prefill: unit = (batch, head, block of QB consecutive queries) -----------
-// QB queries share each K/V row (4, or 2 for the widest heads to stay in registers); which
-// queries are grouped is a launch choice, a query's arithmetic is the same in any group.
-// The running merge state (M, L, A) is touched once per split, so it lives in shared
-// memory, one private slot per thread, and the registers hold the per-key state.
-constexpr int PREFILL_THREADS = 128;
-template <int DL> struct PrefillCfg { static constexpr int QB = DL >= 8 ? 2 : 4; };
-
-template <typename T, int DL>
-__global__ void __launch_bounds__(PREFILL_THREADS) prefill_kernel(const T* __restrict__ q, const T* __restrict__ k,
-                                                      const T* __restrict__ v, T* __restrict__ out, int B, int Hq,
-                                                      int Hkv, int Tq, int L, KvLayout lay, float scale, int causal,
-                                                      int split) {
-    ptx::grid_dep_launch();   // the next kernel of the stream may start its set-up
-    ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
-    constexpr int D = 32 * DL;
-    constexpr int NL = NCHUNK * DL;
-    constexpr int QB = PrefillCfg<DL>::QB;
-    extern __shared__ float merge_state[];  // [(QB * (NL + 2))][PREFILL_THREADS]
-    const int lane = threadIdx.x & 31;
-    const int r = lane & (OCT - 1);
-    const int nblk = (Tq + QB - 1) / QB;
-    const long long units = (long long)B * Hq * nblk;
-    const long long oct = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * OCT_PER_WARP + (lane >> 3);
-    const bool unit_ok = oct < units;
-    long long u = unit_ok ? oct : 0;
-    const int blk = (int)(u % nblk); u /= nblk;
-    const int h = (int)(u % Hq); u /= Hq;
-    const int b = (int)u;
-    const int hk = h / (Hq / Hkv);
-    const int q0 = blk * QB;
-
-    const T* kb = k + (int64_t)b * lay.sb + (int64_t)hk * lay.sh;
-    const T* vb = v + (int64_t)b * lay.sb + (int64_t)hk * lay.sh;
-
-    int nkeys[QB];
-    float qf[QB][NL];
-    int nkeys_max = 0;
-#pragma unroll
-    for (int iq = 0; iq < QB; ++iq) {
-        const int qi = min(q0 + iq, Tq - 1);
-        nkeys[iq] = (unit_ok && q0 + iq < Tq) ? (causal ? (L - Tq + qi + 1) : L) : 0;
-        nkeys_max = max(nkeys_max, nkeys[iq]);
-        const T* qr = q + (((int64_t)b * Hq + h) * Tq + qi) * D;
-        load_slice<T, DL>(qr, r, qf[iq]);
-#pragma unroll
-        for (int d = 0; d < NL; ++d) qf[iq][d] = mul_rn(qf[iq][d], scale);
-    }
-    int warp_max = nkeys_max;
-    warp_max = max(warp_max, __shfl_xor_sync(0xffffffffu, warp_max, 8));
-    warp_max = max(warp_max, __shfl_xor_sync(0xffffffffu, warp_max, 16));
-    const int nsplit = (warp_max + split - 1) / split;
-
-    float* const slot = merge_state + threadIdx.x;  // element e of this thread: slot[e * PREFILL_THREADS]
-    constexpr int STRIDE = PREFILL_THREADS;
-    float m[QB], l[QB], acc[QB][NL];
-#pragma unroll
-    for (int iq = 0; iq < QB; ++iq) {
-        slot[(iq * (NL + 2) + 0) * STRIDE] = -INFINITY;
-        slot[(iq * (NL + 2) + 1) * STRIDE] = 0.0f;
-#pragma unroll
-        for (int d = 0; d < NL; ++d) slot[(iq * (NL + 2) + 2 + d) * STRIDE] = 0.0f;
-    }
-
-    for (int sp = 0; sp < nsplit; ++sp) {
-#pragma unroll
-        for (int iq = 0; iq < QB; ++iq) {
-            m[iq] = -INFINITY; l[iq] = 0.0f;
-#pragma unroll
-            for (int d = 0; d < NL; ++d) acc[iq][d] = 0.0f;
-        }
-        const int j0 = sp * split;
-        const int j1 = min(warp_max, j0 + split);
-        constexpr bool PF = DL < 4;  // wider heads have no registers left for a look-ahead row
-        float kf[NL], vf[NL];
-        if (PF) {
-            load_slice<T, DL>(kb + (int64_t)j0 * lay.sl, r, kf);
-            load_slice<T, DL>(vb + (int64_t)j0 * lay.sl, r, vf);
-        }
-        for (int j = j0; j < j1; ++j) {
-            bool act[QB];
-#pragma unroll
-            for (int iq = 0; iq < QB; ++iq) act[iq] = j < nkeys[iq];
-            if (PF) {
-                float kn[NL], vn[NL];
-                const int jn = (j + 1 < j1) ? j + 1 : j0;
-                load_slice<T, DL>(kb + (int64_t)jn * lay.sl, r, kn);
-                load_slice<T, DL>(vb + (int64_t)jn * lay.sl, r, vn);
-                key_update<QB, DL>(kf, vf, qf, m, l, acc, act);
-#pragma unroll
-                for (int d = 0; d < NL; ++d) { kf[d] = kn[d]; vf[d] = vn[d]; }
-            } else {
-                load_slice<T, DL>(kb + (int64_t)j * lay.sl, r, kf);
-                load_slice<T, DL>(vb + (int64_t)j * lay.sl, r, vf);
-                key_update<QB, DL>(kf, vf, qf, m, l, acc, act);
-            }
-        }
-#pragma unroll
-        for (int iq = 0; iq < QB; ++iq) {
-            if (j0 < nkeys[iq]) {
-                float* st = slot + (iq * (NL + 2)) * STRIDE;
-                float Mq = st[0], Lq = st[STRIDE], c_old, c_new;
-                merge_coeffs(Mq, Lq, m[iq], l[iq], c_old, c_new);
-                st[0] = Mq; st[STRIDE] = Lq;
-#pragma unroll
-                for (int d = 0; d < NL; ++d)
-                    st[(2 + d) * STRIDE] = merge_acc(st[(2 + d) * STRIDE], c_old, acc[iq][d], c_new);
-            }
-        }
-    }
-
-#pragma unroll
-    for (int iq = 0; iq < QB; ++iq) {
-        if (unit_ok && q0 + iq < Tq) {
-            T* o = out + (((int64_t)b * Hq + h) * Tq + q0 + iq) * D;
-            using C = Chunk<T, DL>;
-            const float* st = slot + (iq * (NL + 2)) * STRIDE;
-            const float Lq = st[STRIDE];
-#pragma unroll
-            for (int j = 0; j < NCHUNK; ++j) {
-                C c;
-#pragma unroll
-                for (int d = 0; d < DL; ++d) c.v[d] = Cvt<T>::down(div_canon(st[(2 + j * DL + d) * STRIDE], Lq));
-                reinterpret_cast<C*>(o)[r + OCT * j] = c;
-            }
-        }
-    }
-}
-
-int check_common(const char* op, const void* q, const void* k, const void* v, const void* out, int64_t B,
-                 int64_t Hq, int64_t Hkv, int64_t Tq, int64_t L, int64_t D, const KvLayout& lay, int split,
-                 int dtype) {
-    if (!dtype_ok(dtype)) return fail(BI_ERR_UNSUPPORTED, "%s: dtype %d", op, dtype);
-    if (B < 0 || Hq <= 0 || Hkv <= 0 || Tq <= 0 || L <= 0 || D <= 0 || split <= 0)
-        return fail(BI_ERR_BAD_ARG, "%s: bad sizes B=%lld Hq=%lld Hkv=%lld Tq=%lld L=%lld D=%lld split=%d", op,
-                    (long long)B, (long long)Hq, (long long)Hkv, (long long)Tq, (long long)L, (long long)D, split);
-    if (Hq % Hkv != 0) return fail(BI_ERR_UNSUPPORTED, "%s: Hq=%lld not a multiple of Hkv=%lld", op, (long long)Hq, (long long)Hkv);
-    if (D != 32 && D != 64 && D != 128 && D != 256)
-        return fail(BI_ERR_UNSUPPORTED, "%s: head_dim %lld (supported: 32, 64, 128, 256)", op, (long long)D);
-    if (B == 0) return BI_OK;
-    if (!q || !k || !v || !out) return fail(BI_ERR_BAD_ARG, "%s: null pointer", op);
-    const size_t cb = (size_t)(D / 32) * dtype_size(dtype);  // bytes of one chunk load
-    const size_t al = cb > 16 ? 16 : cb;
-    if (!aligned(q, al) || !aligned(k, al) || !aligned(v, al) || !aligned(out, al))
-        return fail(BI_ERR_MISALIGNED, "%s: pointers must be %zu-byte aligned", op, al);
-    const int64_t se = (int64_t)(al / dtype_size(dtype));
-    if (se > 1 && (lay.sb % se || lay.sh % se || lay.sl % se))
-        return fail(BI_ERR_MISALIGNED, "%s: k/v strides must be multiples of %lld elements", op, (long long)se);
-    if (lay.sl < D) return fail(BI_ERR_BAD_ARG, "%s: key stride %lld < head_dim", op, (long long)lay.sl);
-    if (L > (1 << 30) || B * Hq * Tq > (1LL << 40))
-        return fail(BI_ERR_UNSUPPORTED, "%s: problem too large", op);
-    return BI_OK;
-}
-
 template <typename T, int DL>
 int launch_decode(const void* q, const void* k, const void* v, void* out, const int32_t* kv_lens, float* ws,
                   int64_t B, int64_t Hq, int64_t Hkv, int64_t L, const KvLayout& lay, float scale, int split,
@@ -1200,50 +1040,8 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
     return launch_decode_combine<T>(pm, pl, pacc, kv_lens, out, BH, (int)Hq, D, (int)L, split, nsplit, sink, st);
 }
 
-template <typename T, int DL>
-int launch_prefill(const void* q, const void* k, const void* v, void* out, int64_t B, int64_t Hq, int64_t Hkv,
-                   int64_t Tq, int64_t L, const KvLayout& lay, float scale, int causal, int split, cudaStream_t st) {
-    constexpr int QB = PrefillCfg<DL>::QB;
-    const int64_t nblk = (Tq + QB - 1) / QB;
-    const int64_t units = B * Hq * nblk;
-    constexpr int warps = PREFILL_THREADS / 32;
-    const int64_t blocks = (units + warps * OCT_PER_WARP - 1) / (warps * OCT_PER_WARP);
-    if (blocks > 0x7fffffffLL) return fail(BI_ERR_UNSUPPORTED, "bi_attn_prefill: grid too large");
-    const size_t smem = (size_t)QB * (NCHUNK * DL + 2) * PREFILL_THREADS * sizeof(float);
-    auto kern = prefill_kernel<T, DL>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail(BI_ERR_CUDA, "bi_attn_prefill smem attr: %s", cudaGetErrorString(e));
-    }
-    kern<<<(unsigned)blocks, PREFILL_THREADS, smem, st>>>(
-        static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), static_cast<T*>(out), (int)B,
-        (int)Hq, (int)Hkv, (int)Tq, (int)L, lay, scale, causal, split);
-    return check_launch("bi_attn_prefill");
-}
-
 }  // namespace
 }  // namespace bi
-
-#define BI_DISPATCH_T_DL(FN, ...)                                                        \
-    do {                                                                                 \
-        const int dl_ = (int)(D / 32);                                                   \
-        if (dtype == BI_F32) {                                                           \
-            if (dl_ == 1) return FN<float, 1>(__VA_ARGS__);                              \
-            if (dl_ == 2) return FN<float, 2>(__VA_ARGS__);                              \
-            if (dl_ == 4) return FN<float, 4>(__VA_ARGS__);                              \
-            return FN<float, 8>(__VA_ARGS__);                                            \
-        } else if (dtype == BI_F16) {                                                    \
-            if (dl_ == 1) return FN<__half, 1>(__VA_ARGS__);                             \
-            if (dl_ == 2) return FN<__half, 2>(__VA_ARGS__);                             \
-            if (dl_ == 4) return FN<__half, 4>(__VA_ARGS__);                             \
-            return FN<__half, 8>(__VA_ARGS__);                                           \
-        } else {                                                                         \
-            if (dl_ == 1) return FN<__nv_bfloat16, 1>(__VA_ARGS__);                      \
-            if (dl_ == 2) return FN<__nv_bfloat16, 2>(__VA_ARGS__);                      \
-            if (dl_ == 4) return FN<__nv_bfloat16, 4>(__VA_ARGS__);                      \
-            return FN<__nv_bfloat16, 8>(__VA_ARGS__);                                    \
-        }                                                                                \
-    } while (0)
 
 extern "C" size_t bi_attn_decode_workspace_bytes(int64_t B, int64_t Hq, int64_t L, int64_t D, int split_size) {
     if (B <= 0 || Hq <= 0 || L <= 0 || D <= 0 || split_size <= 0) return 0;
@@ -1257,7 +1055,7 @@ extern "C" int bi_attn_decode(const void* q, const void* k, const void* v, void*
                               int dtype, void* stream) {
     using namespace bi;
     KvLayout lay{kv_sb, kv_sh, kv_sl};
-    int rc = check_common("bi_attn_decode", q, k, v, out, B, Hq, Hkv, 1, L, D, lay, split_size, dtype);
+    int rc = check_attention("bi_attn_decode", q, k, v, out, B, Hq, Hkv, 1, L, D, lay, split_size, dtype);
     if (rc || B == 0) return rc;
     const size_t need = bi_attn_decode_workspace_bytes(B, Hq, L, D, split_size);
     if (!workspace || workspace_bytes < need)
@@ -1280,7 +1078,7 @@ extern "C" int bi_attn_decode_push(const void* q, const void* k, const void* v, 
     PushSink sink;
     int rc = make_sink("bi_attn_decode_push", dst, peer_flags, counters, rank, world, wait, status, dtype_ok(dtype) ? dtype_size(dtype) : 1, &sink);
     if (rc) return rc;
-    rc = check_common("bi_attn_decode_push", q, k, v, dst[rank], B, Hq, Hkv, 1, L, D, lay, split_size, dtype);
+    rc = check_attention("bi_attn_decode_push", q, k, v, dst[rank], B, Hq, Hkv, 1, L, D, lay, split_size, dtype);
     if (rc || B == 0) return rc;
     const size_t need = bi_attn_decode_workspace_bytes(B, Hq, L, D, split_size);
     if (!workspace || workspace_bytes < need)
@@ -1291,18 +1089,6 @@ extern "C" int bi_attn_decode_push(const void* q, const void* k, const void* v, 
     const PushSink* sp = &sink;
     void* out = nullptr;
     BI_DISPATCH_T_DL(launch_decode, q, k, v, out, kv_lens, ws, B, Hq, Hkv, L, lay, scale, split_size, st, sp);
-}
-
-extern "C" int bi_attn_prefill(const void* q, const void* k, const void* v, void* out, int64_t B, int64_t Hq,
-                               int64_t Hkv, int64_t Tq, int64_t L, int64_t D, int64_t kv_sb, int64_t kv_sh,
-                               int64_t kv_sl, float scale, int causal, int split_size, int dtype, void* stream) {
-    using namespace bi;
-    KvLayout lay{kv_sb, kv_sh, kv_sl};
-    int rc = check_common("bi_attn_prefill", q, k, v, out, B, Hq, Hkv, Tq, L, D, lay, split_size, dtype);
-    if (rc || B == 0) return rc;
-    if (causal && Tq > L) return fail(BI_ERR_BAD_ARG, "bi_attn_prefill: causal needs Tq <= L (Tq=%lld L=%lld)", (long long)Tq, (long long)L);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    BI_DISPATCH_T_DL(launch_prefill, q, k, v, out, B, Hq, Hkv, Tq, L, lay, scale, causal, split_size, st);
 }
 
 extern "C" int bi_attn_decode_paged(const void* q, const void* k_pages, const void* v_pages, void* out, const int32_t* kv_lens,
@@ -1318,7 +1104,7 @@ extern "C" int bi_attn_decode_paged(const void* q, const void* k_pages, const vo
     if (dtype == BI_F32 || D != 128) return fail(BI_ERR_UNSUPPORTED, "bi_attn_decode_paged: 16-bit caches with head_dim 128 only");
     const int64_t L = max_pages * page_size;
     KvLayout lay{pg_sp, pg_sh, pg_sl, block_table, (int)page_size, (int)table_stride};
-    int rc = check_common("bi_attn_decode_paged", q, k_pages, v_pages, out, B, Hq, Hkv, 1, L, D, lay, split_size, dtype);
+    int rc = check_attention("bi_attn_decode_paged", q, k_pages, v_pages, out, B, Hq, Hkv, 1, L, D, lay, split_size, dtype);
     if (rc || B == 0) return rc;
     const size_t need = bi_attn_decode_workspace_bytes(B, Hq, L, D, split_size);
     if (!workspace || workspace_bytes < need)

@@ -105,6 +105,10 @@ enum { BI_MATMUL_AUTO = 0, BI_MATMUL_SPLIT = 1, BI_MATMUL_FUSED = 2, BI_MATMUL_S
 #define BI_MATMUL_COUNTER_BYTES 16384
 
 size_t bi_matmul_workspace_bytes(int64_t M, int64_t N, int64_t K, int dtype);
+/* The workspace with which BI_MATMUL_AUTO has every launch shape to choose from (at least
+ * bi_matmul_workspace_bytes; more for fp32 batches that are faster split over their K groups). Optional: with
+ * less, AUTO folds in place. Same bits either way. */
+size_t bi_matmul_scratch_bytes(int64_t M, int64_t N, int64_t K, int dtype);
 
 int bi_matmul(const void* a, const void* b, void* out, void* workspace, size_t workspace_bytes,
               int64_t M, int64_t N, int64_t K, int64_t a_sm, int64_t a_sk, int64_t b_sk,

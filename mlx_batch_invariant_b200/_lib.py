@@ -38,6 +38,7 @@ SIGNATURES = {
     "bi_rms_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_float, c_int, c_void_p]),
     "bi_layer_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_float, c_int, c_void_p]),
     "bi_matmul_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int]),
+    "bi_matmul_scratch_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int]),
     "bi_matmul": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_int64, c_int64, c_int64, c_int64,
                           c_int64, c_int64, c_int64, c_int, c_int, c_void_p, c_void_p]),
     "bi_matmul_bias": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_int64, c_int64, c_int64, c_int64,

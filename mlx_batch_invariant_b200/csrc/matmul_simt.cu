@@ -21,16 +21,6 @@
 namespace bi {
 namespace {
 
-constexpr int BN = 64;
-constexpr int BK = 16;
-constexpr int THREADS = 256;
-
-// Affine dequantization of one code: fma in fp32, then one rounding to the staged type T.
-template <typename T>
-__device__ __forceinline__ float dequant_code(uint32_t code, float s, float b) {
-    return Cvt<T>::up(Cvt<T>::down(fma_rn((float)code, s, b)));
-}
-
 struct QuantArgs {
     const uint32_t* w;   // [N, K*bits/32]
     const void* scales;  // [N, K/gs]
@@ -39,98 +29,228 @@ struct QuantArgs {
     const void* out_bias;  // optional [N] bias of the linear layer (dense and quantized alike), in T
 };
 
-// TM rows x 4 columns per thread; tile = (16*TM) x 64.
-template <typename T, int TM, bool SPLIT, bool QUANT>
-__global__ void __launch_bounds__(THREADS) simt_matmul_kernel(const T* __restrict__ a, const T* __restrict__ b,
-                                                              QuantArgs qa, void* __restrict__ outp, int M, int N,
-                                                              int K, int64_t a_sm, int64_t a_sk, int64_t b_sk,
-                                                              int64_t b_sn) {
+// Affine dequantization of one code: fma in fp32, then one rounding to the staged type T.
+template <typename T>
+__device__ __forceinline__ float dequant_code(uint32_t code, float s, float b) {
+    return Cvt<T>::up(Cvt<T>::down(fma_rn((float)code, s, b)));
+}
+
+// V consecutive floats of shared memory (V = 1, 2, 4, aligned to their size).
+template <int V> __device__ __forceinline__ void ld_floats(const float* p, float* v) {
+    if constexpr (V == 4) { const float4 w = *reinterpret_cast<const float4*>(p); v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w; }
+    else if constexpr (V == 2) { const float2 w = *reinterpret_cast<const float2*>(p); v[0] = w.x; v[1] = w.y; }
+    else v[0] = *p;
+}
+
+// A thread's W rows (or columns) of an operand tile lie in runs of four (the last may be shorter), each run one stripe of
+// `lanes` such runs after the one before. place(): tile row of element u of thread idx; ld_tile(): all of them at one k.
+template <int W> __host__ __device__ constexpr int run_len(int r) { return W - 4 * r < 4 ? W - 4 * r : 4; }
+template <int W> __device__ __forceinline__ int place(int idx, int u, int lanes) {
+    return lanes * 4 * (u / 4) + idx * run_len<W>(u / 4) + u % 4;
+}
+template <int W, int R = 0> __device__ __forceinline__ void ld_tile(const float* row, int idx, int lanes, int sw, float* v) {
+    if constexpr (4 * R < W) {
+        ld_floats<run_len<W>(R)>(row + ((lanes * 4 * R + idx * run_len<W>(R)) ^ sw), v + 4 * R);
+        ld_tile<W, R + 1>(row, idx, lanes, sw, v);
+    }
+}
+
+// A CTA owns BM x BN outputs (BM = MG * TM, BN = NL * TN); thread (mg, nl) holds a TM x TN tile of them. Operand tiles lie
+// k-major in shared memory ([k][row]): the TN values of a k are read as consecutive registers, so that the accumulators and
+// the operand of every fma can sit in different register banks (k-contiguous tiles, read four k at a time, ran at 60 % of
+// the fp32 pipe with the issue slots lost to operand conflicts). A stage is fetched into registers while the one before is
+// multiplied and then stored transposed; the row index is swizzled with k / 4 so that a warp's stores meet no bank conflict
+// and groups of four rows stay together. k runs in order inside every accumulator; past the end of the operands the
+// stages hold zeros (fma(0, 0, acc) leaves acc). Bound by the fp32 pipe from about 16 rows on, below by the stream of weights.
+// VEC: fp32 operands with k contiguous and 16-byte aligned rows, fetched as float4. Otherwise element by element (16-bit
+// operands, any strides, packed codes).
+template <typename T, int TM, int TN, int MG, int NL, bool SPLIT, bool QUANT, bool VEC>
+__global__ void __launch_bounds__(MG * NL, (SPLIT ? (TM * TN > 64 ? 256 : (MG * NL == 64 && TM * TN == 64 ? 320 : 512)) : 256) / (MG * NL))
+simt_matmul_kernel(const T* __restrict__ a, const T* __restrict__ b, QuantArgs qa, void* __restrict__ outp, int M, int N, int K,
+                   int64_t a_sm, int64_t a_sk, int64_t b_sk, int64_t b_sn) {
     ptx::grid_dep_launch();   // the next kernel of the stream may start its set-up
     ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
-    constexpr int BM = 16 * TM;
-    __shared__ float As[BK][BM];
-    __shared__ float Bs[BK][BN];
+    constexpr int BM = MG * TM, BN = NL * TN, THREADS = MG * NL;
+    constexpr int SLAB = 16, SWZ = 3;                                       // k per stage; row ^= (k / 4) << SWZ
+    constexpr int PA = (BM + 31) / 32 * 32, PB = (BN + 31) / 32 * 32;       // row pitches of the k-major tiles
+    __shared__ __align__(16) float As[2][SLAB][PA];
+    __shared__ __align__(16) float Bs[2][SLAB][PB];
     const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
+    const int nl = tid % NL, mg = tid / NL;
     const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
-    const int ngroups = (K + GROUP_K - 1) / GROUP_K;
     const int g0 = SPLIT ? (int)blockIdx.z : 0;
-    const int g1 = SPLIT ? g0 + 1 : ngroups;
+    const int kbeg = g0 * GROUP_K, kend = SPLIT ? min(K, kbeg + GROUP_K) : K;
+    const int nslab = (kend - kbeg + SLAB - 1) / SLAB;
+    constexpr int SEGS = SLAB / 4;                                          // float4 pieces of a row
+    constexpr int STEP = THREADS / SEGS;                                    // rows between a thread's pieces
+    constexpr int FA = (BM + STEP - 1) / STEP, FB = (BN + STEP - 1) / STEP; // pieces a thread fetches of either operand
 
-    float total[TM][4];
+    // The thread's first piece is row `pr`, k offset 4 * `seg`; the others are STEP rows apart.
+    const int pr = tid / SEGS, seg = tid % SEGS;
+    float4 fa[FA], fb[FB];
+    auto element = [&](bool isa, int i, int k) -> float {
+        if (isa) return Cvt<T>::up(a[(int64_t)i * a_sm + (int64_t)k * a_sk]);
+        if (QUANT) {
+            const int per_word = 32 / qa.bits;
+            const uint32_t word = qa.w[(int64_t)i * (K / per_word) + k / per_word];
+            const uint32_t code = (word >> ((k % per_word) * qa.bits)) & ((1u << qa.bits) - 1u);
+            const int64_t gi = (int64_t)i * (K / qa.gs) + k / qa.gs;
+            return dequant_code<T>(code, Cvt<T>::up(static_cast<const T*>(qa.scales)[gi]), Cvt<T>::up(static_cast<const T*>(qa.biases)[gi]));
+        }
+        return Cvt<T>::up(b[(int64_t)k * b_sk + (int64_t)i * b_sn]);
+    };
+    auto piece = [&](bool isa, int row, int tile_rows, int first, int limit, const T* base, int64_t stride, int k) -> float4 {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (row < tile_rows && first + row < limit && k < kend) {
+            if constexpr (VEC) v = __ldg(reinterpret_cast<const float4*>(base + (int64_t)(first + row) * stride + k));
+            else {
+                v.x = element(isa, first + row, k);
+                if (k + 1 < kend) v.y = element(isa, first + row, k + 1);
+                if (k + 2 < kend) v.z = element(isa, first + row, k + 2);
+                if (k + 3 < kend) v.w = element(isa, first + row, k + 3);
+            }
+        }
+        return v;
+    };
+    auto fetch = [&](int s) {
+        const int k = s < nslab ? kbeg + s * SLAB + seg * 4 : kend;
+#pragma unroll
+        for (int f = 0; f < FA; ++f) fa[f] = piece(true, pr + f * STEP, BM, m0, M, a, a_sm, k);
+#pragma unroll
+        for (int f = 0; f < FB; ++f) fb[f] = piece(false, pr + f * STEP, BN, n0, N, b, b_sn, k);
+    };
+    auto store = [&](int buf) {
+        auto put = [&](float* d, int pitch, const float4& v) { d[0] = v.x; d[pitch] = v.y; d[2 * pitch] = v.z; d[3 * pitch] = v.w; };
+#pragma unroll
+        for (int f = 0; f < FA; ++f)
+            if (BM % STEP == 0 || pr + f * STEP < BM) put(&As[buf][seg * 4][(pr + f * STEP) ^ (seg << SWZ)], PA, fa[f]);
+#pragma unroll
+        for (int f = 0; f < FB; ++f)
+            if (BN % STEP == 0 || pr + f * STEP < BN) put(&Bs[buf][seg * 4][(pr + f * STEP) ^ (seg << SWZ)], PB, fb[f]);
+    };
+
+    // Accumulators as pairs of columns (two independent fma per instruction; a's value rides in both halves).
+    constexpr int TP = TN / 2;
+    uint64_t acc[TM][TP], total[SPLIT ? 1 : TM][SPLIT ? 1 : TP];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) total[i][j] = 0.0f;
+        for (int j = 0; j < TP; ++j) {
+            acc[i][j] = 0;
+            if constexpr (!SPLIT) total[i][j] = 0;
+        }
 
-    for (int g = g0; g < g1; ++g) {
-        float acc[TM][4];
+    fetch(0);
+    for (int s = 0; s < nslab; ++s) {
+        const int buf = s & 1;
+        store(buf);
+        __syncthreads();                                            // slab s visible; slab s - 1 was read before the barrier of s
+        fetch(s + 1);
 #pragma unroll
-        for (int i = 0; i < TM; ++i)
+        for (int k = 0; k < SLAB; ++k) {
+            const int sw = (k >> 2) << SWZ;
+            float av[TM], bv[TN];
+            ld_tile<TM>(&As[buf][k][0], mg, MG, sw, av);
+            ld_tile<TN>(&Bs[buf][k][0], nl, NL, sw, bv);
+            uint64_t b2[TP];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-        const int kg0 = g * GROUP_K;
-        const int kg1 = min(K, kg0 + GROUP_K);
-        for (int k0 = kg0; k0 < kg1; k0 += BK) {
-            const int kc = min(BK, kg1 - k0);
-            // stage A: k fastest when a is k-contiguous, else m fastest
-            for (int e = tid; e < BM * BK; e += THREADS) {
-                int kk, i;
-                if (a_sk == 1) { kk = e % BK; i = e / BK; } else { i = e % BM; kk = e / BM; }
-                const int m = m0 + i, k = k0 + kk;
-                As[kk][i] = (m < M && kk < kc) ? Cvt<T>::up(a[(int64_t)m * a_sm + (int64_t)k * a_sk]) : 0.0f;
+            for (int j = 0; j < TP; ++j) b2[j] = ptx::pack2(bv[2 * j], bv[2 * j + 1]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                const uint64_t a2 = ptx::pack2(av[i], av[i]);
+#pragma unroll
+                for (int j = 0; j < TP; ++j) acc[i][j] = ptx::fma2_rn(a2, b2[j], acc[i][j]);
             }
-            for (int e = tid; e < BN * BK; e += THREADS) {
-                int kk, j;
-                if (QUANT || b_sk == 1) { kk = e % BK; j = e / BK; } else { j = e % BN; kk = e / BN; }
-                const int n = n0 + j, k = k0 + kk;
-                float v = 0.0f;
-                if (n < N && kk < kc) {
-                    if (QUANT) {
-                        const int per_word = 32 / qa.bits;
-                        const uint32_t word = qa.w[(int64_t)n * (K / per_word) + k / per_word];
-                        const uint32_t code = (word >> ((k % per_word) * qa.bits)) & ((1u << qa.bits) - 1u);
-                        const int64_t gi = (int64_t)n * (K / qa.gs) + k / qa.gs;
-                        const float s = Cvt<T>::up(static_cast<const T*>(qa.scales)[gi]);
-                        const float bb = Cvt<T>::up(static_cast<const T*>(qa.biases)[gi]);
-                        v = dequant_code<T>(code, s, bb);
-                    } else {
-                        v = Cvt<T>::up(b[(int64_t)k * b_sk + (int64_t)n * b_sn]);
-                    }
-                }
-                Bs[kk][j] = v;
-            }
-            __syncthreads();
-            for (int kk = 0; kk < kc; ++kk) {
-                float av[TM], bv[4];
-#pragma unroll
-                for (int i = 0; i < TM; ++i) av[i] = As[kk][ty * TM + i];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx * 4 + j];
+        }
+        if constexpr (!SPLIT) {
+            if ((s + 1) % (GROUP_K / SLAB) == 0 || s + 1 == nslab) {   // a K group is complete
 #pragma unroll
                 for (int i = 0; i < TM; ++i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] = fma_rn(av[i], bv[j], acc[i][j]);
+                    for (int j = 0; j < TP; ++j) { total[i][j] = ptx::add2_rn(total[i][j], acc[i][j]); acc[i][j] = 0; }
             }
-            __syncthreads();
         }
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) total[i][j] = SPLIT ? acc[i][j] : add_rn(total[i][j], acc[i][j]);
     }
 
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
-        const int m = m0 + ty * TM + i;
+        const int m = m0 + place<TM>(mg, i, MG);
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + place<TN>(nl, j, NL);
             if (n >= N) continue;
-            if (SPLIT) static_cast<float*>(outp)[((int64_t)g0 * M + m) * N + n] = total[i][j];
-            else static_cast<T*>(outp)[(int64_t)m * N + n] = round_out<T>(total[i][j], static_cast<const T*>(qa.out_bias), n);
+            float lo, hi;
+            ptx::unpack2(SPLIT ? acc[i][j / 2] : total[SPLIT ? 0 : i][SPLIT ? 0 : j / 2], lo, hi);
+            const float r = (j & 1) ? hi : lo;
+            if constexpr (SPLIT) static_cast<float*>(outp)[((int64_t)g0 * M + m) * N + n] = r;
+            else static_cast<T*>(outp)[(int64_t)m * N + n] = round_out<T>(r, static_cast<const T*>(qa.out_bias), n);
         }
+    }
+}
+
+// Up to eight rows of fp32: a stream of the weight. Thread nl owns column n0 + nl of all TM rows; the stages keep k
+// contiguous, as in memory, and are filled by 16-byte cp.async two stages ahead (4096 x 4096 at M = 1: 15.3 us with the
+// combine launch, of which 10.4 us are the weight's bytes; 22.5 us with the register-fetched stages of the tile kernel).
+constexpr int STREAM_N = 128, STREAM_SLAB = 32, STREAM_PITCH = STREAM_SLAB + 4, STREAM_STAGES = 3;
+template <int TM, bool SPLIT>
+__global__ void __launch_bounds__(STREAM_N) simt_stream_kernel(const float* __restrict__ a, const float* __restrict__ b, QuantArgs qa,
+                                                               float* __restrict__ out, int M, int N, int K, int64_t a_sm, int64_t b_sn) {
+    ptx::grid_dep_launch();   // the next kernel of the stream may start its set-up
+    ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
+    extern __shared__ __align__(16) float stream_smem[];
+    constexpr int ROWS = TM + STREAM_N, SEGS = STREAM_SLAB / 4;
+    const int tid = threadIdx.x, n0 = blockIdx.x * STREAM_N;
+    const int g0 = SPLIT ? (int)blockIdx.z : 0;
+    const int kbeg = g0 * GROUP_K, kend = SPLIT ? min(K, kbeg + GROUP_K) : K;
+    const int nslab = (kend - kbeg + STREAM_SLAB - 1) / STREAM_SLAB;
+    auto fill = [&](int s) {
+        if (s < nslab) {
+            const uint32_t d0 = ptx::smem_u32(stream_smem + (s % STREAM_STAGES) * ROWS * STREAM_PITCH);
+            for (int e = tid; e < ROWS * SEGS; e += STREAM_N) {
+                const int r = e / SEGS, k = kbeg + s * STREAM_SLAB + (e % SEGS) * 4;
+                const bool isa = r < TM;
+                const int i = isa ? r : n0 + r - TM;
+                const bool ok = i < (isa ? M : N) && k < kend;
+                const float* src = ok ? (isa ? a + (int64_t)i * a_sm : b + (int64_t)i * b_sn) + k : a;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d0 + (r * STREAM_PITCH + (e % SEGS) * 4) * 4), "l"(src), "r"(ok ? 16 : 0) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[TM], total[TM];
+#pragma unroll
+    for (int i = 0; i < TM; ++i) { acc[i] = 0.0f; total[i] = 0.0f; }
+    for (int s = 0; s < STREAM_STAGES - 1; ++s) fill(s);
+    for (int s = 0; s < nslab; ++s) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STREAM_STAGES - 2) : "memory");
+        __syncthreads();                                            // slab s visible; everyone is done with slab s - 1
+        fill(s + STREAM_STAGES - 1);
+        const float* const st = stream_smem + (s % STREAM_STAGES) * ROWS * STREAM_PITCH;
+#pragma unroll 2
+        for (int k4 = 0; k4 < STREAM_SLAB; k4 += 4) {
+            float bv[4];
+            ld_floats<4>(st + (TM + tid) * STREAM_PITCH + k4, bv);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                float av[4];
+                ld_floats<4>(st + i * STREAM_PITCH + k4, av);
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) acc[i] = fma_rn(av[kk], bv[kk], acc[i]);
+            }
+        }
+        if (!SPLIT && ((s + 1) % (GROUP_K / STREAM_SLAB) == 0 || s + 1 == nslab)) {      // a K group is complete
+#pragma unroll
+            for (int i = 0; i < TM; ++i) { total[i] = add_rn(total[i], acc[i]); acc[i] = 0.0f; }
+        }
+    }
+    const int n = n0 + tid;
+    if (n >= N) return;
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        if (i >= M) break;
+        if (SPLIT) out[((int64_t)g0 * M + i) * N + n] = acc[i];
+        else out[(int64_t)i * N + n] = round_out<float>(total[i], static_cast<const float*>(qa.out_bias), n);
     }
 }
 
@@ -244,24 +364,79 @@ __global__ void __launch_bounds__(256) combine_rope_kernel(const float* __restri
     else          static_cast<T*>(r.k_cache)[(int64_t)b * r.c_sb + (int64_t)(h - r.Hq) * r.c_sh + pos * r.c_sl + d] = o;
 }
 
+// Tiles of a launch: TM x TN outputs per thread, MG x NL threads, all 128 columns wide. `cost`: time per fma relative to
+// the last one (4096 x 4096 at M = 128, split: 134 / 105 / 95 us): a smaller thread tile reads shared memory more often,
+// but wastes fewer rows of a small batch. Taller thread tiles (12 and 16 rows) and 256-thread CTAs measured no faster.
+struct SimtTile { int tm, tn, mg, nl; double cost; };
+constexpr SimtTile SIMT_TILES[] = {{8, 4, 2, 32, 1.41}, {8, 8, 4, 16, 1.10}, {8, 8, 8, 16, 1.0}};
+constexpr int SIMT_NTILES = sizeof(SIMT_TILES) / sizeof(SIMT_TILES[0]);
+constexpr int STREAM_M_MAX = 8;
+
+int simt_tile(int64_t M) {
+    int best = 0;
+    double least = 0;
+    for (int i = 0; i < SIMT_NTILES; ++i) {
+        const int64_t bm = SIMT_TILES[i].tm * SIMT_TILES[i].mg;
+        const double c = SIMT_TILES[i].cost * (double)((M + bm - 1) / bm * bm);
+        if (i == 0 || c < least) { best = i; least = c; }
+    }
+    return best;
+}
+
+struct SimtArgs {
+    const void *a, *b;
+    QuantArgs qa;
+    void* dst;
+    int64_t M, N, K, a_sm, a_sk, b_sk, b_sn;
+    bool split;
+    cudaStream_t st;
+};
+
+template <int TM>
+int simt_stream(const SimtArgs& p) {
+    const int64_t G = (p.K + GROUP_K - 1) / GROUP_K;
+    if (G > 65535) return fail(BI_ERR_UNSUPPORTED, "matmul (cuda-core path): K=%lld too large", (long long)p.K);
+    dim3 grid((unsigned)((p.N + STREAM_N - 1) / STREAM_N), 1, p.split ? (unsigned)G : 1u);
+    constexpr size_t smem = (size_t)STREAM_STAGES * (TM + STREAM_N) * STREAM_PITCH * sizeof(float);
+    auto kern = p.split ? simt_stream_kernel<TM, true> : simt_stream_kernel<TM, false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return fail(BI_ERR_CUDA, "matmul (cuda-core path) smem attr: %s", cudaGetErrorString(e));
+    launch_overlapped(kern, grid, dim3(STREAM_N), smem, p.st, static_cast<const float*>(p.a), static_cast<const float*>(p.b), p.qa,
+                      static_cast<float*>(p.dst), (int)p.M, (int)p.N, (int)p.K, p.a_sm, p.b_sn);
+    return check_launch("matmul (cuda-core path)");
+}
+
+template <typename T, bool QUANT, bool VEC, int I>
+int simt_launch(int tile, const SimtArgs& p) {
+    if constexpr (I < SIMT_NTILES) {
+        if (tile != I) return simt_launch<T, QUANT, VEC, I + 1>(tile, p);
+        constexpr SimtTile t = SIMT_TILES[I];
+        constexpr int bm = t.tm * t.mg, bn = t.tn * t.nl;
+        const int64_t G = (p.K + GROUP_K - 1) / GROUP_K, gy = (p.M + bm - 1) / bm;
+        if (gy > 65535 || G > 65535) return fail(BI_ERR_UNSUPPORTED, "matmul (cuda-core path): M=%lld K=%lld too large", (long long)p.M, (long long)p.K);
+        dim3 grid((unsigned)((p.N + bn - 1) / bn), (unsigned)gy, p.split ? (unsigned)G : 1u);
+        auto kern = p.split ? simt_matmul_kernel<T, t.tm, t.tn, t.mg, t.nl, true, QUANT, VEC> : simt_matmul_kernel<T, t.tm, t.tn, t.mg, t.nl, false, QUANT, VEC>;
+        launch_overlapped(kern, grid, dim3(t.mg * t.nl), 0, p.st, static_cast<const T*>(p.a), static_cast<const T*>(p.b), p.qa, p.dst, (int)p.M, (int)p.N,
+                          (int)p.K, p.a_sm, p.a_sk, p.b_sk, p.b_sn);
+        return check_launch("matmul (cuda-core path)");
+    }
+    return fail(BI_ERR_UNSUPPORTED, "matmul (cuda-core path): no tile %d", tile);
+}
+
 template <typename T, bool QUANT>
 int simt_t(const void* a, const void* b, const QuantArgs& qa, void* out, float* part, int64_t M, int64_t N,
            int64_t K, int64_t a_sm, int64_t a_sk, int64_t b_sk, int64_t b_sn, bool split, cudaStream_t st) {
-    const int G = (int)((K + GROUP_K - 1) / GROUP_K);
-    const bool skinny = M <= 16;
-    const int BM = skinny ? 16 : 64;
-    dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)((M + BM - 1) / BM), split ? G : 1);
-    if (grid.y > 65535) return fail(BI_ERR_UNSUPPORTED, "matmul (cuda-core path): M=%lld too large", (long long)M);
-    const T* ap = static_cast<const T*>(a);
-    const T* bp = static_cast<const T*>(b);
-    void* dst = split ? static_cast<void*>(part) : out;
-#define BI_SIMT(TMV, SP) simt_matmul_kernel<T, TMV, SP, QUANT><<<grid, THREADS, 0, st>>>(ap, bp, qa, dst, (int)M, (int)N, (int)K, a_sm, a_sk, b_sk, b_sn)
-    if (skinny) { if (split) BI_SIMT(1, true); else BI_SIMT(1, false); }
-    else        { if (split) BI_SIMT(4, true); else BI_SIMT(4, false); }
-#undef BI_SIMT
-    int rc = check_launch("matmul (cuda-core path)");
+    const SimtArgs p{a, b, qa, split ? static_cast<void*>(part) : out, M, N, K, a_sm, a_sk, b_sk, b_sn, split, st};
+    int rc;
+    if constexpr (sizeof(T) == 4 && !QUANT) {
+        const bool vec = a_sk == 1 && b_sk == 1 && K % 4 == 0 && (M == 1 || a_sm % 4 == 0) && (N == 1 || b_sn % 4 == 0) && aligned(a, 16) && aligned(b, 16);
+        if (vec && M <= STREAM_M_MAX) rc = M <= 1 ? simt_stream<1>(p) : (M <= 2 ? simt_stream<2>(p) : (M <= 4 ? simt_stream<4>(p) : simt_stream<8>(p)));
+        else rc = vec ? simt_launch<T, QUANT, true, 0>(simt_tile(M), p) : simt_launch<T, QUANT, false, 0>(simt_tile(M), p);
+    } else {
+        rc = simt_launch<T, QUANT, false, 0>(simt_tile(M), p);
+    }
     if (rc || !split) return rc;
-    return combine_t<T>(part, out, G, M * N, st, qa.out_bias, N);
+    return combine_t<T>(part, out, (int)((K + GROUP_K - 1) / GROUP_K), M * N, st, qa.out_bias, N);
 }
 
 }  // namespace

@@ -103,7 +103,7 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
         return None
     out = torch.empty((M, N), dtype=out_dtype, device=dev)
     with torch.cuda.device(dev):
-        word, ws, nbytes = _launch_shape(path, batch_tile, M, N, K, lib.bi_matmul_workspace_bytes(M, N, K, code), dev)
+        word, ws, nbytes = _launch_shape(path, batch_tile, M, N, K, lib.bi_matmul_scratch_bytes(M, N, K, code), dev)
         args = (a2.data_ptr(), bt.data_ptr(), out.data_ptr(), _lib.ptr(ws), nbytes, M, N, K,
                 a2.stride(0) if M > 1 else K, a2.stride(1), bt.stride(0), bt.stride(1), code,
                 word, _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev))

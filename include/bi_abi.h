@@ -92,12 +92,16 @@ int bi_layer_norm(const void* x, const void* w, const void* b, void* out, int64_
  *                            call leaves them zero (unless a device wait    *
  *                            ran out: zero them again then). The partials   *
  *                            follow that block. Lets AUTO use SPLIT_FOLD.   *
- *   BI_MATMUL_BATCH_TILE(n)  batch rows per tile: 16, 32, 64 or 128         *
+ *   BI_MATMUL_BATCH_TILE(n)  batch rows per tile: 16, 32, 64 or 128; with   *
+ *                            BI_MATMUL_PAIR (256 weight rows on two SMs,    *
+ *                            tensor-core path only; bi_qmm needs N*K*2      *
+ *                            workspace bytes) pass n / 2, n a multiple of   *
+ *                            32 up to 256                                   *
  *   BI_QMM_STAGE_SMEM/_TMEM  bi_qmm only: stage the dequantized weight in   *
  *                            shared memory (tile body) or in tensor memory  *
  *                            (streaming; batch tiles of at most 64 rows)    *
  * ------------------------------------------------------------------------ */
-enum { BI_MATMUL_AUTO = 0, BI_MATMUL_SPLIT = 1, BI_MATMUL_FUSED = 2, BI_MATMUL_SPLIT_FOLD = 3 };
+enum { BI_MATMUL_AUTO = 0, BI_MATMUL_SPLIT = 1, BI_MATMUL_FUSED = 2, BI_MATMUL_SPLIT_FOLD = 3, BI_MATMUL_PAIR = 4 };
 #define BI_MATMUL_WS_ZEROED 0x100
 #define BI_MATMUL_BATCH_TILE(n) ((n) << 16)
 #define BI_QMM_STAGE_SMEM 0x1000000
@@ -133,6 +137,9 @@ int bi_matmul_bias(const void* a, const void* b, const void* bias, void* out, vo
  * [N, K/gs] contiguous in x's dtype; out: [M, N] contiguous, x's dtype.     *
  * ------------------------------------------------------------------------ */
 size_t bi_qmm_workspace_bytes(int64_t M, int64_t N, int64_t K, int dtype);
+/* The workspace with which BI_MATMUL_AUTO has every launch shape to choose from (at least bi_qmm_workspace_bytes; more
+ * for batches that are faster with the weight unpacked once per call). Optional. Same bits either way. */
+size_t bi_qmm_scratch_bytes(int64_t M, int64_t N, int64_t K, int dtype);
 
 int bi_qmm(const void* x, const uint32_t* w, const void* scales, const void* biases, void* out,
            void* workspace, size_t workspace_bytes, int64_t M, int64_t N, int64_t K, int64_t x_sm,

@@ -18,7 +18,7 @@ LIB_PATH = Path(__file__).resolve().parent / "libbi_b200.so"
 BI_OK = 0
 BI_ERR_UNSUPPORTED, BI_ERR_BAD_ARG, BI_ERR_MISALIGNED, BI_ERR_WORKSPACE, BI_ERR_CUDA, BI_ERR_DEVICE_WAIT = 1, 2, 3, 4, 5, 6
 BI_F32, BI_F16, BI_BF16 = 0, 1, 2
-PATH_AUTO, PATH_SPLIT, PATH_FUSED, PATH_SPLIT_FOLD = 0, 1, 2, 3
+PATH_AUTO, PATH_SPLIT, PATH_FUSED, PATH_SPLIT_FOLD, PATH_PAIR = 0, 1, 2, 3, 4
 WS_ZEROED = 0x100                 # BI_MATMUL_WS_ZEROED
 QMM_STAGE_SMEM, QMM_STAGE_TMEM = 0x1000000, 0x2000000
 COUNTER_BYTES = 16384             # BI_MATMUL_COUNTER_BYTES
@@ -39,6 +39,7 @@ SIGNATURES = {
     "bi_layer_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_float, c_int, c_void_p]),
     "bi_matmul_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int]),
     "bi_matmul_scratch_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int]),
+    "bi_qmm_scratch_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int]),
     "bi_matmul": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_int64, c_int64, c_int64, c_int64,
                           c_int64, c_int64, c_int64, c_int, c_int, c_void_p, c_void_p]),
     "bi_matmul_bias": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_int64, c_int64, c_int64, c_int64,

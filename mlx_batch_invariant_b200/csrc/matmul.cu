@@ -24,8 +24,8 @@ int64_t ngroups(int64_t K) { return (K + GROUP_K - 1) / GROUP_K; }
 // Quantized weights at decode (the streaming variant, M <= 8) are bound by the dequantizers' instruction stream, so
 // they want every SM: with fewer weight tiles than SMs they split (the partials of <= 8 rows are tiny) -- 4096 ->
 // 14336 at M = 1: 26.4 us split over 148 CTAs against 27.5 us fused on 112.
-TcShape tc_auto_shape(int64_t M, int64_t N, int64_t K, bool quant = false) {
-    TcShape sh{false, 128, nullptr, TcShape::STAGE_AUTO, Await{nullptr, nullptr, 0, 0}, nullptr};
+TcShape tc_one_sm_shape(int64_t M, int64_t N, int64_t K, bool quant) {
+    TcShape sh{false, 128, nullptr, TcShape::STAGE_AUTO, Await{nullptr, nullptr, 0, 0}, nullptr, false};
     const int64_t G = ngroups(K);
     const int64_t nt = (N + 127) / 128;
     if (quant && M <= 8 && G > 1 && nt < sm_count()) { sh.split = true; return sh; }
@@ -39,6 +39,30 @@ TcShape tc_auto_shape(int64_t M, int64_t N, int64_t K, bool quant = false) {
     sh.bm = bm_fill ? bm_fill : 16;
     return sh;
 }
+constexpr int64_t PAIR_QUANT_ELEMS = 128 << 20;      // largest quantized weight that is unpacked into the workspace (256 MB)
+
+// One SM or a pair of SMs per tile: the cheaper by what a K step of 64 was measured to take, in us, at the batch tile's
+// height (bm), times K steps, times waves of tiles, plus the launch. One SM: 0.17 + 0.0023 bm dense (N = 4096, K = 4096:
+// bm = 32 / 64 / 128 0.23 / 0.29 / 0.46), 0.28 + 0.0039 bm with packed weights, which it unpacks once per batch tile
+// (0.41 / 0.53 / 0.81). A pair: 0.29 + 0.0012 bm (bm = 96 / 128 / 256: 0.41 / 0.44 / 0.60) for 256 weight rows, and with
+// packed weights a pass that unpacks them first (0.45 us per million). The pair's taller tiles win from about 300 rows on;
+// where few tiles fill only part of a wave (small layers, short batches) one SM per tile keeps more SMs busy. Sizes
+// whose one-SM shape splits K keep it.
+constexpr int64_t PAIR_BM_MAX = 256, PAIR_BM_STEP = 32;
+TcShape tc_auto_shape(int64_t M, int64_t N, int64_t K, bool quant = false) {
+    TcShape sh = tc_one_sm_shape(M, N, K, quant);
+    if (sh.split || M <= 64 || (quant && N * K > PAIR_QUANT_ELEMS)) return sh;
+    const int64_t sms = sm_count(), pairs = sms / 2, steps = (K + 63) / 64;
+    auto waves = [](int64_t units, int64_t slots) { return (double)((units + slots - 1) / slots); };
+    const double one = 4.0 + waves((N + 127) / 128 * ((M + sh.bm - 1) / sh.bm), sms) * steps * (quant ? 0.28 + 0.0039 * sh.bm : 0.17 + 0.0023 * sh.bm);
+    double best = 0.95 * one;
+    for (int64_t bm = PAIR_BM_STEP; bm <= PAIR_BM_MAX; bm += PAIR_BM_STEP) {
+        const double cost = 5.0 + (quant ? 2.0 + 0.45e-6 * (double)(N * K) : 0.0) +
+                            waves((N + 255) / 256 * ((M + bm - 1) / bm), pairs) * steps * (0.29 + 0.0012 * bm);
+        if (cost < best) { best = cost; sh.pair = true; sh.bm = (int)bm; }
+    }
+    return sh;
+}
 // The scratch bi_matmul_workspace_bytes() promises the CUDA-core path (reference rule: M <= 32 and more than one group).
 // With more (bi_matmul_scratch_bytes) AUTO splits at any M: the split shape has G times the CTAs and no running totals in
 // registers, and won at every measured size (M = 100, 4096 x 4096: 93 against 200 us fused; M = 256, 14336 x 4096 with 235 MB
@@ -49,7 +73,7 @@ bool simt_split(int64_t M, int64_t N, int64_t K) { return ngroups(K) > 1 && ngro
 
 // `path` as the ABI packs it -> kind, flags, forced batch tile, forced staging.
 struct PathArg {
-    int kind;       // BI_MATMUL_AUTO / SPLIT / FUSED / SPLIT_FOLD
+    int kind;       // BI_MATMUL_AUTO / SPLIT / FUSED / SPLIT_FOLD / PAIR
     bool zeroed;    // BI_MATMUL_WS_ZEROED
     int bm;         // 0 = choose
     int stage;      // TcShape::STAGE_*
@@ -59,8 +83,10 @@ int parse_path(const char* op, int path, PathArg* pa) {
     pa->zeroed = (path & BI_MATMUL_WS_ZEROED) != 0;
     pa->bm = (path >> 16) & 0xff;
     pa->stage = (path & BI_QMM_STAGE_SMEM) ? TcShape::STAGE_SMEM : ((path & BI_QMM_STAGE_TMEM) ? TcShape::STAGE_TMEM : TcShape::STAGE_AUTO);
-    if (pa->kind > BI_MATMUL_SPLIT_FOLD) return fail(BI_ERR_BAD_ARG, "%s: unknown path %d", op, pa->kind);
-    if (pa->bm != 0 && pa->bm != 16 && pa->bm != 32 && pa->bm != 64 && pa->bm != 128)
+    if (pa->kind > BI_MATMUL_PAIR) return fail(BI_ERR_BAD_ARG, "%s: unknown path %d", op, pa->kind);
+    if (pa->kind == BI_MATMUL_PAIR) {
+        if (pa->bm % 16 || pa->bm > 128) return fail(BI_ERR_BAD_ARG, "%s: batch tile %d of a pair (a multiple of 32 up to 256)", op, 2 * pa->bm);
+    } else if (pa->bm != 0 && pa->bm != 16 && pa->bm != 32 && pa->bm != 64 && pa->bm != 128)
         return fail(BI_ERR_BAD_ARG, "%s: batch tile %d (16, 32, 64 or 128)", op, pa->bm);
     if (pa->kind == BI_MATMUL_SPLIT_FOLD && !pa->zeroed)
         return fail(BI_ERR_BAD_ARG, "%s: BI_MATMUL_SPLIT_FOLD needs BI_MATMUL_WS_ZEROED (a zeroed counter block)", op);
@@ -72,6 +98,22 @@ int parse_path(const char* op, int path, PathArg* pa) {
 int tc_shape(const char* op, const PathArg& pa, void* ws, size_t ws_bytes, int64_t M, int64_t N, int64_t K,
              TcShape* sh, float** part, bool quant = false) {
     *sh = tc_auto_shape(M, N, K, quant);
+    *part = nullptr;
+    if (pa.kind == BI_MATMUL_PAIR || (pa.kind == BI_MATMUL_AUTO && sh->pair && !pa.bm && pa.stage == TcShape::STAGE_AUTO)) {
+        const size_t head = quant && pa.zeroed ? COUNTER_BYTES : 0;
+        const size_t need = quant ? head + (size_t)N * (size_t)K * 2 : 0;      // the weight in 16 bits
+        const bool fits = !quant || (ws && ws_bytes >= need && aligned(ws, 16) && N * K <= PAIR_QUANT_ELEMS);
+        if (fits || pa.kind == BI_MATMUL_PAIR) {
+            if (!fits) return fail(BI_ERR_WORKSPACE, "%s: the pair shape needs %zu workspace bytes (16-byte aligned, at most 256 MB of weight), got %zu", op, need, ws_bytes);
+            if (!sh->pair) sh->bm = 256;
+            if (pa.bm) sh->bm = 2 * pa.bm;
+            sh->pair = true;
+            sh->split = false;
+            if (quant) *part = reinterpret_cast<float*>(static_cast<char*>(ws) + head);
+            return BI_OK;
+        }
+    }
+    if (sh->pair) *sh = tc_one_sm_shape(M, N, K, quant);
     if (pa.kind == BI_MATMUL_SPLIT || pa.kind == BI_MATMUL_SPLIT_FOLD) { sh->split = true; sh->bm = 128; }
     if (pa.kind == BI_MATMUL_FUSED && sh->split) {
         sh->split = false;
@@ -142,6 +184,14 @@ extern "C" size_t bi_qmm_workspace_bytes(int64_t M, int64_t N, int64_t K, int dt
     return COUNTER_BYTES + (size_t)ngroups(K) * (size_t)M * (size_t)N * sizeof(float);
 }
 
+extern "C" size_t bi_qmm_scratch_bytes(int64_t M, int64_t N, int64_t K, int dtype) {
+    using namespace bi;
+    const size_t least = bi_qmm_workspace_bytes(M, N, K, dtype);
+    if (dtype == BI_F32 || M <= 0 || N <= 0 || K <= 0 || N * K > PAIR_QUANT_ELEMS || !tc_auto_shape(M, N, K, true).pair) return least;
+    const size_t pair = COUNTER_BYTES + (size_t)N * (size_t)K * 2;
+    return pair > least ? pair : least;
+}
+
 namespace bi {
 namespace {
 int check_await(const char* op, const Await& aw) {
@@ -185,6 +235,7 @@ int matmul_impl(const void* a, const void* b, void* out, void* workspace, size_t
         sh.await = aw;
         sh.bias = bias;
         const int64_t w_ld = N == 1 ? K : b_sn;
+        if (sh.pair) return launch_pair_matmul(a, x_ld, b, w_ld, out, M, N, K, dtype, sh, status, st);
         rc = launch_tc_matmul(a, x_ld, b, w_ld, nullptr, out, part, M, N, K, dtype, sh, status, st);
         if (rc || !sh.split || sh.counters) return rc;
         if (rope) return launch_combine_rope(part, (int)ngroups(K), M * N, dtype, st, *rope);
@@ -262,6 +313,10 @@ int qmm_impl(const void* x, const uint32_t* w, const void* scales, const void* b
         rc = tc_shape("bi_qmm", pa, workspace, workspace_bytes, M, N, K, &sh, &part, true);
         if (rc) return rc;
         sh.await = aw;
+        if (sh.pair) {
+            rc = launch_dequant(q, part, N, K, dtype, st);
+            return rc ? rc : launch_pair_matmul(x, x_ld, part, K, out, M, N, K, dtype, sh, status, st);
+        }
         rc = launch_tc_matmul(x, x_ld, nullptr, 0, &q, out, part, M, N, K, dtype, sh, status, st);
         if (rc || !sh.split || sh.counters) return rc;
         if (rope) return launch_combine_rope(part, (int)ngroups(K), M * N, dtype, st, *rope);

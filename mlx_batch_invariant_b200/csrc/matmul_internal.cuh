@@ -54,6 +54,8 @@ bool tc_matmul_supported(const void* x, int64_t x_ld, const void* w, int64_t w_l
 //   counters  split only: per-tile arrival counters (all zero) -> the last CTA of a tile folds the partials and
 //             writes `out` itself; nullptr -> the caller launches the combine kernel
 //   stage     quantized only: how the dequantized weight operand reaches the MMA
+//   pair      tiles of 256 weight rows x bm batch rows (a multiple of 32, at most 256) on pairs of SMs, folding in
+//             registers (matmul_pair.cu); split, counters and stage do not apply
 //   await     the activation is the destination of a peer gather whose arrival nobody has waited for yet: the
 //             kernel starts streaming weights at once and reads the activation only after every peer's flag
 //             has reached *epoch (bounded wait); flags == nullptr -> nothing to wait for
@@ -70,9 +72,14 @@ struct TcShape {
     int stage;
     Await await;
     const void* bias;     // optional [N] bias in the output dtype, added after the output's rounding
+    bool pair;
 };
 int launch_tc_matmul(const void* x, int64_t x_ld, const void* w, int64_t w_ld, const TcQuant* q, void* out,
                      float* part, int64_t M, int64_t N, int64_t K, int dtype, const TcShape& shape, int32_t* status,
                      cudaStream_t st);
+// Packed weight -> 16-bit [N, K] rows at `out` (16-byte aligned); K a multiple of the group size, N * K / 8 below 2^31.
+int launch_dequant(const TcQuant& q, void* out, int64_t N, int64_t K, int dtype, cudaStream_t st);
+int launch_pair_matmul(const void* x, int64_t x_ld, const void* w, int64_t w_ld, void* out, int64_t M, int64_t N, int64_t K, int dtype,
+                       const TcShape& shape, int32_t* status, cudaStream_t st);
 
 }  // namespace bi

@@ -1,0 +1,167 @@
+// Pieces shared by the tensor-core matmul kernels: bounded barrier waits, the affine dequantizer and the
+// tensor-map encoders.
+#pragma once
+#include <cuda.h>
+#include "bi_common.cuh"
+#include "bi_ptx.cuh"
+
+namespace bi {
+namespace {
+
+constexpr int BLOCK_N = 128;  // weight rows of an operand tile (the MMA's M, per CTA)
+constexpr int BLOCK_K = 64;   // elements per tile along K: 128 bytes = one swizzle row
+constexpr int UMMA_K = 16;
+constexpr uint64_t WAIT_LIMIT_NS = 2000000000ull;
+#ifndef BI_EPI_SLEEP_NS
+#define BI_EPI_SLEEP_NS 100
+#endif
+
+enum { ROLE_TMA = 1, ROLE_MMA = 2, ROLE_EPI = 3, ROLE_DEQ = 4 };
+
+struct Ctl {
+    int32_t* status;
+    volatile int* abort_flag;  // shared memory
+};
+
+__device__ __forceinline__ void report(const Ctl& c, int role, int idx) {
+    *c.abort_flag = 1;
+    if (c.status) atomicCAS(c.status, 0, (int)(0x10000 | (role << 8) | (idx & 0xff)));
+}
+
+// Wait for barrier phase `parity` to complete. Gives up after WAIT_LIMIT_NS or when another
+// role has raised the abort flag; returns false then. CLUSTER: the arrivals come from the other CTA of a pair.
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity, const Ctl& c, int role, int idx) {
+    if (role == ROLE_EPI || role == ROLE_DEQ) {
+        // whole warps wait here; back off so they do not take issue slots from the TMA and MMA threads
+        for (int i = 0; i < 2048; ++i) {
+            if ((CLUSTER ? ptx::mbar_try_wait_cluster(bar, parity) : ptx::mbar_try_wait(bar, parity))) return true;
+            __nanosleep(BI_EPI_SLEEP_NS);
+        }
+    } else {
+        for (int i = 0; i < 4096; ++i)
+            if ((CLUSTER ? ptx::mbar_try_wait_cluster(bar, parity) : ptx::mbar_try_wait(bar, parity))) return true;
+    }
+    const uint64_t t0 = ptx::globaltimer_ns();
+    while (true) {
+        for (int i = 0; i < 256; ++i)
+            if ((CLUSTER ? ptx::mbar_try_wait_cluster(bar, parity) : ptx::mbar_try_wait(bar, parity))) return true;
+        if (*c.abort_flag) return false;
+        if (ptx::globaltimer_ns() - t0 > WAIT_LIMIT_NS) { report(c, role, idx); return false; }
+    }
+}
+
+template <typename T> struct Pack2;
+template <> struct Pack2<__nv_bfloat16> {
+    static __device__ __forceinline__ uint32_t rn(float lo, float hi) {
+        __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);  // .x = lo (low address)
+        return *reinterpret_cast<uint32_t*>(&v);
+    }
+};
+template <> struct Pack2<__half> {
+    static __device__ __forceinline__ uint32_t rn(float lo, float hi) {
+        __half2 v = __floats2half2_rn(lo, hi);
+        return *reinterpret_cast<uint32_t*>(&v);
+    }
+};
+
+// Byte offset, inside a chunk's packed codes, of 16-byte piece `piece` of weight row `row` (pieces count along the
+// row's bytes of the chunk). The codes lie as boxes of 128 rows x span bytes under the TMA swizzle of that span:
+// the piece index inside a span is XORed with bits [7, 7 + log2(span / 16)) of the byte address.
+__device__ __forceinline__ uint32_t raw_piece_offset(int row, int piece, int span) {
+    const int per = span >> 4;                         // pieces per row of one box: 2, 4 or 8
+    const int box = piece / per, pb = piece - box * per;
+    const int sw = ((row * span) >> 7) & (per - 1);
+    return (uint32_t)(box * (BLOCK_N * span) + row * span + ((pb ^ sw) << 4));
+}
+
+// Eight consecutive codes -> eight T values, one 16-byte swizzle chunk.
+//   value = T(fma(float(code), scale, bias))   fp32 fma, one rounding.
+// float(code) is formed exactly without an integer->float conversion: a byte permute drops the code
+// into the low mantissa byte of 2^23 (0x4B0000cc = 8388608 + cc) and 2^23 is subtracted, which is
+// exact. The subtract and the fma run as packed f32x2 instructions: two independent IEEE
+// round-to-nearest operations each, same bits as the scalar forms.
+template <typename T, int QBITS>
+__device__ __forceinline__ uint4 dequant8(const uint32_t* words, uint64_t s2, uint64_t b2) {
+    const uint64_t neg_magic = ptx::pack2(-8388608.0f, -8388608.0f);
+    uint32_t src_even[4], src_odd[4];  // register + byte index holding codes 2i and 2i+1
+    uint32_t o[4];
+    if (QBITS == 4) {
+        const uint32_t lo = words[0] & 0x0F0F0F0Fu;          // bytes: codes 0, 2, 4, 6
+        const uint32_t hi = (words[0] >> 4) & 0x0F0F0F0Fu;   // bytes: codes 1, 3, 5, 7
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            src_even[i] = __byte_perm(lo, 0x4B000000u, 0x7540u + i);
+            src_odd[i] = __byte_perm(hi, 0x4B000000u, 0x7540u + i);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            src_even[i] = __byte_perm(words[i >> 1], 0x4B000000u, 0x7540u + 2 * (i & 1));
+            src_odd[i] = __byte_perm(words[i >> 1], 0x4B000000u, 0x7540u + 2 * (i & 1) + 1);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint64_t v = ptx::pack2(__uint_as_float(src_even[i]), __uint_as_float(src_odd[i]));
+        v = ptx::add2_rn(v, neg_magic);
+        v = ptx::fma2_rn(v, s2, b2);
+        float x, y;
+        ptx::unpack2(v, x, y);
+        o[i] = Pack2<T>::rn(x, y);
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// ---- host side -----------------------------------------------------------------
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+[[maybe_unused]] EncodeTiledFn encode_fn() {
+    static EncodeTiledFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<EncodeTiledFn>(p);
+    }();
+    return fn;
+}
+
+// 2-D row-major tensor [rows, cols] with `ld` elements between rows; box = [box_rows, box_cols].
+[[maybe_unused]] int make_map(CUtensorMap* m, CUtensorMapDataType dt, size_t esize, const void* base, uint64_t cols, uint64_t rows,
+             uint64_t ld, uint32_t box_cols, uint32_t box_rows, CUtensorMapSwizzle sw) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return fail(BI_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    cuuint64_t gdim[2] = {cols, rows};
+    cuuint64_t gstr[1] = {ld * esize};
+    cuuint32_t box[2] = {box_cols, box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = fn(m, dt, 2, const_cast<void*>(base), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(BI_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+    return BI_OK;
+}
+
+// The same tensor seen as [K/64 blocks][rows][inner elements] (needs K % 64 == 0; inner = the elements that hold
+// 64 values of K: 64 for 16-bit data, 8 or 16 words for packed codes): a box of `depth` blocks lands as `depth`
+// consecutive K-step tiles of box_rows x (inner * esize) bytes.
+[[maybe_unused]] int make_map3(CUtensorMap* m, CUtensorMapDataType dt, size_t esize, const void* base, uint64_t kblocks, uint64_t rows,
+              uint64_t ld, uint32_t box_rows, uint32_t depth, uint32_t inner = BLOCK_K,
+              CUtensorMapSwizzle sw = CU_TENSOR_MAP_SWIZZLE_128B) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return fail(BI_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    cuuint64_t gdim[3] = {(cuuint64_t)inner, rows, kblocks};
+    cuuint64_t gstr[2] = {ld * esize, (cuuint64_t)inner * esize};
+    cuuint32_t box[3] = {(cuuint32_t)inner, box_rows, depth};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(m, dt, 3, const_cast<void*>(base), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(BI_ERR_CUDA, "cuTensorMapEncodeTiled (3-D) failed with CUresult %d", (int)r);
+    return BI_OK;
+}
+
+}  // namespace
+}  // namespace bi

@@ -18,15 +18,15 @@ from ._util import adopt, dtype_code, give_back, require_cuda, rows_16b
 
 GROUP_K = 256
 
-_PATHS = {"auto": _lib.PATH_AUTO, "split": _lib.PATH_SPLIT, "fused": _lib.PATH_FUSED, "fold": _lib.PATH_SPLIT_FOLD}
+_PATHS = {"auto": _lib.PATH_AUTO, "split": _lib.PATH_SPLIT, "fused": _lib.PATH_FUSED, "fold": _lib.PATH_SPLIT_FOLD, "pair": _lib.PATH_PAIR}
 
 
-def _launch_shape(path: str, batch_tile: int | None, M: int, N: int, K: int, ws_bytes_auto: int, dev: torch.device):
+def _launch_shape(path: str, batch_tile: int | None, M: int, N: int, K: int, ws_bytes_auto: int, dev: torch.device, pair_bytes: int = 0):
     """(path word, workspace tensor or None, workspace bytes) for a call. The workspace is the stream's
     persistent one, whose head holds the zeroed arrival counters of the in-kernel fold."""
     G = (K + GROUP_K - 1) // GROUP_K
-    nbytes = ws_bytes_auto if path in ("auto", "fused") else _lib.COUNTER_BYTES + G * M * N * 4
-    word = _PATHS[path] | _lib.WS_ZEROED | (_lib.batch_tile(batch_tile) if batch_tile else 0)
+    nbytes = ws_bytes_auto if path in ("auto", "fused") else pair_bytes if path == "pair" else _lib.COUNTER_BYTES + G * M * N * 4
+    word = _PATHS[path] | _lib.WS_ZEROED | (_lib.batch_tile(batch_tile // 2 if path == "pair" else batch_tile) if batch_tile else 0)
     ws = _lib.matmul_workspace(dev, nbytes) if nbytes else None
     return word, ws, (ws.numel() if ws is not None else 0)
 
@@ -45,7 +45,8 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
 
     ``a`` may have extra leading dims (flattened into M); ``b`` must be 2-D (a transposed
     view is fine). fp32 accumulation; the output dtype is the promoted input dtype.
-    ``path`` ("auto", "split", "fused", "fold") and ``batch_tile`` (16, 32, 64, 128 batch rows per tile)
+    ``path`` ("auto", "split", "fused", "fold", "pair") and ``batch_tile`` (16, 32, 64, 128 batch rows per tile;
+    "pair": a multiple of 32 up to 256)
     force a launch shape; all give the same bits. ``awaiting`` (flags pointer, epoch pointer, rank, world) says
     that ``a`` is the destination of a peer gather nobody has waited for yet: the kernel waits for it itself,
     after it has started streaming the weight (runner/peer.py). ``bias`` ([N], the output dtype) is added to the

@@ -89,7 +89,8 @@ def batch_invariant_quantized_matmul(x, w, scales, biases, *, group_size: int, b
         return None
     out = torch.empty((M, N), dtype=dt, device=dev)
     with torch.cuda.device(dev):
-        word, ws, nbytes = _launch_shape(path, batch_tile, M, N, K, lib.bi_qmm_workspace_bytes(M, N, K, code), dev)
+        word, ws, nbytes = _launch_shape(path, batch_tile, M, N, K, lib.bi_qmm_scratch_bytes(M, N, K, code), dev,
+                                       _lib.COUNTER_BYTES + 2 * N * K)
         args = (x2.data_ptr(), wt.data_ptr(), st.data_ptr(), bt.data_ptr(), out.data_ptr(),
                 _lib.ptr(ws), nbytes, M, N, K, x2.stride(0) if M > 1 else K, group_size, bits, code,
                 word | _STAGES[stage], _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev))

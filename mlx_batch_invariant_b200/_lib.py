@@ -6,6 +6,7 @@ If the shared object is missing the first kernel call raises, loudly.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import threading
 from ctypes import c_char_p, c_float, c_int, c_int32, c_int64, c_size_t, c_void_p, POINTER
@@ -138,7 +139,16 @@ def check(code: int) -> None:
 
 
 def stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index if device.index is not None else torch.cuda.current_device())
+
+
+_AS_IT_IS = contextlib.nullcontext()
+
+
+def on_device(device: torch.device):
+    """``torch.cuda.device(device)`` where the current device is another one, else a context that does nothing: the
+    switch and its way back cost a decode-sized call 2 us of host time."""
+    return _AS_IT_IS if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def ptr(t: torch.Tensor | None) -> int | None:
@@ -167,7 +177,7 @@ _workspaces: dict[tuple[int, int], torch.Tensor] = {}
 def matmul_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     """A zero-headed workspace of at least `nbytes` for the current stream of `device`."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
-    key = (idx, torch.cuda.current_stream(device).cuda_stream)
+    key = (idx, torch._C._cuda_getCurrentRawStream(idx))
     ws = _workspaces.get(key)
     need = max(nbytes, COUNTER_BYTES)
     if ws is None or ws.numel() < need:

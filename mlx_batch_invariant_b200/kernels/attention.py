@@ -85,13 +85,13 @@ def batch_invariant_decode_attention(q, k, v, *, scale: float, split_size: int =
     nbytes = lib.bi_attn_decode_workspace_bytes(B, Hq, L, D, split_size)
     ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=dev)
     if push is not None:
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             _lib.check(lib.bi_attn_decode_push(qc.data_ptr(), kt.data_ptr(), vt.data_ptr(), _lib.ptr(lens), ws.data_ptr(), nbytes,
                                                B, Hq, Hkv, L, D, sb, sh, sl, float(scale), int(split_size), code,
                                                _lib.stream_ptr(dev), *push, _lib.status_word(dev).data_ptr()))
         return None
     out = torch.empty_like(qc)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.bi_attn_decode(qc.data_ptr(), kt.data_ptr(), vt.data_ptr(), out.data_ptr(), _lib.ptr(lens),
                                       ws.data_ptr(), nbytes, B, Hq, Hkv, L, D, sb, sh, sl, float(scale),
                                       int(split_size), code, _lib.stream_ptr(dev)))
@@ -119,7 +119,7 @@ def batch_invariant_paged_decode_attention(q, k_pages, v_pages, block_table, kv_
     lib = _lib.load()
     nbytes = lib.bi_attn_decode_workspace_bytes(B, Hq, max_pages * page, D, split_size)
     ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.bi_attn_decode_paged(qc.data_ptr(), kt.data_ptr(), vt.data_ptr(), out.data_ptr(), lens.data_ptr(),
                                             table.data_ptr(), ws.data_ptr(), nbytes, B, Hq, Hkv, max_pages, page, D, sp, sh, sl,
                                             table.stride(0), float(scale), int(split_size), code, _lib.stream_ptr(dev)))
@@ -136,7 +136,7 @@ def batch_invariant_prefill_attention(q, k, v, *, scale: float, causal: bool, sp
     qc = qt.contiguous()
     kt, vt, sb, sh, sl = _kv_layout(kt, vt)
     out = torch.empty_like(qc)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.load().bi_attn_prefill(qc.data_ptr(), kt.data_ptr(), vt.data_ptr(), out.data_ptr(), B, Hq, Hkv,
                                                Tq, L, D, sb, sh, sl, float(scale), 1 if causal else 0,
                                                int(split_size), code, _lib.stream_ptr(dev)))

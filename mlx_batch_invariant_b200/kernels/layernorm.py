@@ -30,7 +30,7 @@ def batch_invariant_layer_norm(x, weight, bias, eps: float):
     rows = xt.numel() // D if D else 0
     x2 = xt.reshape(rows, D).contiguous()
     out = torch.empty_like(x2)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(_lib.load().bi_layer_norm(x2.data_ptr(), _lib.ptr(wt), _lib.ptr(bt), out.data_ptr(), rows, D, float(eps),
                                              code, _lib.stream_ptr(dev)))
     return give_back(out.reshape(xt.shape), x, foreign)

@@ -70,9 +70,9 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
         raise ValueError(f"shape mismatch {tuple(at.shape)} @ {tuple(bt.shape)}")
     dev = require_cuda(at, bt)
     N = bt.shape[1]
-    out_dtype = torch.result_type(at, bt)
+    out_dtype = at.dtype if at.dtype == bt.dtype else torch.result_type(at, bt)
     code = dtype_code(out_dtype)
-    a2 = at.reshape(-1, K)
+    a2 = at if at.ndim == 2 and K else at.reshape(-1, K)
     if a2.dtype != out_dtype:
         a2 = a2.to(out_dtype)
     if bt.dtype != out_dtype:
@@ -86,7 +86,7 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
     if rope is not None:
         if bias is not None or push is not None or awaiting is not None or M == 0:
             raise ValueError("rope cannot be combined with bias, push, awaiting or an empty batch")
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             word, ws, nbytes = _launch_shape("split", batch_tile, M, N, K, 0, dev)
             _lib.check(lib.bi_matmul_rope(a2.data_ptr(), bt.data_ptr(), _lib.ptr(ws), nbytes, M, N, K,
                                           a2.stride(0) if M > 1 else K, a2.stride(1), bt.stride(0), bt.stride(1), code, word,
@@ -95,7 +95,7 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
     if push is not None:
         if bias is not None or M == 0:
             raise ValueError("push cannot be combined with bias or an empty batch")
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             word, ws, nbytes = _launch_shape("split", batch_tile, M, N, K, 0, dev)
             aw = awaiting[:2] if awaiting is not None else (None, None)
             _lib.check(lib.bi_matmul_push(a2.data_ptr(), bt.data_ptr(), _lib.ptr(ws), nbytes, M, N, K,
@@ -103,7 +103,7 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
                                           _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev), *aw, *push))
         return None
     out = torch.empty((M, N), dtype=out_dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         word, ws, nbytes = _launch_shape(path, batch_tile, M, N, K, lib.bi_matmul_scratch_bytes(M, N, K, code), dev)
         args = (a2.data_ptr(), bt.data_ptr(), out.data_ptr(), _lib.ptr(ws), nbytes, M, N, K,
                 a2.stride(0) if M > 1 else K, a2.stride(1), bt.stride(0), bt.stride(1), code,
@@ -116,4 +116,4 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
             _lib.check(lib.bi_matmul_bias(args[0], args[1], bias_t.data_ptr(), *args[2:]))
         else:
             _lib.check(lib.bi_matmul(*args) if awaiting is None else lib.bi_matmul_awaiting(*args, *awaiting))
-    return give_back(out.reshape(*lead, N), a, foreign)
+    return give_back(out if at.ndim == 2 else out.reshape(*lead, N), a, foreign)

@@ -62,7 +62,7 @@ def batch_invariant_quantized_matmul(x, w, scales, biases, *, group_size: int, b
         raise ValueError(f"scales/biases shape {tuple(st.shape)} does not match (N={N}, K/group_size={K // group_size})")
     dt = xt.dtype
     code = dtype_code(dt)
-    x2 = rows_16b(xt.reshape(-1, K))
+    x2 = rows_16b(xt if xt.ndim == 2 and K else xt.reshape(-1, K))
     M = x2.shape[0]
     st = st.to(dt).contiguous()
     bt = bt.to(dt).contiguous()
@@ -71,7 +71,7 @@ def batch_invariant_quantized_matmul(x, w, scales, biases, *, group_size: int, b
     if rope is not None:
         if push is not None or awaiting is not None or M == 0:
             raise ValueError("rope cannot be combined with push, awaiting or an empty batch")
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             word, ws, nbytes = _launch_shape("split", batch_tile, M, N, K, 0, dev)
             _lib.check(lib.bi_qmm_rope(x2.data_ptr(), wt.data_ptr(), st.data_ptr(), bt.data_ptr(), _lib.ptr(ws), nbytes, M, N, K,
                                        x2.stride(0) if M > 1 else K, group_size, bits, code, word | _STAGES[stage],
@@ -80,7 +80,7 @@ def batch_invariant_quantized_matmul(x, w, scales, biases, *, group_size: int, b
     if push is not None:
         if M == 0:
             raise ValueError("push cannot be combined with an empty batch")
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             word, ws, nbytes = _launch_shape("split", batch_tile, M, N, K, 0, dev)
             aw = awaiting[:2] if awaiting is not None else (None, None)
             _lib.check(lib.bi_qmm_push(x2.data_ptr(), wt.data_ptr(), st.data_ptr(), bt.data_ptr(), _lib.ptr(ws), nbytes, M, N, K,
@@ -88,11 +88,11 @@ def batch_invariant_quantized_matmul(x, w, scales, biases, *, group_size: int, b
                                        _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev), *aw, *push))
         return None
     out = torch.empty((M, N), dtype=dt, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         word, ws, nbytes = _launch_shape(path, batch_tile, M, N, K, lib.bi_qmm_scratch_bytes(M, N, K, code), dev,
                                        _lib.COUNTER_BYTES + 2 * N * K)
         args = (x2.data_ptr(), wt.data_ptr(), st.data_ptr(), bt.data_ptr(), out.data_ptr(),
                 _lib.ptr(ws), nbytes, M, N, K, x2.stride(0) if M > 1 else K, group_size, bits, code,
                 word | _STAGES[stage], _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev))
         _lib.check(lib.bi_qmm(*args) if awaiting is None else lib.bi_qmm_awaiting(*args, *awaiting))
-    return give_back(out.reshape(*lead, N), x, foreign)
+    return give_back(out if xt.ndim == 2 else out.reshape(*lead, N), x, foreign)

@@ -27,9 +27,9 @@ def batch_invariant_rms_norm(x, weight, eps: float):
             wt = wt.to(xt.dtype)
         wt = wt.contiguous()
     rows = xt.numel() // D if D else 0
-    x2 = xt.reshape(rows, D).contiguous()
-    out = torch.empty_like(x2)
-    with torch.cuda.device(dev):
+    x2 = xt.contiguous()
+    out = torch.empty(xt.shape, dtype=xt.dtype, device=dev)
+    with _lib.on_device(dev):
         _lib.check(_lib.load().bi_rms_norm(x2.data_ptr(), _lib.ptr(wt), out.data_ptr(), rows, D, float(eps), code,
                                            _lib.stream_ptr(dev)))
-    return give_back(out.reshape(xt.shape), x, foreign)
+    return give_back(out, x, foreign)

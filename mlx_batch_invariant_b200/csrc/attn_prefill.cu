@@ -15,12 +15,14 @@
 //      rows, every query element two keys;
 //   B  softmax scalars: a warp takes QB / 4 rows, lane = key: prefix maximum (skipped when no score of the block exceeds
 //      its row's running maximum), one exponential per score, factors to shared memory;
-//   C  accumulation: a thread owns TQ rows x 8 dims and walks the block's keys in order.
+//   C  accumulation: a thread owns TQ rows x 8 dims and walks the block's keys in order, up to the last one its warp sees.
 // K is refilled (cp.async) once the scores exist, V is double buffered. Up to three CTAs share an SM, so that one computes
 // while another waits at a barrier.
 //
 // Measured (bf16, D = 128, 32 query / 8 kv heads, causal): 2048 tokens 1231 us (fma pipe 66 % busy, the rest operand
 // conflicts and barriers), before 4442 us with eight lanes per key stream; 2 x 512 tokens 175 us, before 740 us.
+#include <climits>
+#include <type_traits>
 #include "attn_common.cuh"
 
 namespace bi {
@@ -226,6 +228,16 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
     // accumulation tile of this thread: rows tq .. tq+3, dims td .. td+7
     constexpr int DG = D / 8;
     const int tq = (tid / DG) * TQ, td = (tid % DG) * 8;
+    // Keys that every row of this warp's tiles sees, and that any of them sees (rows past the end do not count).
+    int seen_all = INT_MAX, seen_any = 0;
+#pragma unroll
+    for (int i = 0; i < TQ; ++i) {
+        const int n = ns[tq + i];
+        if (n > 0) seen_all = min(seen_all, n);
+        seen_any = max(seen_any, n);
+    }
+    seen_all = __reduce_min_sync(0xffffffffu, seen_all);
+    seen_any = __reduce_max_sync(0xffffffffu, seen_any);
     uint64_t acc[TQ][4];
     // merged accumulators of the thread: pairs (2i, 2i+1) of its TQ x 4 at tot[i * PF_THREADS]
     ulonglong2* const tot = reinterpret_cast<ulonglong2*>(sm + C::TOFF) + tid;
@@ -313,8 +325,8 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
                     for (int u = 0; u < RG; ++u) {
                         const float e = expf_canon(-fabsf(sub_rn(s4[u], m4[u])));
                         const bool rises = s4[u] >= m4[u];
-                        c4[u] = on4[u] && rises ? e : 1.0f;
-                        p4[u] = on4[u] ? (rises ? 1.0f : e) : 0.0f;
+                        c4[u] = rises ? e : 1.0f;                        // of a key the row does not see: never read
+                        p4[u] = rises ? 1.0f : e;
                     }
                     st_vec<RG>(ps + key * C::PPITCH + rr, p4);
                     st_vec<RG>(cs + key * C::PPITCH + rr, c4);
@@ -322,10 +334,10 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
                 }
             }
             __syncthreads();
-            // ---- C: accumulation, key by key
+            // ---- C: accumulation, key by key. A key that a row does not see leaves the row's state alone: folding it in with
+            // weight 0 would turn an infinity or NaN of a later token's value into NaN in this row.
             const uint8_t* const vb = vs + buf * KB * C::KROW + td * (int)sizeof(T);
-#pragma unroll 8
-            for (int i = 0; i < cnt; ++i) {
+            auto fold = [&](int i, auto masked) {
                 float p[TQ], c[TQ];
                 ld_vec<TQ>(ps + i * C::PPITCH + tq, p);
                 ld_vec<TQ>(cs + i * C::PPITCH + tq, c);
@@ -333,6 +345,7 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
                 value_pairs<T>(vb + i * C::KROW, v2);
 #pragma unroll
                 for (int iq = 0; iq < TQ; ++iq) {
+                    if (decltype(masked)::value && j + i >= ns[tq + iq]) continue;
                     const uint64_t p2 = ptx::pack2(p[iq], p[iq]), c2 = ptx::pack2(c[iq], c[iq]);
                     l[iq] = fma_rn(l[iq], c[iq], p[iq]);
 #pragma unroll
@@ -340,7 +353,12 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
 #pragma unroll
                     for (int d = 0; d < 4; ++d) acc[iq][d] = ptx::fma2_rn(acc[iq][d], c2, t2[d]);
                 }
-            }
+            };
+            const int all = min(cnt, seen_all - j), any = min(cnt, seen_any - j);
+#pragma unroll 8
+            for (int i = 0; i < all; ++i) fold(i, std::false_type{});
+#pragma unroll 1
+            for (int i = max(all, 0); i < any; ++i) fold(i, std::true_type{});
             buf ^= 1;
         }
         // ---- the split's end: fold it into the running state of every row that saw a key of it

@@ -42,3 +42,32 @@ def test_prefill_rows_not_16_byte_aligned(bi):
     _lib.check(_lib.load().bi_attn_prefill(qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), B, H, H, T, T, D, kc.stride(0),
                                            kc.stride(1), kc.stride(2), D ** -0.5, 1, 256, _lib.BI_BF16, _lib.stream_ptr(qc.device)))
     assert R.bits_of(out) == R.bits_of(R.attn_prefill(q, k, v, scale=D ** -0.5, causal=True))
+
+
+# Launches of B sequences x 8 query / 4 kv heads x 45 queries that take 1, 2 and 4 rows per thread (a block is
+# rows * 1024 / head_dim query rows; four rows from two blocks per SM on, two from one per two SMs on, 148 SMs).
+ROWS_PER_THREAD = [(32, 1, 1), (32, 2, 10), (32, 4, 74), (64, 1, 1), (64, 2, 7), (64, 4, 37),
+                   (128, 1, 1), (128, 2, 4), (128, 4, 25), (256, 1, 1), (256, 2, 2), (256, 4, 13)]
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("D,rows,B", ROWS_PER_THREAD)
+def test_later_tokens_never_reach_a_row(bi, dt, D, rows, B):
+    """Infinities and NaN in a later token's key and value: a row that does not see the token keeps the bits it has
+    without them and those of the prefix run alone, in every row block and at every number of rows per thread."""
+    if dt == torch.float32 and D == 256:
+        B = min(B, 2)
+    L, T, split = 77, 45, 32
+    g = torch.Generator().manual_seed(D + rows)
+    q, k, v = (torch.randn(B, h, n, D, generator=g).to(dt).cuda() for h, n in ((8, T), (4, L), (4, L)))
+    run = lambda q, k, v: bi.batch_invariant_prefill_attention(q, k, v, scale=D ** -0.5, causal=True, split_size=split)
+    clean = run(q, k, v)
+    for t in (1, 17, 30, 44):                                     # rows 0 .. t - 1 do not see keys from L - T + t on
+        key = L - T + t
+        kp, vp = k.clone(), v.clone()
+        vp[:, :, key:, 0::2], vp[:, :, key:, 1::2] = float("inf"), float("nan")
+        kp[:, :, key] = float("nan")
+        kp[:, :, key + 1:] = float("-inf")
+        got = run(q, kp, vp)[:, :, :t]
+        assert R.bits_of(got) == R.bits_of(clean[:, :, :t]), t
+        assert R.bits_of(got) == R.bits_of(run(q[:, :, :t], k[:, :, :key], v[:, :, :key])), t

@@ -15,14 +15,12 @@
 //      rows, every query element two keys;
 //   B  softmax scalars: a warp takes QB / 4 rows, lane = key: prefix maximum (skipped when no score of the block exceeds
 //      its row's running maximum), one exponential per score, factors to shared memory;
-//   C  accumulation: a thread owns TQ rows x 8 dims and walks the block's keys in order, up to the last one its warp sees.
+//   C  accumulation: a thread owns TQ rows x 8 dims and walks the block's keys in order.
 // K is refilled (cp.async) once the scores exist, V is double buffered. Up to three CTAs share an SM, so that one computes
 // while another waits at a barrier.
 //
 // Measured (bf16, D = 128, 32 query / 8 kv heads, causal): 2048 tokens 1231 us (fma pipe 66 % busy, the rest operand
 // conflicts and barriers), before 4442 us with eight lanes per key stream; 2 x 512 tokens 175 us, before 740 us.
-#include <climits>
-#include <type_traits>
 #include "attn_common.cuh"
 
 namespace bi {
@@ -163,6 +161,72 @@ __device__ __forceinline__ void value_pairs(const uint8_t* p, uint64_t (&v2)[4])
     }
 }
 
+// Row block of a CTA. Blocks that see the most keys (the last queries, when causal) are dealt first.
+struct RowBlock {
+    long long R, r0;                                               // rows per (batch, kv head); the block's first
+    int bh, rows;
+    __device__ __forceinline__ RowBlock(int B, int Hkv, int G, int Tq, int QB) {
+        R = (long long)G * Tq;
+        const int nb = (int)((R + QB - 1) / QB);
+        const int t = (int)(blockIdx.x / (unsigned)(B * Hkv));
+        bh = (int)(blockIdx.x % (unsigned)(B * Hkv));
+        const int rb = nb % G == 0 ? (t % G) * (nb / G) + (nb / G - 1 - t / G) : nb - 1 - t;
+        r0 = (long long)rb * QB;
+        rows = (int)min((long long)QB, R - r0);
+    }
+};
+
+// One row by one warp, key by key over the n keys it sees, as the canonical arithmetic is written: lane = virtual lane, with
+// its DL dims of q, k, v and the accumulator. For rows the tiled phases cannot keep apart (below).
+template <typename T, int DL>
+__device__ __forceinline__ void literal_row(const T* q, const T* k, const T* v, T* out, int n, int64_t sl, float scale, int split) {
+    const int d0 = (threadIdx.x & 31) * DL;
+    float qf[DL], A[DL], M = -INFINITY, L = 0.0f;
+#pragma unroll
+    for (int d = 0; d < DL; ++d) { qf[d] = mul_rn(Cvt<T>::up(q[d0 + d]), scale); A[d] = 0.0f; }
+    for (int j0 = 0; j0 < n; j0 += split) {
+        float m = -INFINITY, l = 0.0f, acc[DL];
+#pragma unroll
+        for (int d = 0; d < DL; ++d) acc[d] = 0.0f;
+        const int j1 = min(n, j0 + split);
+        for (int j = j0; j < j1; ++j) {
+            const T *kr = k + (int64_t)j * sl + d0, *vr = v + (int64_t)j * sl + d0;
+            float s = 0.0f;
+#pragma unroll
+            for (int d = 0; d < DL; ++d) s = fma_rn(qf[d], Cvt<T>::up(kr[d]), s);
+#pragma unroll
+            for (int off = 16; off; off >>= 1) s = add_rn(s, __shfl_xor_sync(0xffffffffu, s, off));
+            const float e = expf_canon(-fabsf(sub_rn(s, m)));
+            const bool rises = s >= m;
+            const float c = rises ? e : 1.0f, p = rises ? 1.0f : e;
+            m = fmaxf(m, s);
+            l = fma_rn(l, c, p);
+#pragma unroll
+            for (int d = 0; d < DL; ++d) acc[d] = fma_rn(acc[d], c, mul_rn(p, Cvt<T>::up(vr[d])));
+        }
+        float c_old, c_new;
+        merge_coeffs(M, L, m, l, c_old, c_new);
+#pragma unroll
+        for (int d = 0; d < DL; ++d) A[d] = merge_acc(A[d], c_old, acc[d], c_new);
+    }
+#pragma unroll
+    for (int d = 0; d < DL; ++d) out[d0 + d] = Cvt<T>::down(div_canon(A[d], L));
+}
+
+// The rows of this CTA that hold NaN in `ms`, by literal_row. Everything is worked out again from the launch's arguments, so
+// that the kernel keeps no register for it through its loops.
+template <typename T, int DL, int TQ>
+__device__ __noinline__ void literal_rows(const float* ms, const T* q, const T* k, const T* v, T* out, int B, int Hkv, int G, int Tq, int L,
+                                          int64_t sb, int64_t sh, int64_t sl, float scale, int split) {
+    constexpr int D = 32 * DL, QB = PF<T, DL, TQ>::QB;
+    const RowBlock w(B, Hkv, G, Tq, QB);
+    for (int row = threadIdx.x >> 5; row < w.rows; row += PF_THREADS / 32) {
+        if (ms[row] == ms[row]) continue;
+        const int64_t at = ((int64_t)w.bh * w.R + w.r0 + row) * D, kv = (int64_t)(w.bh / Hkv) * sb + (int64_t)(w.bh % Hkv) * sh;
+        literal_row<T, DL>(q + at, k + kv, v + kv, out + at, L - Tq + (int)((w.r0 + row) % Tq) + 1, sl, scale, split);
+    }
+}
+
 template <typename T, int DL, int TQ>
 __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) && sizeof(T) == 2 ? 3 : 2) prefill_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ out, int B, int Hkv, int G, int Tq,
@@ -180,15 +244,9 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
     int* const ns = reinterpret_cast<int*>(sm + C::NOFF);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    // Row block of this CTA. Blocks that see the most keys (the last queries, when causal) are dealt first.
-    const long long R = (long long)G * Tq;                         // rows per (batch, kv head)
-    const int nb = (int)((R + QB - 1) / QB);
-    const int t = (int)(blockIdx.x / (unsigned)(B * Hkv));
-    const int bh = (int)(blockIdx.x % (unsigned)(B * Hkv));
-    const int rb = nb % G == 0 ? (t % G) * (nb / G) + (nb / G - 1 - t / G) : nb - 1 - t;
-    const int b = bh / Hkv, hk = bh % Hkv;
-    const long long r0 = (long long)rb * QB;
-    const int rows = (int)min((long long)QB, R - r0);
+    const RowBlock block(B, Hkv, G, Tq, QB);
+    const long long R = block.R, r0 = block.r0;
+    const int bh = block.bh, rows = block.rows, b = bh / Hkv, hk = bh % Hkv;
     const T* const kbase = k + (int64_t)b * lay.sb + (int64_t)hk * lay.sh;
     const T* const vbase = v + (int64_t)b * lay.sb + (int64_t)hk * lay.sh;
     const T* const qbase = q + ((int64_t)bh * R + r0) * D;         // rows of a (batch, kv head) are contiguous in q and out
@@ -228,16 +286,6 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
     // accumulation tile of this thread: rows tq .. tq+3, dims td .. td+7
     constexpr int DG = D / 8;
     const int tq = (tid / DG) * TQ, td = (tid % DG) * 8;
-    // Keys that every row of this warp's tiles sees, and that any of them sees (rows past the end do not count).
-    int seen_all = INT_MAX, seen_any = 0;
-#pragma unroll
-    for (int i = 0; i < TQ; ++i) {
-        const int n = ns[tq + i];
-        if (n > 0) seen_all = min(seen_all, n);
-        seen_any = max(seen_any, n);
-    }
-    seen_all = __reduce_min_sync(0xffffffffu, seen_all);
-    seen_any = __reduce_max_sync(0xffffffffu, seen_any);
     uint64_t acc[TQ][4];
     // merged accumulators of the thread: pairs (2i, 2i+1) of its TQ x 4 at tot[i * PF_THREADS]
     ulonglong2* const tot = reinterpret_cast<ulonglong2*>(sm + C::TOFF) + tid;
@@ -325,8 +373,8 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
                     for (int u = 0; u < RG; ++u) {
                         const float e = expf_canon(-fabsf(sub_rn(s4[u], m4[u])));
                         const bool rises = s4[u] >= m4[u];
-                        c4[u] = rises ? e : 1.0f;                        // of a key the row does not see: never read
-                        p4[u] = rises ? 1.0f : e;
+                        c4[u] = on4[u] && rises ? e : 1.0f;
+                        p4[u] = on4[u] ? (rises ? 1.0f : e) : 0.0f;
                     }
                     st_vec<RG>(ps + key * C::PPITCH + rr, p4);
                     st_vec<RG>(cs + key * C::PPITCH + rr, c4);
@@ -334,10 +382,10 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
                 }
             }
             __syncthreads();
-            // ---- C: accumulation, key by key. A key that a row does not see leaves the row's state alone: folding it in with
-            // weight 0 would turn an infinity or NaN of a later token's value into NaN in this row.
+            // ---- C: accumulation, key by key
             const uint8_t* const vb = vs + buf * KB * C::KROW + td * (int)sizeof(T);
-            auto fold = [&](int i, auto masked) {
+#pragma unroll 8
+            for (int i = 0; i < cnt; ++i) {
                 float p[TQ], c[TQ];
                 ld_vec<TQ>(ps + i * C::PPITCH + tq, p);
                 ld_vec<TQ>(cs + i * C::PPITCH + tq, c);
@@ -345,7 +393,6 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
                 value_pairs<T>(vb + i * C::KROW, v2);
 #pragma unroll
                 for (int iq = 0; iq < TQ; ++iq) {
-                    if (decltype(masked)::value && j + i >= ns[tq + iq]) continue;
                     const uint64_t p2 = ptx::pack2(p[iq], p[iq]), c2 = ptx::pack2(c[iq], c[iq]);
                     l[iq] = fma_rn(l[iq], c[iq], p[iq]);
 #pragma unroll
@@ -353,12 +400,7 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
 #pragma unroll
                     for (int d = 0; d < 4; ++d) acc[iq][d] = ptx::fma2_rn(acc[iq][d], c2, t2[d]);
                 }
-            };
-            const int all = min(cnt, seen_all - j), any = min(cnt, seen_any - j);
-#pragma unroll 8
-            for (int i = 0; i < all; ++i) fold(i, std::false_type{});
-#pragma unroll 1
-            for (int i = max(all, 0); i < any; ++i) fold(i, std::true_type{});
+            }
             buf ^= 1;
         }
         // ---- the split's end: fold it into the running state of every row that saw a key of it
@@ -383,9 +425,11 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
         __syncthreads();                                                 // ms is read above, reset by the next split
     }
 
+    bool poisoned = false;
 #pragma unroll
     for (int iq = 0; iq < TQ; ++iq) {
         if (tq + iq >= rows) continue;
+        bool nan = false;
         T* o = out + ((int64_t)bh * R + r0 + tq + iq) * D + td;
         alignas(16) T w[8];
 #pragma unroll
@@ -393,6 +437,7 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
             float a0, a1;
             const ulonglong2 x = tot[(iq * 2 + d / 2) * PF_THREADS];
             ptx::unpack2((d & 1) ? x.y : x.x, a0, a1);
+            nan |= a0 != a0 || a1 != a1;
             w[2 * d] = Cvt<T>::down(div_canon(a0, Lt[iq]));
             w[2 * d + 1] = Cvt<T>::down(div_canon(a1, Lt[iq]));
         }
@@ -403,7 +448,15 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
 #pragma unroll
             for (int i = 0; i < 8; ++i) o[i] = w[i];
         }
+        if (nan) ms[tq + iq] = NAN;                                      // a running maximum is never NaN
+        poisoned |= nan;
     }
+    // Phase C folds a key that a row does not see into it with weight 0: no change, unless the key's value holds an infinity
+    // or NaN, whose product with 0 stays in the accumulator as NaN to the end. Rows that end with one are computed again
+    // without their unseen keys, so that no later token reaches a row. (Skipping unseen keys in phase C, or looking for such
+    // values there, cost 2-8 % of every launch and up to 39 % where a row block straddles two heads.)
+    if (causal && __syncthreads_or(poisoned))
+        literal_rows<T, DL, TQ>(ms, q, k, v, out, B, Hkv, G, Tq, L, lay.sb, lay.sh, lay.sl, scale, split);
 }
 
 template <typename T, int DL, int TQ>

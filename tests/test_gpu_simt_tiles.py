@@ -33,3 +33,20 @@ def test_element_wise_fetches_bit_exact(bi, M):
     pad = torch.zeros(M, 303)
     pad[:, 1:301] = x
     assert R.bits_of(bi.batch_invariant_matmul(pad.cuda()[:, 1:301], b.cuda())) == want
+
+
+@pytest.mark.parametrize("dt,K,gs", [(torch.float32, 288, 32), (torch.float32, 640, 128), (torch.bfloat16, 288, 32), (torch.float16, 544, 32)])
+@pytest.mark.parametrize("bits", [4, 8])
+def test_packed_pieces_bit_exact(bi, dt, K, gs, bits):
+    """Packed weights the tensor-core path does not take (fp32, or K no multiple of 64): the four codes of a piece, its scale
+    and bias, at the edges of the tiles and of the K groups."""
+    g = torch.Generator().manual_seed(K + bits)
+    N = 131
+    p, s, b = R.quantize_affine(torch.randn(N, K, generator=g) * 0.02, group_size=gs, bits=bits, dtype=dt)
+    wd = R.dequant(p, s, b, group_size=gs, bits=bits, dtype=dt)
+    for M in (1, 9, 17, 33, 70):
+        x = torch.randn(M, K, generator=g).to(dt)
+        want = R.bits_of(R.matmul_f32order(x, wd.T.contiguous()))
+        for path in ("auto", "split", "fused"):
+            got = bi.batch_invariant_quantized_matmul(x.cuda(), p.cuda(), s.cuda(), b.cuda(), group_size=gs, bits=bits, path=path)
+            assert R.bits_of(got) == want, (M, path)

@@ -69,7 +69,10 @@ TcShape tc_auto_shape(int64_t M, int64_t N, int64_t K, bool quant = false) {
 // of partials: 626 against 777 us), up to the partials kept per stream.
 bool simt_auto_split(int64_t M, int64_t K) { return ngroups(K) > 1 && M <= 32; }
 constexpr int64_t SIMT_PARTIAL_MAX = 256 << 20;
-bool simt_split(int64_t M, int64_t N, int64_t K) { return ngroups(K) > 1 && ngroups(K) * M * N * (int64_t)sizeof(float) <= SIMT_PARTIAL_MAX; }
+bool simt_split(int64_t M, int64_t N, int64_t K) {
+    const int64_t G = ngroups(K);
+    return G > 1 && G <= 65535 && G * M * N * (int64_t)sizeof(float) <= SIMT_PARTIAL_MAX;      // a group per block of grid.z
+}
 
 // `path` as the ABI packs it -> kind, flags, forced batch tile, forced staging.
 struct PathArg {

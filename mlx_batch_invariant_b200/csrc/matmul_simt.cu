@@ -431,7 +431,7 @@ struct SimtArgs {
 template <int TM>
 int simt_stream(const SimtArgs& p) {
     const int64_t G = (p.K + GROUP_K - 1) / GROUP_K;
-    if (G > 65535) return fail(BI_ERR_UNSUPPORTED, "matmul (cuda-core path): K=%lld too large", (long long)p.K);
+    if (p.split && G > 65535) return fail(BI_ERR_UNSUPPORTED, "matmul (cuda-core path): K=%lld too large", (long long)p.K);
     dim3 grid((unsigned)((p.N + STREAM_N - 1) / STREAM_N), 1, p.split ? (unsigned)G : 1u);
     constexpr size_t smem = (size_t)STREAM_STAGES * (TM + STREAM_N) * STREAM_PITCH * sizeof(float);
     auto kern = p.split ? simt_stream_kernel<TM, true> : simt_stream_kernel<TM, false>;
@@ -449,7 +449,7 @@ int simt_launch(int tile, const SimtArgs& p) {
         constexpr SimtTile t = SIMT_TILES[I];
         constexpr int bm = t.tm * t.mg, bn = t.tn * t.nl;
         const int64_t G = (p.K + GROUP_K - 1) / GROUP_K, gy = (p.M + bm - 1) / bm;
-        if (gy > 65535 || G > 65535) return fail(BI_ERR_UNSUPPORTED, "matmul (cuda-core path): M=%lld K=%lld too large", (long long)p.M, (long long)p.K);
+        if (gy > 65535 || (p.split && G > 65535)) return fail(BI_ERR_UNSUPPORTED, "matmul (cuda-core path): M=%lld K=%lld too large", (long long)p.M, (long long)p.K);
         dim3 grid((unsigned)((p.N + bn - 1) / bn), (unsigned)gy, p.split ? (unsigned)G : 1u);
         auto kern = p.split ? simt_matmul_kernel<T, t.tm, t.tn, t.mg, t.nl, true, QUANT, VEC> : simt_matmul_kernel<T, t.tm, t.tn, t.mg, t.nl, false, QUANT, VEC>;
         launch_overlapped(kern, grid, dim3(t.mg * t.nl), 0, p.st, static_cast<const T*>(p.a), static_cast<const T*>(p.b), p.qa, p.dst, (int)p.M, (int)p.N,

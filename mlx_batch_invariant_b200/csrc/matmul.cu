@@ -148,7 +148,9 @@ int simt_shape(const char* op, const PathArg& pa, void* ws, size_t ws_bytes, int
     const size_t head = pa.zeroed ? COUNTER_BYTES : 0;
     const size_t need = head + (size_t)ngroups(K) * (size_t)M * (size_t)N * sizeof(float);
     *part = nullptr;
-    if (*split && pa.kind == BI_MATMUL_AUTO && (!ws || ws_bytes < need)) *split = false;   // AUTO: fold in place instead
+    // AUTO folds in place when the workspace does not serve. Beyond the batches whose scratch is promised the workspace is
+    // optional, so a misaligned one is as good as none.
+    if (*split && pa.kind == BI_MATMUL_AUTO && (!ws || ws_bytes < need || (!simt_auto_split(M, K) && !aligned(ws, 16)))) *split = false;
     if (!*split) return BI_OK;
     if (!ws || ws_bytes < need) return fail(BI_ERR_WORKSPACE, "%s: split path needs %zu workspace bytes, got %zu", op, need, ws_bytes);
     if (!aligned(ws, 16)) return fail(BI_ERR_MISALIGNED, "%s: workspace must be 16-byte aligned", op);

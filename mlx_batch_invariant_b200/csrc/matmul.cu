@@ -144,6 +144,7 @@ int tc_shape(const char* op, const PathArg& pa, void* ws, size_t ws_bytes, int64
 
 int simt_shape(const char* op, const PathArg& pa, void* ws, size_t ws_bytes, int64_t M, int64_t N, int64_t K, bool* split,
                float** part) {
+    if (pa.kind == BI_MATMUL_PAIR) return fail(BI_ERR_UNSUPPORTED, "%s: the pair shape is for weights on the tensor-core path", op);
     *split = pa.kind == BI_MATMUL_AUTO ? simt_split(M, N, K) : (pa.kind != BI_MATMUL_FUSED);
     const size_t head = pa.zeroed ? COUNTER_BYTES : 0;
     const size_t need = head + (size_t)ngroups(K) * (size_t)M * (size_t)N * sizeof(float);
@@ -227,6 +228,7 @@ int matmul_impl(const void* a, const void* b, void* out, void* workspace, size_t
     if (rc) return rc;
     if (sink || rope) {      // the fold kernel is the one that pushes / rotates: always the split shape, folded by the second launch
         if (!weight_tc) return fail(BI_ERR_UNSUPPORTED, "bi_matmul_push / bi_matmul_rope: only weights on the tensor-core path");
+        if (pa.kind == BI_MATMUL_PAIR) return fail(BI_ERR_BAD_ARG, "bi_matmul_push / bi_matmul_rope: the pair shape has no fold to push or rotate");
         pa.kind = BI_MATMUL_SPLIT;
     }
     float* part = nullptr;
@@ -307,6 +309,7 @@ int qmm_impl(const void* x, const uint32_t* w, const void* scales, const void* b
     if (rc) return rc;
     if (sink || rope) {
         if (!weight_tc) return fail(BI_ERR_UNSUPPORTED, "bi_qmm_push / bi_qmm_rope: only weights on the tensor-core path");
+        if (pa.kind == BI_MATMUL_PAIR) return fail(BI_ERR_BAD_ARG, "bi_qmm_push / bi_qmm_rope: the pair shape has no fold to push or rotate");
         pa.kind = BI_MATMUL_SPLIT;
     }
     float* part = nullptr;

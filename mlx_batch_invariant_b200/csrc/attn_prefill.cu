@@ -27,6 +27,7 @@ namespace bi {
 namespace {
 
 constexpr int PF_THREADS = 128;
+constexpr int PF_SMEM_MAX = 227 * 1024;                           // what a CTA may have
 
 template <typename T, int DL, int TQ> struct PF {
     static constexpr int D = 32 * DL;
@@ -463,6 +464,7 @@ template <typename T, int DL, int TQ>
 int launch_prefill_tq(const void* q, const void* k, const void* v, void* out, int64_t B, int64_t Hq, int64_t Hkv,
                    int64_t Tq, int64_t L, const KvLayout& lay, float scale, int causal, int split, cudaStream_t st) {
     using C = PF<T, DL, TQ>;
+    static_assert(C::SMEM <= PF_SMEM_MAX, "more shared memory than a CTA may have");
     const int64_t G = Hq / Hkv;
     const int64_t blocks = B * Hkv * ((G * Tq + C::QB - 1) / C::QB);
     if (blocks > 0x7fffffffLL) return fail(BI_ERR_UNSUPPORTED, "bi_attn_prefill: grid too large");
@@ -489,10 +491,13 @@ int launch_prefill(const void* q, const void* k, const void* v, void* out, int64
                    int64_t Tq, int64_t L, const KvLayout& lay, float scale, int causal, int split, cudaStream_t st) {
     // Rows per thread: four give every loaded operand the most use and win while at least two CTAs per SM are left
     // (32 heads x 2048 tokens: 1231 us with four, 1420 with two, 1908 with one); with fewer CTAs the block's serial
-    // chain is what counts and shorter row blocks are faster (8 heads x 16 queries over 1000 keys: 119 / 75 / 56 us).
+    // chain is what counts and shorter row blocks are faster (8 heads x 16 queries over 1000 keys: 119 / 75 / 56 us). Four
+    // rows of fp32 with 256 dims would take 240 KB of shared memory.
     const int64_t rows = (Hq / Hkv) * Tq, sms = sm_count();
     auto ctas = [&](int qb) { return B * Hkv * ((rows + qb - 1) / qb); };
-    if (ctas(PF<T, DL, 4>::QB) >= 2 * sms) return launch_prefill_tq<T, DL, 4>(q, k, v, out, B, Hq, Hkv, Tq, L, lay, scale, causal, split, st);
+    if constexpr (PF<T, DL, 4>::SMEM <= PF_SMEM_MAX) {
+        if (ctas(PF<T, DL, 4>::QB) >= 2 * sms) return launch_prefill_tq<T, DL, 4>(q, k, v, out, B, Hq, Hkv, Tq, L, lay, scale, causal, split, st);
+    }
     if (ctas(PF<T, DL, 2>::QB) >= sms / 2) return launch_prefill_tq<T, DL, 2>(q, k, v, out, B, Hq, Hkv, Tq, L, lay, scale, causal, split, st);
     return launch_prefill_tq<T, DL, 1>(q, k, v, out, B, Hq, Hkv, Tq, L, lay, scale, causal, split, st);
 }

@@ -1,5 +1,6 @@
 """Prefill attention at the edges of its tiling: row blocks (TQ * 1024 / D rows of one kv head, rows running over the
-heads of the group), 32- or 64-key blocks inside the splits, and every rows-per-thread variant the launch rule picks."""
+heads of the group), 32- or 64-key blocks inside the splits, every rows-per-thread variant the launch rule picks, and
+values that are not finite behind the causal mask."""
 
 import pytest
 import torch
@@ -52,11 +53,20 @@ ROWS_PER_THREAD = [(32, 1, 1), (32, 2, 10), (32, 4, 74), (64, 1, 1), (64, 2, 7),
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("D,rows,B", ROWS_PER_THREAD)
+def test_every_number_of_rows_per_thread(bi, dt, D, rows, B):
+    """(fp32 with 256 dims has no room for four rows and stays at two.)"""
+    g = torch.Generator().manual_seed(D * 10 + rows)
+    q, k, v = (torch.randn(B, h, n, D, generator=g).to(dt) for h, n in ((8, 45), (4, 77), (4, 77)))
+    for causal in (True, False):
+        got = bi.batch_invariant_prefill_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5, causal=causal, split_size=32)
+        assert R.bits_of(got) == R.bits_of(R.attn_prefill(q, k, v, scale=D ** -0.5, causal=causal, split_size=32))
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("D,rows,B", ROWS_PER_THREAD)
 def test_later_tokens_never_reach_a_row(bi, dt, D, rows, B):
     """Infinities and NaN in a later token's key and value: a row that does not see the token keeps the bits it has
     without them and those of the prefix run alone, in every row block and at every number of rows per thread."""
-    if dt == torch.float32 and D == 256:
-        B = min(B, 2)
     L, T, split = 77, 45, 32
     g = torch.Generator().manual_seed(D + rows)
     q, k, v = (torch.randn(B, h, n, D, generator=g).to(dt).cuda() for h, n in ((8, T), (4, L), (4, L)))

@@ -935,7 +935,7 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
         if (dev_ < 0 || dev_ >= 64) dev_ = 0;                                                                           \
         if (!attr_set[dev_]) {                                                                                          \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (NWV) * KLCfg::WARP_BYTES); \
-            if (e != cudaSuccess) return fail(BI_ERR_CUDA, "bi_attn_decode smem attr: %s", cudaGetErrorString(e));      \
+            if (e != cudaSuccess) return fail_cuda("bi_attn_decode smem attr", e);      \
             attr_set[dev_] = true;                                                                                      \
         }                                                                                                               \
         launch_overlapped(kern, dim3((unsigned)ctas), dim3(32 * (NWV)), (size_t)((NWV) * KLCfg::WARP_BYTES), st, qp, kp, vp, kv_lens, pm, pl, pacc, \
@@ -985,7 +985,7 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
         if (dev_ < 0 || dev_ >= 64) dev_ = 0;                                                                           \
         if (!attr_set[dev_] && MW * CW::WARP_BYTES > 40 * 1024) {                                                       \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MW * CW::WARP_BYTES); \
-            if (e != cudaSuccess) return fail(BI_ERR_CUDA, "bi_attn_decode smem attr: %s", cudaGetErrorString(e));      \
+            if (e != cudaSuccess) return fail_cuda("bi_attn_decode smem attr", e);      \
             attr_set[dev_] = true;                                                                                      \
         }                                                                                                               \
         launch_overlapped(kern, dim3((unsigned)blocksw), dim3(32 * wpc), smem_w, st, qp, kp, vp, kv_lens, pm, pl, pacc, (int)B, (int)Hq, (int)Hkv, \
@@ -1008,7 +1008,7 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
         auto kern = decode_stream_kernel<T, DL, GUV>;                                                            \
         if (C::SMEM_BYTES > 40 * 1024) { /* static shared memory counts toward the 48 KB default too */          \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES); \
-            if (e != cudaSuccess) return fail(BI_ERR_CUDA, "bi_attn_decode smem attr: %s", cudaGetErrorString(e)); \
+            if (e != cudaSuccess) return fail_cuda("bi_attn_decode smem attr", e); \
         }                                                                                                        \
         launch_overlapped(kern, dim3((unsigned)blocks2), dim3(32 * DEC2_WARPS), C::SMEM_BYTES, st, qp, kp, vp, kv_lens, pm, pl, pacc, (int)B, \
                                                                           (int)Hq, (int)Hkv, (int)L, lay, scale, split, nsplit, nchunk); \

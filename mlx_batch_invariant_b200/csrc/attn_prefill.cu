@@ -477,7 +477,7 @@ int launch_prefill_tq(const void* q, const void* k, const void* v, void* out, in
     if (dev < 0 || dev >= 64) dev = 0;
     if (!attr_set[dev]) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-        if (e != cudaSuccess) return fail(BI_ERR_CUDA, "bi_attn_prefill smem attr: %s", cudaGetErrorString(e));
+        if (e != cudaSuccess) return fail_cuda("bi_attn_prefill smem attr", e);
         attr_set[dev] = true;
     }
     kern<<<(unsigned)blocks, PF_THREADS, C::SMEM, st>>>(

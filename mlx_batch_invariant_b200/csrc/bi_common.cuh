@@ -23,6 +23,13 @@ inline int check_launch(const char* what) {
     return BI_OK;
 }
 
+// A runtime call other than a launch failed. Its error also stays in the slot that check_launch() reads, where the next
+// launch would report it as its own: taken out here.
+inline int fail_cuda(const char* what, cudaError_t e) {
+    cudaGetLastError();
+    return fail(BI_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+}
+
 // Defined in abi.cu: whether kernels are launched with programmatic dependent launch (BI_PDL=1 turns it on).
 bool pdl_enabled();
 

@@ -355,7 +355,7 @@ int launch_pair_t(const CUtensorMap& mw, const CUtensorMap& mx, const PairParams
     if (dev < 0 || dev >= 64) dev = 0;
     if (!attr_done[dev]) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_LIMIT);
-        if (e != cudaSuccess) return fail(BI_ERR_CUDA, "matmul smem attr: %s", cudaGetErrorString(e));
+        if (e != cudaSuccess) return fail_cuda("matmul smem attr", e);
         attr_done[dev] = true;
     }
     const int clusters = sm_count() / 2;

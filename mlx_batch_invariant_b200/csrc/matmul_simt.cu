@@ -436,7 +436,7 @@ int simt_stream(const SimtArgs& p) {
     constexpr size_t smem = (size_t)STREAM_STAGES * (TM + STREAM_N) * STREAM_PITCH * sizeof(float);
     auto kern = p.split ? simt_stream_kernel<TM, true> : simt_stream_kernel<TM, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return fail(BI_ERR_CUDA, "matmul (cuda-core path) smem attr: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return fail_cuda("matmul (cuda-core path) smem attr", e);
     launch_overlapped(kern, grid, dim3(STREAM_N), smem, p.st, static_cast<const float*>(p.a), static_cast<const float*>(p.b), p.qa,
                       static_cast<float*>(p.dst), (int)p.M, (int)p.N, (int)p.K, p.a_sm, p.b_sn);
     return check_launch("matmul (cuda-core path)");

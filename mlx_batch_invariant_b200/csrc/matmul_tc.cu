@@ -896,7 +896,7 @@ int launch_t(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, cuda
     if (dev < 0 || dev >= 64) dev = 0;
     if (!attr_done[dev]) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
-        if (e != cudaSuccess) return fail(BI_ERR_CUDA, "matmul smem attr: %s", cudaGetErrorString(e));
+        if (e != cudaSuccess) return fail_cuda("matmul smem attr", e);
         attr_done[dev] = true;
     }
     // Units go to CTAs in equal contiguous shares. With few units per CTA an uneven share costs a

@@ -350,8 +350,7 @@ int launch(const void* x, const void* delta, const void* w, void* sum_out, void*
         if (smem > 48 * 1024) {                                                                     \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                                  (int)smem);                                        \
-            if (e != cudaSuccess) return fail(BI_ERR_CUDA, "rms_norm smem attr: %s",               \
-                                              cudaGetErrorString(e));                               \
+            if (e != cudaSuccess) return fail_cuda("rms_norm smem attr", e);                               \
         }                                                                                           \
         launch_overlapped(kern, grid, block, smem, st, xp, dp, wp, sp, op, (int)D, eps, aw);                       \
     } while (0)

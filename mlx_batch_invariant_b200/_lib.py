@@ -168,23 +168,34 @@ def status_word(device: torch.device) -> torch.Tensor:
     return t
 
 
-# Matmul workspaces: one per (device, stream), kept between calls. Its first COUNTER_BYTES are the per-tile
-# arrival counters of the split path's in-kernel fold; they are zero between calls (the kernel leaves them so),
-# which is what the WS_ZEROED flag promises the library. Calls on one stream are ordered, so they can share it.
+# Matmul workspaces of decode-sized calls: one per (device, stream), kept between calls. Its first COUNTER_BYTES are
+# the per-tile arrival counters of the split path's in-kernel fold; they are zero between calls (the kernel leaves them
+# so), which is what the WS_ZEROED flag promises the library. Calls on one stream are ordered, so they can share it.
 _workspaces: dict[tuple[int, int], torch.Tensor] = {}
+KEPT_BYTES = 64 << 20             # the largest workspace that is kept: the partials of 64 rows of a 14336 -> 4096 layer are 59 MB
 
 
-def matmul_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """A zero-headed workspace of at least `nbytes` for the current stream of `device`."""
+def matmul_workspace(device: torch.device, nbytes: int, counters: bool = False) -> tuple[torch.Tensor, bool]:
+    """A workspace of at least `nbytes` for a call on the current stream of `device`, the current device, and whether its
+    head is zero (always when `counters` asks for it).
+
+    Larger workspaces than KEPT_BYTES, and all that a capture records, are the call's own: the allocator hands the memory
+    on in stream order, and inside a capture takes it from the graph's pool. A kept workspace in a graph would be freed
+    under the graph as soon as a larger call replaced it."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
+    need = max(nbytes, COUNTER_BYTES)
+    if need > KEPT_BYTES or torch._C._cuda_isCurrentStreamCapturing():
+        ws = torch.empty(need, dtype=torch.uint8, device=torch.device("cuda", idx))
+        if counters:
+            ws[:COUNTER_BYTES].zero_()
+        return ws, counters
     key = (idx, torch._C._cuda_getCurrentRawStream(idx))
     ws = _workspaces.get(key)
-    need = max(nbytes, COUNTER_BYTES)
     if ws is None or ws.numel() < need:
         ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=torch.device("cuda", idx))
-        ws[:COUNTER_BYTES].zero_()       # only the counters have to start at zero (and a capture records only this small fill)
+        ws[:COUNTER_BYTES].zero_()       # only the counters have to start at zero
         _workspaces[key] = ws
-    return ws
+    return ws, True
 
 
 def check_device_status(device: torch.device | None = None) -> None:

@@ -22,15 +22,17 @@ _PATHS = {"auto": _lib.PATH_AUTO, "split": _lib.PATH_SPLIT, "fused": _lib.PATH_F
 
 
 def _launch_shape(path: str, batch_tile: int | None, M: int, N: int, K: int, ws_bytes_auto: int, dev: torch.device, pair_bytes: int = 0):
-    """(path word, workspace tensor or None, workspace bytes) for a call. The workspace is the stream's
-    persistent one, whose head holds the zeroed arrival counters of the in-kernel fold."""
+    """(path word, workspace tensor or None, workspace bytes) for a call. A workspace that the stream keeps has the
+    zeroed arrival counters of the in-kernel fold at its head."""
     if path == "pair" and batch_tile and (batch_tile % 32 or not 32 <= batch_tile <= 256):
         raise _lib.KernelError(_lib.BI_ERR_BAD_ARG, f"batch tile {batch_tile} of a pair (a multiple of 32 up to 256)")
     G = (K + GROUP_K - 1) // GROUP_K
     nbytes = ws_bytes_auto if path in ("auto", "fused") else pair_bytes if path == "pair" else _lib.COUNTER_BYTES + G * M * N * 4
-    word = _PATHS[path] | _lib.WS_ZEROED | (_lib.batch_tile(batch_tile // 2 if path == "pair" else batch_tile) if batch_tile else 0)
-    ws = _lib.matmul_workspace(dev, nbytes) if nbytes else None
-    return word, ws, (ws.numel() if ws is not None else 0)
+    word = _PATHS[path] | (_lib.batch_tile(batch_tile // 2 if path == "pair" else batch_tile) if batch_tile else 0)
+    if not nbytes:
+        return word, None, 0
+    ws, zeroed = _lib.matmul_workspace(dev, nbytes, path == "fold")
+    return word | _lib.WS_ZEROED if zeroed else word, ws, ws.numel()
 
 
 def _weight_is_tensor_core(b: torch.Tensor, K: int) -> bool:

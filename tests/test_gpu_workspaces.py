@@ -1,0 +1,61 @@
+"""Who owns the matmuls' scratch: a captured graph its own, large calls theirs, decode-sized calls one per stream."""
+
+import pytest
+import torch
+
+from mlx_batch_invariant_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _fp32(m, n, k, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn(m, k, device="cuda", generator=g), torch.randn(n, k, device="cuda", generator=g) / k ** 0.5
+
+
+def test_a_graph_keeps_its_scratch_when_a_larger_call_follows(bi):
+    """Capture on an explicit stream that has been used before, then a larger call on that stream, then tensors that would
+    land in freed scratch: a replay gives the captured call's bits and leaves those tensors alone."""
+    s = torch.cuda.Stream()
+    x, w = _fp32(8, 4096, 4096, 1)
+    big_x, big_w = _fp32(30, 4096, 14336, 2)
+    want = bi.batch_invariant_matmul(x, w.T, path="fused")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        bi.batch_invariant_matmul(x, w.T)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            out = bi.batch_invariant_matmul(x, w.T)
+        bi.batch_invariant_matmul(big_x, big_w.T)
+        others = [torch.full((1 << 20,), 7, dtype=torch.uint8, device="cuda") for _ in range(64)]
+        out.zero_()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    assert all(bool((t == 7).all()) for t in others)
+
+
+def test_large_scratch_is_not_kept(bi):
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        x, w = _fp32(300, 8192, 4096, 3)                            # 157 MB of partials
+        got = bi.batch_invariant_matmul(x, w.T)
+        assert torch.equal(got, bi.batch_invariant_matmul(x, w.T, path="fused"))
+    torch.cuda.synchronize()
+    assert max((ws.numel() for ws in _lib._workspaces.values()), default=0) <= _lib.KEPT_BYTES
+
+
+def test_the_fold_inside_a_capture_finds_its_counters_zero(bi):
+    x = torch.randn(16, 4096, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(4096, 4096, device="cuda") / 64).to(torch.bfloat16)
+    want = bi.batch_invariant_matmul(x, w.T, path="split")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = bi.batch_invariant_matmul(x, w.T, path="fold")
+    for _ in range(3):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    bi.check_device_status()

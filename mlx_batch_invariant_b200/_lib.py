@@ -168,10 +168,26 @@ def status_word(device: torch.device) -> torch.Tensor:
     return t
 
 
-# Matmul workspaces of decode-sized calls: one per (device, stream), kept between calls. Its first COUNTER_BYTES are
-# the per-tile arrival counters of the split path's in-kernel fold; they are zero between calls (the kernel leaves them
-# so), which is what the WS_ZEROED flag promises the library. Calls on one stream are ordered, so they can share it.
-_workspaces: dict[tuple[int, int], torch.Tensor] = {}
+# Matmul workspaces of decode-sized calls: one per thread, device and stream, kept between calls. Its first COUNTER_BYTES
+# are the per-tile arrival counters of the split path's in-kernel fold; they are zero between calls (the kernel leaves them
+# so), which is what the WS_ZEROED flag promises the library. A thread's calls on one stream are ordered, so they can share
+# it; the two launches of a split call can lie on either side of another thread's. A thread's workspaces go with the thread.
+class _Workspaces(threading.local):
+    epoch = 0                     # of all threads: a new one drops every workspace
+
+    def __init__(self):
+        self.seen, self.by_stream = _Workspaces.epoch, {}
+
+    def current(self) -> dict[tuple[int, int], torch.Tensor]:
+        if self.seen != _Workspaces.epoch:
+            self.seen, self.by_stream = _Workspaces.epoch, {}
+        return self.by_stream
+
+    def values(self):
+        return self.current().values()
+
+
+_workspaces = _Workspaces()
 KEPT_BYTES = 64 << 20             # the largest workspace that is kept: the partials of 64 rows of a 14336 -> 4096 layer are 59 MB
 
 
@@ -190,11 +206,12 @@ def matmul_workspace(device: torch.device, nbytes: int, counters: bool = False) 
             ws[:COUNTER_BYTES].zero_()
         return ws, counters
     key = (idx, torch._C._cuda_getCurrentRawStream(idx))
-    ws = _workspaces.get(key)
+    kept = _workspaces.current()
+    ws = kept.get(key)
     if ws is None or ws.numel() < need:
         ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=torch.device("cuda", idx))
         ws[:COUNTER_BYTES].zero_()       # only the counters have to start at zero
-        _workspaces[key] = ws
+        kept[key] = ws
     return ws, True
 
 
@@ -207,5 +224,5 @@ def check_device_status(device: torch.device | None = None) -> None:
     if code != BI_OK:
         msg = last_error()
         word.zero_()
-        _workspaces.clear()          # a kernel that gave up may have left arrival counters behind
+        _Workspaces.epoch += 1       # a kernel that gave up may have left arrival counters behind
         raise KernelError(code, msg)

@@ -1,5 +1,7 @@
 """Who owns the matmuls' scratch: a captured graph its own, large calls theirs, decode-sized calls one per stream."""
 
+import threading
+
 import pytest
 import torch
 
@@ -58,4 +60,36 @@ def test_the_fold_inside_a_capture_finds_its_counters_zero(bi):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, want)
+    bi.check_device_status()
+
+
+def test_threads_on_one_stream_do_not_share_scratch(bi):
+    """A split call is two launches; another thread's may lie between them on the same stream."""
+    kept = {}
+
+    def call(name):
+        kept[name], zeroed = _lib.matmul_workspace(torch.device("cuda", 0), 1 << 21)
+        assert zeroed and _lib.matmul_workspace(torch.device("cuda", 0), 1 << 20)[0] is kept[name]
+
+    threads = [threading.Thread(target=call, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+        t.join()
+    call("here")
+    assert len({ws.data_ptr() for ws in kept.values()}) == 4
+
+
+def test_a_wait_that_ran_out_drops_the_scratch_of_every_thread(bi):
+    before = _lib.matmul_workspace(torch.device("cuda", 0), 1 << 20)[0]
+    word = _lib.status_word(torch.device("cuda", 0))
+    word.fill_(0x10000)
+
+    def check():
+        with pytest.raises(_lib.KernelError):
+            bi.check_device_status()
+
+    t = threading.Thread(target=check)
+    t.start()
+    t.join()
+    assert _lib.matmul_workspace(torch.device("cuda", 0), 1 << 20)[0] is not before
     bi.check_device_status()

@@ -2,6 +2,7 @@
 // choice between the tensor-core and the CUDA-core path (a property of the
 // weight, never of the batch) and between the split and fused launch shapes (a
 // function of M that moves no rounding).
+#include <algorithm>
 #include "bi_common.cuh"
 #include "matmul_internal.cuh"
 
@@ -47,14 +48,19 @@ constexpr int64_t PAIR_QUANT_ELEMS = 128 << 20;      // largest quantized weight
 // (0.41 / 0.53 / 0.81). A pair: 0.29 + 0.0012 bm (bm = 96 / 128 / 256: 0.41 / 0.44 / 0.60) for 256 weight rows, and with
 // packed weights a pass that unpacks them first (0.45 us per million). The pair's taller tiles win from about 300 rows on;
 // where few tiles fill only part of a wave (small layers, short batches) one SM per tile keeps more SMs busy. Sizes
-// whose one-SM shape splits K keep it.
-constexpr int64_t PAIR_BM_MAX = 256, PAIR_BM_STEP = 32;
+// whose one-SM shape splits K keep it. Two limits, from runs over weights that are not in L2: up to 96 rows of a dense
+// batch the pair was nowhere faster (65 rows of 4096 -> 14336 / 28672: 38.9 / 70.7 against 31.7 / 55.3 us; 96 rows of
+// 14336 -> 4096: 88 against 78 us); and over a long K the packed one-SM kernel has a dearer start and cheaper steps, 10 us
+// and 0.27 + 0.003 bm (200 rows of 14336 -> 4096: 4 bits 113, 8 bits 105 us; pairs 114 and 116 us).
+constexpr int64_t PAIR_BM_MAX = 256, PAIR_BM_STEP = 32, PAIR_M_MIN = 97;
 TcShape tc_auto_shape(int64_t M, int64_t N, int64_t K, bool quant = false) {
     TcShape sh = tc_one_sm_shape(M, N, K, quant);
-    if (sh.split || M <= 64 || (quant && N * K > PAIR_QUANT_ELEMS)) return sh;
+    if (sh.split || M <= 64 || (quant ? N * K > PAIR_QUANT_ELEMS : M < PAIR_M_MIN)) return sh;
     const int64_t sms = sm_count(), pairs = sms / 2, steps = (K + 63) / 64;
     auto waves = [](int64_t units, int64_t slots) { return (double)((units + slots - 1) / slots); };
-    const double one = 4.0 + waves((N + 127) / 128 * ((M + sh.bm - 1) / sh.bm), sms) * steps * (quant ? 0.28 + 0.0039 * sh.bm : 0.17 + 0.0023 * sh.bm);
+    const double one_steps = waves((N + 127) / 128 * ((M + sh.bm - 1) / sh.bm), sms) * steps;
+    const double one = quant ? std::min(4.0 + one_steps * (0.28 + 0.0039 * sh.bm), 10.0 + one_steps * (0.27 + 0.003 * sh.bm))
+                             : 4.0 + one_steps * (0.17 + 0.0023 * sh.bm);
     double best = 0.95 * one;
     for (int64_t bm = PAIR_BM_STEP; bm <= PAIR_BM_MAX; bm += PAIR_BM_STEP) {
         const double cost = 5.0 + (quant ? 2.0 + 0.45e-6 * (double)(N * K) : 0.0) +

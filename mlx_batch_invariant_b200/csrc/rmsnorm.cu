@@ -169,7 +169,8 @@ __global__ void __launch_bounds__(TG) rms_norm_kernel(const T* x, const T* __res
 // holds (it keeps the half its lane bit names and adds its partner's), 16 and 8 add whole lanes, 4, 2, 1 meet over the
 // same three lane bits -- the canonical pairs, whose order inside an add is free.
 // What bounds it: memory, with 8 KB in flight per warp and no barrier. The CTA per row above spends a row's time on
-// load, five barriers and store in series. bf16 4093 x 4096: 18.0 -> 14.1 us, 4093 x 896: 14.9 -> 6.7 us.
+// load, five barriers and store in series. Rows that are not in L2: bf16 4093 x 4096 19.3 -> 17.8 us, 8192 x 4096
+// 36.8 -> 29.3 us, 4093 x 896 15.0 -> 7.3 us.
 constexpr int WARP_ROWS = 4;
 template <typename T> struct WarpRow { static constexpr int MAX = sizeof(T) == 2 ? 4096 : 1024; };   // longest row kept in registers
 template <typename T, bool HAS_W>
@@ -332,11 +333,14 @@ int launch(const void* x, const void* delta, const void* w, void* sum_out, void*
     const T* wp = static_cast<const T*>(w);
     T* sp = static_cast<T*>(sum_out);
     T* op = static_cast<T*>(out);
-    // A warp per row once there are rows enough to fill the SMs with one warp each: rows of up to 4 KB from 1024 rows on
-    // (bf16 896: 592 rows 3.4 us either way, 1024 rows 5.1 -> 3.6 us; fp32 896: 4.9 -> 3.9 us), rows of 8 KB from 2048 on
-    // (bf16 4096: 1024 rows 7.3 against 8.0 us, 2048 rows 10.5 -> 8.6 us). fp32 rows of 16 KB leave too few warps in flight
-    // (4093 x 4096: 24.8 against 30.0 us), and with the residual's second stream the CTA per row is not slower.
-    if (staged && !delta && D % 8 == 0 && D <= WarpRow<T>::MAX && (!w || aligned(w, 16)) && rows >= (row_bytes <= 4096 ? 1024 : 2048)) {
+    // A warp per row once there are rows enough for it, by times over rows that are not in L2: rows of up to 4 KB from 1024
+    // on (bf16 896: 5.2 -> 4.1 us; fp32 896: 5.7 -> 4.1 us), of up to 6 KB from 2048 on (bf16 3072: 10.2 -> 9.0 us, 1024 rows
+    // 6.8 us either way). Rows of 8 KB fill the SMs 2368 at a time, and a second wave that is nearly empty costs more than the
+    // warps gain (bf16 4096: 2048 rows 11.3 against 11.4 us, 3000 rows 14.9 against 16.3 us, 3600 rows 17.2 against 17.3 us):
+    // from 3800 on (17.9 -> 17.2 us). fp32 rows of 16 KB leave too few warps in flight (4093 x 4096: 24.8 against 30.0 us),
+    // and with the residual's second stream the CTA per row is not slower.
+    const int64_t warp_rows = row_bytes <= 4096 ? 1024 : (row_bytes <= 6144 ? 2048 : 3800);
+    if (staged && !delta && D % 8 == 0 && D <= WarpRow<T>::MAX && (!w || aligned(w, 16)) && rows >= warp_rows) {
         const dim3 wgrid((unsigned)((rows + WARP_ROWS - 1) / WARP_ROWS)), wblock(32 * WARP_ROWS);
         auto kern = w ? rms_norm_warp_kernel<T, true> : rms_norm_warp_kernel<T, false>;
         launch_overlapped(kern, wgrid, wblock, 0, st, xp, wp, op, (long long)rows, (int)D, eps);

@@ -9,7 +9,7 @@
 namespace bi {
 namespace {
 
-constexpr int64_t SPLIT_M_MAX = 64;             // up to here the CUDA-core path may split; the tensor-core path always may
+constexpr int64_t SPLIT_M_MAX = 64;             // the tensor-core path: up to here the partials may be of any size
 constexpr int64_t SPLIT_PARTIAL_MAX = 80 << 20;  // beyond 64 rows: only while the fp32 partials stay L2-sized
 constexpr int64_t FOLD_M_MAX = 0;               // AUTO never folds in the kernel: the fence / count / read-back chain of every unit measured slower than the second launch (M = 1: 16.4 us against 12.6 us)
 constexpr size_t COUNTER_BYTES = BI_MATMUL_COUNTER_BYTES;
@@ -70,14 +70,20 @@ TcShape tc_auto_shape(int64_t M, int64_t N, int64_t K, bool quant = false) {
     return sh;
 }
 // The scratch bi_matmul_workspace_bytes() promises the CUDA-core path (reference rule: M <= 32 and more than one group).
-// With more (bi_matmul_scratch_bytes) AUTO splits at any M: the split shape has G times the CTAs and no running totals in
-// registers, and won at every measured size (M = 100, 4096 x 4096: 93 against 200 us fused; M = 256, 14336 x 4096 with 235 MB
-// of partials: 626 against 777 us), up to the partials kept per stream.
+// With more (bi_matmul_scratch_bytes) AUTO splits larger batches too: the split shape has G times the CTAs and no running
+// totals in registers (M = 100, 4096 x 4096: 94 against 279 us fused; M = 256, 14336 x 4096: 629 against 790 us). It pays
+// for that with a round trip of the partials and a launch, and is not taken where that was the slower side: K below two
+// whole groups (M = 256, K = 300, N = 4096: 24 against 19 us); more than about three waves of fused tiles, which keep the SMs
+// busy anyway (M = 2000, N = 4096: K = 512 184 against 172 us, K = 2048 712 against 669 us); two groups of tiles that fill
+// half a wave to a whole one (M = 100, K = 512, N = 14336: 56 against 53 us).
 bool simt_auto_split(int64_t M, int64_t K) { return ngroups(K) > 1 && M <= 32; }
 constexpr int64_t SIMT_PARTIAL_MAX = 256 << 20;
 bool simt_split(int64_t M, int64_t N, int64_t K) {
     const int64_t G = ngroups(K);
-    return G > 1 && G <= 65535 && G * M * N * (int64_t)sizeof(float) <= SIMT_PARTIAL_MAX;      // a group per block of grid.z
+    if (G <= 1 || G > 65535 || G * M * N * (int64_t)sizeof(float) > SIMT_PARTIAL_MAX) return false;      // a group per block of grid.z
+    if (simt_auto_split(M, K)) return true;
+    const double waves = simt_waves(M, N);
+    return K >= 2 * GROUP_K && waves <= 3.25 && !(G == 2 && waves > 0.5 && waves <= 1.0);
 }
 
 // `path` as the ABI packs it -> kind, flags, forced batch tile, forced staging.

@@ -30,6 +30,8 @@ struct RopeSink {
 int launch_combine_rope(const float* part, int G, int64_t MN, int dtype, cudaStream_t st, const RopeSink& rope);
 
 // CUDA-core path (fp32 inputs, or weights TMA cannot address).
+// Waves of its fused tiles at M x N outputs: tiles over the CTAs that are resident at one time.
+double simt_waves(int64_t M, int64_t N);
 int launch_simt_matmul(const void* a, const void* b, void* out, float* part, int64_t M, int64_t N, int64_t K,
                        int64_t a_sm, int64_t a_sk, int64_t b_sk, int64_t b_sn, int dtype, bool split,
                        cudaStream_t st, const void* bias = nullptr);
@@ -57,8 +59,9 @@ bool tc_matmul_supported(const void* x, int64_t x_ld, const void* w, int64_t w_l
 //   pair      tiles of 256 weight rows x bm batch rows (a multiple of 32, at most 256) on pairs of SMs, folding in
 //             registers (matmul_pair.cu); split, counters and stage do not apply
 //   await     the activation is the destination of a peer gather whose arrival nobody has waited for yet: the
-//             kernel starts streaming weights at once and reads the activation only after every peer's flag
-//             has reached *epoch (bounded wait); flags == nullptr -> nothing to wait for
+//             kernel reads it only after every peer's flag has reached *epoch (bounded wait). The one-SM kernel fills
+//             its ring with weight tiles first, the pair kernel (prompt-sized batches) loads nothing before the flags;
+//             flags == nullptr -> nothing to wait for
 struct Await {
     const uint32_t* flags;   // this rank's flag array, one word per rank
     const uint32_t* epoch;   // the gather's epoch, in device memory

@@ -477,6 +477,12 @@ int simt_t(const void* a, const void* b, const QuantArgs& qa, void* out, float* 
 
 }  // namespace
 
+double simt_waves(int64_t M, int64_t N) {
+    const SimtTile& t = SIMT_TILES[simt_tile(M)];
+    const int64_t bm = t.tm * t.mg, bn = t.tn * t.nl, resident = sm_count() * (256 / (t.mg * t.nl));   // launch bounds: 256 threads an SM
+    return (double)((M + bm - 1) / bm * ((N + bn - 1) / bn)) / (double)resident;
+}
+
 int launch_combine_rope(const float* part, int G, int64_t MN, int dtype, cudaStream_t st, const RopeSink& rope) {
     if (rope.D > 256 || 256 % rope.D != 0) return fail(BI_ERR_UNSUPPORTED, "matmul + rope: head_dim %d (must divide 256)", rope.D);
     const int64_t blocks = (MN + 255) / 256;

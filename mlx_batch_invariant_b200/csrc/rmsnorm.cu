@@ -17,6 +17,7 @@
 // elements there, results are written back in place and leave with 16-byte
 // stores. Rows too long for shared memory, or not 16-byte aligned, take the
 // same arithmetic straight from global memory.
+#include <type_traits>
 #include "bi_common.cuh"
 #include "bi_ptx.cuh"
 
@@ -335,12 +336,14 @@ int launch(const void* x, const void* delta, const void* w, void* sum_out, void*
     T* op = static_cast<T*>(out);
     // A warp per row once there are rows enough for it, by times over rows that are not in L2: rows of up to 4 KB from 1024
     // on (bf16 896: 5.2 -> 4.1 us; fp32 896: 5.7 -> 4.1 us), of up to 6 KB from 2048 on (bf16 3072: 10.2 -> 9.0 us, 1024 rows
-    // 6.8 us either way). Rows of 8 KB fill the SMs 2368 at a time, and a second wave that is nearly empty costs more than the
-    // warps gain (bf16 4096: 2048 rows 11.3 against 11.4 us, 3000 rows 14.9 against 16.3 us, 3600 rows 17.2 against 17.3 us):
-    // from 3800 on (17.9 -> 17.2 us). fp32 rows of 16 KB leave too few warps in flight (4093 x 4096: 24.8 against 30.0 us),
-    // and with the residual's second stream the CTA per row is not slower.
-    const int64_t warp_rows = row_bytes <= 4096 ? 1024 : (row_bytes <= 6144 ? 2048 : 3800);
-    if (staged && !delta && D % 8 == 0 && D <= WarpRow<T>::MAX && (!w || aligned(w, 16)) && rows >= warp_rows) {
+    // 6.8 us either way). Longer rows likewise, but for bf16, whose registers leave 16 warps an SM (fp16: 20), only up to the
+    // one wave that is resident and again where the second is well filled: just above 2368 rows it costs more than the warps
+    // gain (4096: 2368 rows 12.5 -> 11.9 us, 2400 rows 12.5 against 14.1 us, 3600 rows 17.2 against 17.3 us, 3800 rows
+    // 17.9 -> 17.2 us; 3584: 2400 rows 12.1 against 13.0 us, 3400 rows 15.7 -> 15.1 us). fp32 rows of 16 KB leave too few
+    // warps in flight (4093 x 4096: 24.8 against 30.0 us), and with the residual's second stream the CTA per row is not slower.
+    const int64_t resident = (int64_t)sm_count() * 16, refilled = row_bytes <= 7168 ? 3300 : 3750;
+    const bool bf16_tail = std::is_same<T, __nv_bfloat16>::value && row_bytes > 6144 && rows > resident && rows < refilled;
+    if (staged && !delta && D % 8 == 0 && D <= WarpRow<T>::MAX && (!w || aligned(w, 16)) && rows >= (row_bytes <= 4096 ? 1024 : 2048) && !bf16_tail) {
         const dim3 wgrid((unsigned)((rows + WARP_ROWS - 1) / WARP_ROWS)), wblock(32 * WARP_ROWS);
         auto kern = w ? rms_norm_warp_kernel<T, true> : rms_norm_warp_kernel<T, false>;
         launch_overlapped(kern, wgrid, wblock, 0, st, xp, wp, op, (long long)rows, (int)D, eps);

@@ -50,6 +50,10 @@ const char* bi_last_error(void);
  * No counterpart in the reference; benchmarks use it to state how many of the library's kernels a step runs. */
 unsigned long long bi_launch_count(void);
 
+/* The id of the capture that `stream` records into, another for each capture of the process; 0 when it records none. For
+ * callers that keep a workspace per capture. */
+unsigned long long bi_capture_id(void* stream);
+
 /*
  * Device status word. The tensor-core matmul kernels wait on shared-memory
  * barriers with an iteration limit; a wait that runs out stores a non-zero

@@ -35,6 +35,7 @@ SIGNATURES = {
     "bi_version": (c_int, []),
     "bi_last_error": (c_char_p, []),
     "bi_launch_count": (ctypes.c_ulonglong, []),
+    "bi_capture_id": (ctypes.c_ulonglong, [c_void_p]),
     "bi_read_device_status": (c_int, [c_void_p, POINTER(c_int32), c_void_p]),
     "bi_rms_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_float, c_int, c_void_p]),
     "bi_layer_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_float, c_int, c_void_p]),
@@ -176,15 +177,14 @@ class _Workspaces(threading.local):
     epoch = 0                     # of all threads: a new one drops every workspace
 
     def __init__(self):
-        self.seen, self.by_stream = _Workspaces.epoch, {}
+        self.reset()
 
-    def current(self) -> dict[tuple[int, int], torch.Tensor]:
-        if self.seen != _Workspaces.epoch:
-            self.seen, self.by_stream = _Workspaces.epoch, {}
-        return self.by_stream
+    def reset(self):
+        self.seen, self.by_stream = _Workspaces.epoch, {}
+        self.capture, self.captured = 0, {}
 
     def values(self):
-        return self.current().values()
+        return self.by_stream.values()
 
 
 _workspaces = _Workspaces()
@@ -195,24 +195,36 @@ def matmul_workspace(device: torch.device, nbytes: int, counters: bool = False) 
     """A workspace of at least `nbytes` for a call on the current stream of `device`, the current device, and whether its
     head is zero (always when `counters` asks for it).
 
-    Larger workspaces than KEPT_BYTES, and all that a capture records, are the call's own: the allocator hands the memory
-    on in stream order, and inside a capture takes it from the graph's pool. A kept workspace in a graph would be freed
-    under the graph as soon as a larger call replaced it."""
+    Larger workspaces than KEPT_BYTES are the call's own: the allocator hands the memory on in stream order. The calls of one
+    capture share one that comes from the graph's pool and is let go when the capture is over: a kept workspace in a graph
+    would be freed under the graph as soon as a larger call replaced it. (One of its own for each captured call spreads the
+    partials over more of L2: 64 sequences of the decoder step 6.02 against 5.98 ms.)"""
     idx = device.index if device.index is not None else torch.cuda.current_device()
-    need = max(nbytes, COUNTER_BYTES)
-    if need > KEPT_BYTES or torch._C._cuda_isCurrentStreamCapturing():
-        ws = torch.empty(need, dtype=torch.uint8, device=torch.device("cuda", idx))
-        if counters:
-            ws[:COUNTER_BYTES].zero_()
-        return ws, counters
     key = (idx, torch._C._cuda_getCurrentRawStream(idx))
-    kept = _workspaces.current()
-    ws = kept.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=torch.device("cuda", idx))
-        ws[:COUNTER_BYTES].zero_()       # only the counters have to start at zero
-        kept[key] = ws
-    return ws, True
+    mine = _workspaces
+    if not torch._C._cuda_isCurrentStreamCapturing():
+        if nbytes <= KEPT_BYTES:
+            if mine.captured or mine.seen != _Workspaces.epoch:
+                mine.capture, mine.captured = 0, {}
+                if mine.seen != _Workspaces.epoch:
+                    mine.reset()
+            ws = mine.by_stream.get(key)
+            if ws is None or ws.numel() < nbytes:
+                ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=torch.device("cuda", idx))
+                ws[:COUNTER_BYTES].zero_()       # only the counters have to start at zero
+                mine.by_stream[key] = ws
+            return ws, True
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=torch.device("cuda", idx))
+    else:
+        capture = load().bi_capture_id(key[1])
+        if not capture or capture != mine.capture:
+            mine.capture, mine.captured = capture, {}
+        ws = mine.captured.get(key)
+        if ws is None or ws.numel() < nbytes:
+            ws = mine.captured[key] = torch.empty(max(nbytes, COUNTER_BYTES), dtype=torch.uint8, device=torch.device("cuda", idx))
+    if counters:
+        ws[:COUNTER_BYTES].zero_()
+    return ws, counters
 
 
 def check_device_status(device: torch.device | None = None) -> None:

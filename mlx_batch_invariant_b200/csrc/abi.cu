@@ -36,6 +36,16 @@ extern "C" const char* bi_last_error(void) { return bi::g_err; }
 
 extern "C" unsigned long long bi_launch_count(void) { return bi::g_launches.load(std::memory_order_relaxed); }
 
+extern "C" unsigned long long bi_capture_id(void* stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &status, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return status == cudaStreamCaptureStatusActive ? id : 0;
+}
+
 extern "C" int bi_read_device_status(const int32_t* status, int32_t* host_value, void* stream) {
     using namespace bi;
     if (!status || !host_value) return fail(BI_ERR_BAD_ARG, "bi_read_device_status: null pointer");

@@ -93,3 +93,22 @@ def test_a_wait_that_ran_out_drops_the_scratch_of_every_thread(bi):
     t.join()
     assert _lib.matmul_workspace(torch.device("cuda", 0), 1 << 20)[0] is not before
     bi.check_device_status()
+
+
+def test_the_calls_of_a_capture_share_scratch_and_captures_do_not(bi):
+    x, w = _fp32(8, 2048, 4096, 4)
+    want = bi.batch_invariant_matmul(x, w.T, path="fused")
+    torch.cuda.synchronize()
+    graphs, outs, used = [torch.cuda.CUDAGraph() for _ in range(2)], [], []
+    s = torch.cuda.Stream()
+    for graph in graphs:
+        with torch.cuda.graph(graph, stream=s):
+            outs += [bi.batch_invariant_matmul(x, w.T), bi.batch_invariant_matmul(x, w.T)]
+            used += [_lib.matmul_workspace(x.device, 1 << 20)[0].data_ptr() for _ in range(2)]
+    assert used[0] == used[1] and used[2] == used[3] and used[0] != used[2]
+    bi.batch_invariant_matmul(x, w.T)
+    assert not _lib._workspaces.captured                               # an eager call lets the captures' scratch go
+    for graph in graphs:
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in outs)

@@ -19,8 +19,8 @@
 // K is refilled (cp.async) once the scores exist, V is double buffered. Up to three CTAs share an SM, so that one computes
 // while another waits at a barrier.
 //
-// Measured (bf16, D = 128, 32 query / 8 kv heads, causal): 2048 tokens 1231 us (fma pipe 66 % busy, the rest operand
-// conflicts and barriers), before 4442 us with eight lanes per key stream; 2 x 512 tokens 175 us, before 740 us.
+// Measured (bf16, D = 128, 32 query / 8 kv heads, causal): 2048 tokens 1231 us (the 0.82 ms of fp32 operations are two
+// thirds of it), before 4442 us with eight lanes per key stream; 2 x 512 tokens 175 us, before 740 us.
 #include "attn_common.cuh"
 
 namespace bi {

@@ -10,7 +10,7 @@
 // totals live in the registers of eight epilogue warps (each thread one weight row, half of the batch tile), while
 // the MMAs of the next group fill the other of two accumulators of 256 tensor-memory columns.
 //
-// What bounds it: the copies into shared memory. A K step of 64 takes 0.29 us + 1.2 ns per batch row of the tile, the
+// What bounds it: the copies into shared memory, then the drain of the accumulators. A K step of 64 takes 0.29 us + 1.2 ns per batch row of the tile, the
 // time of its (128 + bm/2) 128-byte rows at 57 GB/s an SM (the same with a quarter of the MMAs; without the copies it
 // takes 0.42 us at bm = 256, the MMAs alone 0.27). One SM per tile (128 x 128, matmul_tc.cu) takes 0.46 us a step for
 // a quarter of the pair's outputs, its partials on a round trip through tensor memory. fp16 1900 x 4096 -> 14336:

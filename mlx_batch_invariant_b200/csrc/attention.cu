@@ -609,15 +609,15 @@ __global__ void __launch_bounds__(32 * MAXW) decode_warp_stream_kernel(
 //     exp(-|s - m|) -- 32 exponentials per instruction instead of one;
 //   * accumulation: lane d owns dims 4d..4d+3 of all NH heads and walks the block's keys in order:
 //     l = fma(l, corr, p), acc = fma(acc, corr, p * v), the factors read back from shared memory.
-// A warp is one work item (batch, kv head, chunk of NH heads, split) at a time; items are dealt to a
+// A warp is one work item (batch, kv head, chunk of NH heads, split) at a time; the items that hold keys are dealt to a
 // persistent grid round-robin, full splits first.
 // Launch-shape constants, from measurements on B200 (bf16, 32/8 heads): two K blocks per warp beat one (eight and ten
 // warps with one K block: 53.7 / 65.7 us against 50.1 us with seven warps and two at 64 x 560 keys; ten warps cap the
 // kernel at 168 registers). Eight warps with two K blocks fit once the softmax factors of a block live in that
 // block's own K buffer, which nothing reads after the scores.
-constexpr int KL_WARPS = 8;    // most warps per CTA (one CTA per SM): two per scheduler. With fewer than two work items per
-                               // warp the launch uses seven: each warp is then faster and the tail is what counts
-                               // (64 x 560 keys: 50.1 us with seven, 53.2 with eight; 64 x 4096 keys: 268 against 248 us)
+constexpr int KL_WARPS = 8;    // most warps per CTA (one CTA per SM): two per scheduler. With few items the launch uses seven:
+                               // each warp is then faster and the tail is what counts (64 x 560 keys: 50.1 us with
+                               // seven, 53.2 with eight; 64 x 4096 keys: 268 against 248 us)
 constexpr int KL_KBUFS = 2;    // K blocks in shared memory per warp: the next block is fetched a whole block ahead
 constexpr int KL_UNROLL = 8;   // keys of the accumulation loop in flight
 constexpr int KL_KEYS = 32;
@@ -670,7 +670,59 @@ __device__ __forceinline__ void kl_node(const uint8_t* krow, const uint8_t* qs, 
     for (int h = 0; h < NH; ++h) out[h] = ptx::add2_rn(a[h], b[h]);
 }
 
-template <typename T, int NH, int NW>
+// The work items of a warp when the sequences differ in length, in ascending order: item i of the launch is (sequence, split,
+// kv head, chunk of query heads), the full splits of all sequences first, then the partly filled ones. Only splits that hold
+// keys are counted, from the lengths in device memory: a warp keeps the inclusive item counts of 32 sequences in its lanes
+// and moves on to the next 32, whose lengths are already on their way, when its index has passed them.
+struct KLItems {
+    const int32_t* kv_lens;
+    int B, L, split, per_seq;                              // per_seq: items of one split of a sequence (kv heads x chunks)
+    int phase, b0, len, ahead, incl;                       // this lane: length and inclusive item count of sequence b0 + lane
+    long long before;                                      // items in front of sequence b0
+    __device__ __forceinline__ int fetch(int from) const {
+        const int b = from + (int)(threadIdx.x & 31);
+        return b < B ? kv_lens[b] : 0;
+    }
+    __device__ __forceinline__ void count() {
+        const int lane = threadIdx.x & 31;
+        len = min(ahead, L);
+        ahead = fetch(b0 + 32 < B ? b0 + 32 : 0);
+        incl = (phase ? (len > 0 && len % split ? 1 : 0) : max(len, 0) / split) * per_seq;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += y;
+        }
+    }
+    __device__ __forceinline__ KLItems(const int32_t* lens, int B_, int L_, int split_, int per_seq_)
+        : kv_lens(lens), B(B_), L(L_), split(split_), per_seq(per_seq_), phase(L_ < split_ ? 1 : 0), b0(0), len(0), ahead(fetch(0)), incl(0), before(0) { count(); }
+    // item `i` (never smaller than in the call before): sequence, split, index among the split's per_seq items, keys
+    __device__ __forceinline__ bool find(long long i, int& b, int& sp, int& sub, int& nk) {
+        while (true) {
+            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            if (i < before + total) break;
+            before += total;
+            b0 += 32;
+            if (b0 >= B) {
+                if (phase) return false;
+                phase = 1;
+                b0 = 0;
+            }
+            count();
+        }
+        const int r = (int)(i - before);
+        const int src = __ffs(__ballot_sync(0xffffffffu, r < incl)) - 1;
+        const int prev = __shfl_sync(0xffffffffu, incl, max(src - 1, 0)), n = __shfl_sync(0xffffffffu, len, src);
+        const int rel = r - (src ? prev : 0);
+        b = b0 + src;
+        sp = phase ? n / split : rel / per_seq;
+        sub = phase ? rel : rel - sp * per_seq;
+        nk = phase ? n - sp * split : split;
+        return true;
+    }
+};
+
+template <typename T, int NH, int NW, bool LENS>
 __global__ void __launch_bounds__(32 * NW, 1) decode_keylane_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const int32_t* __restrict__ kv_lens,
     float* __restrict__ pm, float* __restrict__ pl, float* __restrict__ pacc, int B, int Hq, int Hkv, int L,
@@ -691,16 +743,30 @@ __global__ void __launch_bounds__(32 * NW, 1) decode_keylane_kernel(
     const long long per_split = (long long)B * Hkv * nchunk;
     const long long items = per_split * nsplit;
 
-    for (long long item = (long long)blockIdx.x * NW + wid; item < items; item += (long long)gridDim.x * NW) {
-        const int sp = (int)(item / per_split);
-        long long u = item - (long long)sp * per_split;
-        const int chunk = (int)(u % nchunk); u /= nchunk;
-        const int hk = (int)(u % Hkv);
-        const int b = (int)(u / Hkv);
-        const int Lb = kv_lens ? min(kv_lens[b], L) : L;
+    // Where items differ in length, consecutive ones go to different SMs: an SM's share of the keys is then close to the mean
+    // (64 sequences of 1 ... 4096 keys: 168 -> 125 us; 64 x 561 keys, whose last splits hold 49: 48.1 -> 46.4 us). Items of
+    // one length are as many an SM either way; its warps then take neighbours, the kv heads of one sequence (64 x 4096 keys
+    // 240 us, 245 dealt apart).
+    const bool apart = LENS || L % split != 0;
+    long long item = apart ? (long long)wid * gridDim.x + blockIdx.x : (long long)blockIdx.x * NW + wid;
+    KLItems work(kv_lens, LENS ? B : 0, L, split, Hkv * nchunk);
+    for (;; item += (long long)gridDim.x * NW) {
+        int b, sp, hk, chunk, nk;                                            // warp-uniform
+        if (LENS) {
+            int sub;
+            if (!work.find(item, b, sp, sub, nk)) break;
+            hk = sub / nchunk;
+            chunk = sub - hk * nchunk;
+        } else {
+            if (item >= items) break;
+            sp = (int)(item / per_split);
+            long long u = item - (long long)sp * per_split;
+            chunk = (int)(u % nchunk); u /= nchunk;
+            hk = (int)(u % Hkv);
+            b = (int)(u / Hkv);
+            nk = min(L, sp * split + split) - sp * split;
+        }
         const int j0 = sp * split;
-        const int nk = j0 < Lb ? (min(Lb, j0 + split) - j0) : 0;             // warp-uniform
-        if (nk == 0) continue;
         const int h0 = hk * G + chunk * NH;
         const int gcount = min(NH, G - chunk * NH);
         const T* const kb = k + (int64_t)b * lay.sb + (int64_t)hk * lay.sh + (int64_t)j0 * lay.sl;
@@ -924,11 +990,16 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
                 if (nh > 1 && B * Hkv * ((G + nh - 1) / nh) * nsplit < sms * 4) nh = 1;
                 const int nck = (G + nh - 1) / nh;
                 const int64_t items = B * Hkv * nck * nsplit;
-                const int nw = items >= 2 * sms * KL_WARPS ? KL_WARPS : KL_WARPS - 1;
+                // Seven warps where an SM has fewer than two items for each of eight, unless the eighth saves a round: 9 x
+                // 4096 keys, 1152 items, 69 us with seven and 43.5 with eight. How many items sequences of different
+                // length have is known on the device only: more than one round of them if all were full takes eight (8 x
+                // 1 ... 8192 keys: 60 us with seven, 45 with eight; where both are one round eight costs about 2 %).
+                const int64_t fit7 = sms * (KL_WARPS - 1), fit8 = sms * KL_WARPS;
+                const int nw = (kv_lens ? items > fit7 : items >= 2 * fit8 || (items + fit8 - 1) / fit8 < (items + fit7 - 1) / fit7) ? KL_WARPS : KL_WARPS - 1;
                 const int64_t ctas = std::min<int64_t>(sms, (items + nw - 1) / nw);
-#define BI_KL_LAUNCH(NHV, NWV)                                                                                         \
+#define BI_KL_LAUNCH(NHV, NWV, LENSV)                                                                                         \
     do {                                                                                                                \
-        auto kern = decode_keylane_kernel<T, NHV, (NWV)>;                                                                \
+        auto kern = decode_keylane_kernel<T, NHV, (NWV), LENSV>;                                                              \
         static bool attr_set[64] = {false};                                                                             \
         int dev_ = 0;                                                                                                   \
         cudaGetDevice(&dev_);                                                                                           \
@@ -941,8 +1012,9 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
         launch_overlapped(kern, dim3((unsigned)ctas), dim3(32 * (NWV)), (size_t)((NWV) * KLCfg::WARP_BYTES), st, qp, kp, vp, kv_lens, pm, pl, pacc, \
                           (int)B, (int)Hq, (int)Hkv, (int)L, lay, scale, split, nsplit, nck);                           \
     } while (0)
-#define BI_KL_LAUNCH_NH(NWV) do { if (nh == 4) BI_KL_LAUNCH(4, NWV); else if (nh == 2) BI_KL_LAUNCH(2, NWV); else BI_KL_LAUNCH(1, NWV); } while (0)
-                if (nw == KL_WARPS) BI_KL_LAUNCH_NH(KL_WARPS); else BI_KL_LAUNCH_NH(KL_WARPS - 1);
+#define BI_KL_LAUNCH_NH(NWV, LENSV) do { if (nh == 4) BI_KL_LAUNCH(4, NWV, LENSV); else if (nh == 2) BI_KL_LAUNCH(2, NWV, LENSV); else BI_KL_LAUNCH(1, NWV, LENSV); } while (0)
+                if (kv_lens) { if (nw == KL_WARPS) BI_KL_LAUNCH_NH(KL_WARPS, true); else BI_KL_LAUNCH_NH(KL_WARPS - 1, true); }
+                else { if (nw == KL_WARPS) BI_KL_LAUNCH_NH(KL_WARPS, false); else BI_KL_LAUNCH_NH(KL_WARPS - 1, false); }
 #undef BI_KL_LAUNCH_NH
 #undef BI_KL_LAUNCH
                 int rck = check_launch("bi_attn_decode (key per lane)");

@@ -193,36 +193,42 @@ struct ChunkIter {
 // One weight row's 64 codes of K step `kstep` of a chunk -> 32 packed pairs of T, written to the row's
 // tensor-memory lane at columns taddr .. taddr+31 (column c holds elements 2c and 2c+1 of the row, low half
 // first) in two stores of 16 columns. `raw` is the chunk's packed codes as the TMA boxes left them (rows of 128
-// bytes, 128-byte swizzle); (s2a, b2a) apply to codes 0..31, (s2b, b2b) to codes 32..63.
+// bytes, 128-byte swizzle); the low halves of (scales, biases) apply to codes 0..31, the high halves to codes 32..63.
 template <typename T, int QBITS>
-__device__ __forceinline__ void dequant_row64_to_tmem(const uint8_t* raw, int row, int kstep, uint64_t s2a, uint64_t b2a,
-                                                      uint64_t s2b, uint64_t b2b, uint32_t taddr) {
+__device__ __forceinline__ void dequant_row64_to_tmem(const uint8_t* raw, int row, int kstep, uint32_t scales, uint32_t biases, uint32_t taddr) {
     constexpr int PIECES = BLOCK_K * QBITS / 8 / 16;     // 16-byte pieces behind 64 codes: 2 (4-bit) or 4 (8-bit)
     constexpr int HP = PIECES / 2;                       // pieces behind 32 codes
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const uint64_t s2 = h ? s2b : s2a, b2 = h ? b2b : b2a;
+    constexpr int WORDS = QBITS / 4;                     // words behind eight codes
+    const bool packed = __all_sync(0xffffffffu, dequant_exact<T, QBITS>(scales & 0xffffu, biases & 0xffffu) && dequant_exact<T, QBITS>(scales >> 16, biases >> 16));
+    auto half = [&](int h, auto&& eight) {               // 32 codes -> 16 columns
         uint32_t o[16];
 #pragma unroll
         for (int cc = 0; cc < HP; ++cc) {
             const uint4 q = *reinterpret_cast<const uint4*>(raw + raw_piece_offset(row, kstep * PIECES + h * HP + cc, 128));
             const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-            if (QBITS == 4) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint4 v = dequant8<T, 4>(&w[i], s2, b2);
-                    o[i * 4 + 0] = v.x; o[i * 4 + 1] = v.y; o[i * 4 + 2] = v.z; o[i * 4 + 3] = v.w;
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const uint4 v = dequant8<T, 8>(&w[2 * i], s2, b2);
-                    o[(cc * 2 + i) * 4 + 0] = v.x; o[(cc * 2 + i) * 4 + 1] = v.y;
-                    o[(cc * 2 + i) * 4 + 2] = v.z; o[(cc * 2 + i) * 4 + 3] = v.w;
-                }
+            for (int i = 0; i < 4 / WORDS; ++i) {
+                const uint4 v = eight(&w[WORDS * i]);
+                uint32_t* d = o + (cc * (4 / WORDS) + i) * 4;
+                d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
             }
         }
         ptx::tmem_st_32x16(taddr + 16u * h, o);
+    };
+    if (packed) {
+        const uint32_t s2 = dequant_scale<T>(scales);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t sh = h ? prmt<0x3232>(s2, 0u) : prmt<0x1010>(s2, 0u), bh = h ? prmt<0x3232>(biases, 0u) : prmt<0x1010>(biases, 0u);
+            half(h, [&](const uint32_t* w) { return dequant8_packed<T, QBITS>(w, sh, bh); });
+        }
+    } else {
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+            const float sf = word16_up<T>(h ? scales >> 16 : scales & 0xffffu), bf = word16_up<T>(h ? biases >> 16 : biases & 0xffffu);
+            const uint64_t s2 = ptx::pack2(sf, sf), b2 = ptx::pack2(bf, bf);
+            half(h, [&](const uint32_t* w) { return dequant8<T, QBITS>(w, s2, b2); });
+        }
     }
 }
 
@@ -725,10 +731,7 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             if ((qi >> 1) == 1) wd = wds[1];
             if ((qi >> 1) == 2) wd = wds[2];
             if ((qi >> 1) == 3) wd = wds[3];
-            const unsigned short h = (unsigned short)((qi & 1) ? (wd >> 16) : (wd & 0xffffu));
-            T tv;
-            *reinterpret_cast<unsigned short*>(&tv) = h;
-            return Cvt<T>::up(tv);
+            return word16_up<T>((qi & 1) ? (wd >> 16) : (wd & 0xffffu));
         };
         uint32_t sw[4] = {0u, 0u, 0u, 0u}, bw[4] = {0u, 0u, 0u, 0u};      // current K group
         uint32_t sw_n[4], bw_n[4];                                        // next K group, in flight
@@ -809,11 +812,6 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 bv = __ldg(biases + e);
             }
         };
-        auto to_f = [&](uint32_t h) {
-            T tv;
-            *reinterpret_cast<unsigned short*>(&tv) = (unsigned short)h;
-            return Cvt<T>::up(tv);
-        };
         uint32_t qs[DEPTH], qb[DEPTH];
         ChunkIter pf(p, ub, ue);
 #pragma unroll
@@ -839,9 +837,7 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             if (jstep < kst) {
                 advance();
                 ptx::tc_fence_after();
-                const float s0 = to_f(sv & 0xffffu), s1 = to_f(sv >> 16), b0 = to_f(bv & 0xffffu), b1 = to_f(bv >> 16);
-                dequant_row64_to_tmem<T, QB>(smem_gen + (raw_chunk(l) - smem_base), row, jstep, ptx::pack2(s0, s0), ptx::pack2(b0, b0),
-                                             ptx::pack2(s1, s1), ptx::pack2(b1, b1),
+                dequant_row64_to_tmem<T, QB>(smem_gen + (raw_chunk(l) - smem_base), row, jstep, sv, bv,
                                              a_lane + (uint32_t)((w * KS + jstep) * TMEM_A_STEP));
                 ptx::tmem_st_wait();
             } else {

@@ -130,6 +130,25 @@ def load() -> ctypes.CDLL:
     return _lib
 
 
+_bound = None
+
+
+def calls():
+    """The hot entry points of the loaded library as C functions of a CPython module (csrc/calls.c): same arguments, a
+    tenth of ctypes' cost a call."""
+    global _bound
+    if _bound is None:
+        lib = load()
+        with _lock:
+            try:
+                from . import _calls
+            except ImportError as e:
+                raise RuntimeError(f"{LIB_PATH.parent / '_calls.so'} is missing: build it with `python -m mlx_batch_invariant_b200.build`") from e
+            _calls.bind(lib._handle)
+            _bound = _calls
+    return _bound
+
+
 def last_error() -> str:
     return load().bi_last_error().decode("utf-8", "replace")
 

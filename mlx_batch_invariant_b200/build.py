@@ -1,4 +1,5 @@
-"""Build libbi_b200.so (the C-ABI kernel library) in-tree with nvcc for sm_100a.
+"""Build libbi_b200.so (the C-ABI kernel library) in-tree with nvcc for sm_100a, and _calls.so (the CPython face of its
+hot entry points) with the C compiler.
 
     python -m mlx_batch_invariant_b200.build          # rebuild if sources changed
     python -m mlx_batch_invariant_b200.build --force
@@ -14,12 +15,14 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OUT = PKG / "libbi_b200.so"
+CALLS = PKG / "_calls.so"
 OBJ = PKG / "build"
 SOURCES = ["abi.cu", "rmsnorm.cu", "attention.cu", "attn_prefill.cu", "attn_decode_static.cu", "matmul_simt.cu", "matmul_tc.cu", "matmul_pair.cu", "dequant.cu", "matmul.cu", "glue.cu", "peer.cu"]
 
@@ -44,17 +47,18 @@ def _sources() -> list[Path]:
 
 def _fingerprint() -> str:
     h = hashlib.sha256()
-    for p in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + [PKG.parent / "include" / "bi_abi.h"]):
+    for p in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.c")) + [PKG.parent / "include" / "bi_abi.h"]):
         h.update(p.name.encode())
         h.update(p.read_bytes())
     h.update(" ".join(NVCC_FLAGS).encode())
+    h.update(sys.version.encode())
     return h.hexdigest()
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
     stamp = OBJ / "fingerprint.txt"
     fp = _fingerprint()
-    if not force and OUT.exists() and stamp.exists() and stamp.read_text() == fp:
+    if not force and OUT.exists() and CALLS.exists() and stamp.exists() and stamp.read_text() == fp:
         return OUT
     OBJ.mkdir(exist_ok=True)
     nvcc = _nvcc()
@@ -76,6 +80,11 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     r = subprocess.run([nvcc, "-shared", "-o", str(OUT), *map(str, objs)], capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    cc = os.environ.get("CC") or shutil.which("gcc") or shutil.which("cc") or "gcc"
+    r = subprocess.run([cc, "-O2", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], "-o", str(CALLS), str(CSRC / "calls.c"), "-ldl"],
+                       capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{cc} failed for calls.c:\n{r.stdout}\n{r.stderr}")
     stamp.write_text(fp)
     return OUT
 

@@ -81,18 +81,18 @@ def batch_invariant_decode_attention(q, k, v, *, scale: float, split_size: int =
         lens = adopt(kv_lens)[0].to(device=dev, dtype=torch.int32).contiguous()
         if lens.shape != (B,):
             raise ValueError(f"kv_lens must have shape ({B},), got {tuple(lens.shape)}")
-    lib = _lib.load()
-    nbytes = lib.bi_attn_decode_workspace_bytes(B, Hq, L, D, split_size)
+    calls = _lib.calls()
+    nbytes = calls.bi_attn_decode_workspace_bytes(B, Hq, L, D, split_size)
     ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=dev)
     if push is not None:
         with _lib.on_device(dev):
-            _lib.check(lib.bi_attn_decode_push(qc.data_ptr(), kt.data_ptr(), vt.data_ptr(), _lib.ptr(lens), ws.data_ptr(), nbytes,
+            _lib.check(_lib.load().bi_attn_decode_push(qc.data_ptr(), kt.data_ptr(), vt.data_ptr(), _lib.ptr(lens), ws.data_ptr(), nbytes,
                                                B, Hq, Hkv, L, D, sb, sh, sl, float(scale), int(split_size), code,
                                                _lib.stream_ptr(dev), *push, _lib.status_word(dev).data_ptr()))
         return None
     out = torch.empty_like(qc)
     with _lib.on_device(dev):
-        _lib.check(lib.bi_attn_decode(qc.data_ptr(), kt.data_ptr(), vt.data_ptr(), out.data_ptr(), _lib.ptr(lens),
+        _lib.check(calls.bi_attn_decode(qc.data_ptr(), kt.data_ptr(), vt.data_ptr(), out.data_ptr(), _lib.ptr(lens),
                                       ws.data_ptr(), nbytes, B, Hq, Hkv, L, D, sb, sh, sl, float(scale),
                                       int(split_size), code, _lib.stream_ptr(dev)))
     return give_back(out, q, foreign)
@@ -137,7 +137,7 @@ def batch_invariant_prefill_attention(q, k, v, *, scale: float, causal: bool, sp
     kt, vt, sb, sh, sl = _kv_layout(kt, vt)
     out = torch.empty_like(qc)
     with _lib.on_device(dev):
-        _lib.check(_lib.load().bi_attn_prefill(qc.data_ptr(), kt.data_ptr(), vt.data_ptr(), out.data_ptr(), B, Hq, Hkv,
+        _lib.check(_lib.calls().bi_attn_prefill(qc.data_ptr(), kt.data_ptr(), vt.data_ptr(), out.data_ptr(), B, Hq, Hkv,
                                                Tq, L, D, sb, sh, sl, float(scale), 1 if causal else 0,
                                                int(split_size), code, _lib.stream_ptr(dev)))
     return give_back(out, q, foreign)

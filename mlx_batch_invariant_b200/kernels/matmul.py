@@ -14,7 +14,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from ._util import adopt, dtype_code, give_back, require_cuda, rows_16b
+from ._util import adopt, dtype_code, empty, give_back, require_cuda, rows_16b
 
 GROUP_K = 256
 
@@ -38,9 +38,10 @@ def _launch_shape(path: str, batch_tile: int | None, M: int, N: int, K: int, ws_
 def _weight_is_tensor_core(b: torch.Tensor, K: int) -> bool:
     """The predicate bi_matmul applies to the weight (16-bit, rows of K contiguous elements
     that TMA can address). Used only to decide whether the activation needs an aligned copy."""
-    es = b.element_size()
-    return (b.dtype != torch.float32 and b.stride(0) == 1 and K % 8 == 0 and b.data_ptr() % 16 == 0
-            and (b.shape[1] == 1 or ((b.stride(1) * es) % 16 == 0 and b.stride(1) >= K)))
+    if b.dtype == torch.float32:
+        return False
+    sk, sn = b.stride()
+    return sk == 1 and K % 8 == 0 and b.data_ptr() % 16 == 0 and (b.shape[1] == 1 or (sn % 8 == 0 and sn >= K))
 
 
 def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None = None, awaiting=None, bias=None, push=None,
@@ -106,18 +107,19 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
                                           a2.stride(0) if M > 1 else K, a2.stride(1), bt.stride(0), bt.stride(1), code, word,
                                           _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev), *aw, *push))
         return None
-    out = torch.empty((M, N), dtype=out_dtype, device=dev)
+    out = empty(a2, (M, N), out_dtype)
+    calls = _lib.calls()
     with _lib.on_device(dev):
-        word, ws, nbytes = _launch_shape(path, batch_tile, M, N, K, lib.bi_matmul_scratch_bytes(M, N, K, code), dev)
-        args = (a2.data_ptr(), bt.data_ptr(), out.data_ptr(), _lib.ptr(ws), nbytes, M, N, K,
-                a2.stride(0) if M > 1 else K, a2.stride(1), bt.stride(0), bt.stride(1), code,
+        word, ws, nbytes = _launch_shape(path, batch_tile, M, N, K, calls.bi_matmul_scratch_bytes(M, N, K, code), dev)
+        sm, sk = a2.stride()
+        args = (a2.data_ptr(), bt.data_ptr(), out.data_ptr(), _lib.ptr(ws), nbytes, M, N, K, sm if M > 1 else K, sk, *bt.stride(), code,
                 word, _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev))
         if bias is not None:
             bias_t = adopt(bias)[0]
             if bias_t.shape != (N,) or bias_t.dtype != out_dtype or not bias_t.is_cuda or awaiting is not None:
                 raise ValueError("bias must be a CUDA tensor of shape [N] in the output dtype (and cannot be combined with awaiting)")
             bias_t = bias_t.contiguous()
-            _lib.check(lib.bi_matmul_bias(args[0], args[1], bias_t.data_ptr(), *args[2:]))
+            _lib.check(calls.bi_matmul_bias(args[0], args[1], bias_t.data_ptr(), *args[2:]))
         else:
-            _lib.check(lib.bi_matmul(*args) if awaiting is None else lib.bi_matmul_awaiting(*args, *awaiting))
+            _lib.check(calls.bi_matmul(*args) if awaiting is None else lib.bi_matmul_awaiting(*args, *awaiting))
     return give_back(out if at.ndim == 2 else out.reshape(*lead, N), a, foreign)

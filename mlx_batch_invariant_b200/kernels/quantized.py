@@ -15,7 +15,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from ._util import adopt, dtype_code, give_back, require_cuda, rows_16b
+from ._util import adopt, dtype_code, empty, give_back, require_cuda, rows_16b
 from .matmul import _launch_shape
 
 SUPPORTED_BITS = (4, 8)
@@ -87,12 +87,13 @@ def batch_invariant_quantized_matmul(x, w, scales, biases, *, group_size: int, b
                                        x2.stride(0) if M > 1 else K, group_size, bits, code, word | _STAGES[stage],
                                        _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev), *aw, *push))
         return None
-    out = torch.empty((M, N), dtype=dt, device=dev)
+    out = empty(x2, (M, N), dt)
+    calls = _lib.calls()
     with _lib.on_device(dev):
-        word, ws, nbytes = _launch_shape(path, batch_tile, M, N, K, lib.bi_qmm_scratch_bytes(M, N, K, code), dev,
+        word, ws, nbytes = _launch_shape(path, batch_tile, M, N, K, calls.bi_qmm_scratch_bytes(M, N, K, code), dev,
                                        _lib.COUNTER_BYTES + 2 * N * K)
         args = (x2.data_ptr(), wt.data_ptr(), st.data_ptr(), bt.data_ptr(), out.data_ptr(),
                 _lib.ptr(ws), nbytes, M, N, K, x2.stride(0) if M > 1 else K, group_size, bits, code,
                 word | _STAGES[stage], _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev))
-        _lib.check(lib.bi_qmm(*args) if awaiting is None else lib.bi_qmm_awaiting(*args, *awaiting))
+        _lib.check(calls.bi_qmm(*args) if awaiting is None else lib.bi_qmm_awaiting(*args, *awaiting))
     return give_back(out if xt.ndim == 2 else out.reshape(*lead, N), x, foreign)

@@ -10,7 +10,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from ._util import adopt, dtype_code, give_back, require_cuda
+from ._util import adopt, dtype_code, empty, give_back, require_cuda
 
 
 def batch_invariant_rms_norm(x, weight, eps: float):
@@ -28,8 +28,8 @@ def batch_invariant_rms_norm(x, weight, eps: float):
         wt = wt.contiguous()
     rows = xt.numel() // D if D else 0
     x2 = xt.contiguous()
-    out = torch.empty(xt.shape, dtype=xt.dtype, device=dev)
+    out = empty(x2, xt.shape, xt.dtype)
     with _lib.on_device(dev):
-        _lib.check(_lib.load().bi_rms_norm(x2.data_ptr(), _lib.ptr(wt), out.data_ptr(), rows, D, float(eps), code,
+        _lib.check(_lib.calls().bi_rms_norm(x2.data_ptr(), _lib.ptr(wt), out.data_ptr(), rows, D, float(eps), code,
                                            _lib.stream_ptr(dev)))
     return give_back(out, x, foreign)

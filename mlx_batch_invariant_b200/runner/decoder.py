@@ -126,7 +126,7 @@ class KernelBackend(TorchGlue):
         args = (x.data_ptr(), delta.data_ptr(), w.data_ptr(), s.data_ptr(), out.data_ptr(), rows, D, float(eps),
                 _lib.DTYPE_CODE[x.dtype], _lib.stream_ptr(x.device))
         if awaiting is None:
-            _lib.check(_lib.load().bi_add_rms_norm(*args))
+            _lib.check(_lib.calls().bi_add_rms_norm(*args))
         else:
             _lib.check(_lib.load().bi_add_rms_norm_awaiting(*args, *awaiting, _lib.status_word(x.device).data_ptr()))
         return s, out

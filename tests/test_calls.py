@@ -1,0 +1,31 @@
+"""The CPython face of the hot entry points: the same functions as through ctypes, and its argument checks."""
+
+import pytest
+
+from mlx_batch_invariant_b200 import _lib
+
+
+def test_the_same_answers_as_through_ctypes():
+    c, l = _lib.calls(), _lib.load()
+    for M, N, K in ((1, 4096, 4096), (64, 4096, 14336), (300, 4096, 4096), (100, 4096, 4096)):
+        for dt in (_lib.BI_F32, _lib.BI_F16, _lib.BI_BF16):
+            assert c.bi_matmul_scratch_bytes(M, N, K, dt) == l.bi_matmul_scratch_bytes(M, N, K, dt)
+            assert c.bi_qmm_scratch_bytes(M, N, K, dt) == l.bi_qmm_scratch_bytes(M, N, K, dt)
+    assert c.bi_attn_decode_workspace_bytes(2, 32, 257, 128, 256) == l.bi_attn_decode_workspace_bytes(2, 32, 257, 128, 256)
+
+
+@pytest.mark.parametrize("name", ["bi_rms_norm", "bi_add_rms_norm", "bi_matmul", "bi_matmul_bias", "bi_qmm", "bi_attn_decode", "bi_attn_prefill"])
+def test_arguments(name):
+    """Null pointers (None) are the library's own error, with its message, never a launch; a call takes as many arguments as
+    the prototype has, and of their kinds."""
+    fn, args = getattr(_lib.calls(), name), _lib.SIGNATURES[name][1]
+    values = [0.5 if a is _lib.c_float else None if a is _lib.c_void_p else 1 for a in args]
+    code, said = fn(*values), _lib.last_error()
+    assert code == getattr(_lib.load(), name)(*values) != _lib.BI_OK
+    assert said == _lib.last_error()
+    with pytest.raises(TypeError):
+        fn(*values[:-1])
+    with pytest.raises(TypeError):
+        fn(*[0.5] * len(values))
+    with pytest.raises(OverflowError):
+        fn(*[2 ** 70] * len(values))

@@ -164,22 +164,107 @@ __global__ void __launch_bounds__(TG) rms_norm_kernel(const T* x, const T* __res
     }
 }
 
-// A warp per row, for many rows of up to 4096 16-bit or 1024 fp32 elements: lane l owns virtual threads 8 l ... 8 l + 7, whose stride-256
-// elements are exactly the 16-byte pieces l, l + 32, ... of the row (two pieces each for fp32). The row stays in the
-// lane's registers from the load to the store, and the tree is shuffles: levels 128, 64, 32 halve the eight values a lane
-// holds (it keeps the half its lane bit names and adds its partner's), 16 and 8 add whole lanes, 4, 2, 1 meet over the
-// same three lane bits -- the canonical pairs, whose order inside an add is free.
-// What bounds it: memory, with 8 KB in flight per warp and no barrier. The CTA per row above spends a row's time on
-// load, five barriers and store in series. Rows that are not in L2: bf16 4093 x 4096 19.3 -> 17.8 us, 8192 x 4096
-// 36.8 -> 29.3 us, 4093 x 896 15.0 -> 7.3 us.
-constexpr int WARP_ROWS = 4;
-template <typename T> struct WarpRow { static constexpr int MAX = sizeof(T) == 2 ? 4096 : 1024; };   // longest row kept in registers
+// A warp per row, for many rows: lane l owns virtual threads 8 l ... 8 l + 7, whose stride-256 elements are exactly pieces
+// l, l + 32, ... of eight elements of the row, and the tree is shuffles: levels 128, 64, 32 halve the eight values a lane
+// holds (it keeps the half its lane bit names and adds its partner's), 16 and 8 add whole lanes, 4, 2, 1 meet over the same
+// three lane bits -- the canonical pairs, whose order inside an add is free.
+__device__ __forceinline__ float warp_tree_sum(const float (&ss)[8], int lane) {
+    float h4[4], h2[2], h;
+    const bool b16 = lane & 16, b8 = lane & 8, b4 = lane & 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {                        // red[t] + red[t + 128]
+        const float got = __shfl_xor_sync(0xffffffffu, b16 ? ss[e] : ss[e + 4], 16);
+        h4[e] = add_rn(b16 ? ss[e + 4] : ss[e], got);
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {                        // 64
+        const float got = __shfl_xor_sync(0xffffffffu, b8 ? h4[e] : h4[e + 2], 8);
+        h2[e] = add_rn(b8 ? h4[e + 2] : h4[e], got);
+    }
+    {                                                    // 32
+        const float got = __shfl_xor_sync(0xffffffffu, b4 ? h2[0] : h2[1], 4);
+        h = add_rn(b4 ? h2[1] : h2[0], got);
+    }
+    h = add_rn(h, __shfl_xor_sync(0xffffffffu, h, 2));   // 16
+    h = add_rn(h, __shfl_xor_sync(0xffffffffu, h, 1));   // 8
+    h = add_rn(h, __shfl_xor_sync(0xffffffffu, h, 16));  // 4: the value kept by the other half
+    h = add_rn(h, __shfl_xor_sync(0xffffffffu, h, 8));   // 2
+    h = add_rn(h, __shfl_xor_sync(0xffffffffu, h, 4));   // 1
+    return h;
+}
+
+// 16-bit rows of up to 16 KB: the row waits in shared memory, brought by cp.async in two halves (a lane reads only what it
+// copied itself, so nothing but its own wait stands between the copies and the sums). What bounds it: memory, by the bytes in
+// flight. With the row in registers 16 to 20 warps fit an SM (160 KB in flight, and 2400 rows of bf16 took a second wave);
+// staged, 28 rows of 8 KB do, and longer rows no longer fall back to a CTA per row, which spends its time on load, five
+// barriers and store in series. Rows that are not in L2, bf16: 4093 x 4096 13.8 -> 12.7 us (6000: 20.7 -> 17.5; 2400: 12.0 ->
+// 8.5), 4093 x 896 6.6 -> 4.7 us, 4093 x 8192 35.5 -> 26.0 us. Two rows a CTA: four are up to 5 % slower where the last wave
+// is short; one piece of copies instead of two halves, and loops unrolled by four, 5 to 20 % slower.
+constexpr int STAGED_ROWS = 2;
+constexpr size_t STAGED_ROW_MAX = 16 * 1024;
 template <typename T, bool HAS_W>
-__global__ void __launch_bounds__(32 * WARP_ROWS) rms_norm_warp_kernel(const T* x, const T* __restrict__ w, T* out, long long rows, int D,
-                                                                       float eps) {
+__global__ void __launch_bounds__(32 * STAGED_ROWS, 14) rms_norm_staged_warp_kernel(const T* x, const T* __restrict__ w, T* out, long long rows,
+                                                                                    int D, float eps) {
+    static_assert(sizeof(T) == 2 && STAGED_ROWS * STAGED_ROW_MAX <= 48 * 1024, "a piece of eight elements is one 16-byte word; no shared-memory opt-in");
     ptx::grid_dep_launch();
     ptx::grid_dep_wait();
-    constexpr int PIECES = WarpRow<T>::MAX / 256;          // eight elements of a lane each
+    extern __shared__ uint4 stage_raw[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long row = (long long)blockIdx.x * STAGED_ROWS + wid;
+    if (row >= rows) return;
+    const int n = D >> 3, half = (n >> 6) << 5;          // pieces of the row; whole rounds of the warp in front of the second wait
+    const size_t at = (size_t)row * (size_t)D;
+    uint4* const buf = stage_raw + (size_t)wid * (size_t)n;
+    const uint4* const src = reinterpret_cast<const uint4*>(x + at);
+    const uint32_t buf_s = (uint32_t)__cvta_generic_to_shared(buf);
+    auto fetch = [&](int i) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(buf_s + (uint32_t)i * 16u), "l"(src + i) : "memory"); };
+#pragma unroll 8
+    for (int i = lane; i < half; i += 32) fetch(i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll 8
+    for (int i = half + lane; i < n; i += 32) fetch(i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    float ss[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss[e] = 0.0f;
+    auto add = [&](int i) {
+        const uint4 v = buf[i];
+        const T* a = reinterpret_cast<const T*>(&v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { const float f = Cvt<T>::up(a[e]); ss[e] = fma_rn(f, f, ss[e]); }
+    };
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+#pragma unroll 8
+    for (int i = lane; i < half; i += 32) add(i);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll 8
+    for (int i = half + lane; i < n; i += 32) add(i);
+    const float h = warp_tree_sum(ss, lane);
+    const float inv = rsqrt_canon(add_rn(div_canon(h, (float)D), eps));
+    uint4* const dst = reinterpret_cast<uint4*>(out + at);
+#pragma unroll 8
+    for (int i = lane; i < n; i += 32) {
+        uint4 v = buf[i], wv = make_uint4(0u, 0u, 0u, 0u);
+        if (HAS_W) wv = reinterpret_cast<const uint4*>(w)[i];
+        T* a = reinterpret_cast<T*>(&v);
+        const T* b = reinterpret_cast<const T*>(&wv);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) a[e] = Cvt<T>::down(mul_rn(mul_rn(Cvt<T>::up(a[e]), inv), HAS_W ? Cvt<T>::up(b[e]) : 1.0f));
+        dst[i] = v;
+    }
+}
+
+// fp32 rows of up to 1024 elements: the row stays in the lane's registers from the load to the store (two 16-byte words a
+// piece; staged like the 16-bit rows 4093 x 896 takes 7.8 against 6.3 us).
+constexpr int WARP_ROWS = 4;
+constexpr int WARP_ROW_MAX = 1024;                       // longest row kept in registers
+template <bool HAS_W>
+__global__ void __launch_bounds__(32 * WARP_ROWS) rms_norm_warp_kernel(const float* x, const float* __restrict__ w, float* out, long long rows,
+                                                                       int D, float eps) {
+    using T = float;
+    ptx::grid_dep_launch();
+    ptx::grid_dep_wait();
+    constexpr int PIECES = WARP_ROW_MAX / 256;          // eight elements of a lane each
     constexpr int Q = sizeof(T) / 2;                     // 16-byte words per piece
     struct Piece { uint4 q[Q]; };
     const int lane = threadIdx.x & 31;
@@ -213,27 +298,7 @@ __global__ void __launch_bounds__(32 * WARP_ROWS) rms_norm_warp_kernel(const T* 
             for (int e = 0; e < 8; ++e) { const float f = Cvt<T>::up(a[e]); ss[e] = fma_rn(f, f, ss[e]); }
         }
     }
-    float h4[4], h2[2], h;
-    const bool b16 = lane & 16, b8 = lane & 8, b4 = lane & 4;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {                        // red[t] + red[t + 128]
-        const float got = __shfl_xor_sync(0xffffffffu, b16 ? ss[e] : ss[e + 4], 16);
-        h4[e] = add_rn(b16 ? ss[e + 4] : ss[e], got);
-    }
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {                        // 64
-        const float got = __shfl_xor_sync(0xffffffffu, b8 ? h4[e] : h4[e + 2], 8);
-        h2[e] = add_rn(b8 ? h4[e + 2] : h4[e], got);
-    }
-    {                                                    // 32
-        const float got = __shfl_xor_sync(0xffffffffu, b4 ? h2[0] : h2[1], 4);
-        h = add_rn(b4 ? h2[1] : h2[0], got);
-    }
-    h = add_rn(h, __shfl_xor_sync(0xffffffffu, h, 2));   // 16
-    h = add_rn(h, __shfl_xor_sync(0xffffffffu, h, 1));   // 8
-    h = add_rn(h, __shfl_xor_sync(0xffffffffu, h, 16));  // 4: the value kept by the other half
-    h = add_rn(h, __shfl_xor_sync(0xffffffffu, h, 8));   // 2
-    h = add_rn(h, __shfl_xor_sync(0xffffffffu, h, 4));   // 1
+    const float h = warp_tree_sum(ss, lane);
     const float inv = rsqrt_canon(add_rn(div_canon(h, (float)D), eps));
 #pragma unroll
     for (int j = 0; j < PIECES; ++j) {
@@ -334,20 +399,24 @@ int launch(const void* x, const void* delta, const void* w, void* sum_out, void*
     const T* wp = static_cast<const T*>(w);
     T* sp = static_cast<T*>(sum_out);
     T* op = static_cast<T*>(out);
-    // A warp per row once there are rows enough for it, by times over rows that are not in L2: rows of up to 4 KB from 1024
-    // on (bf16 896: 5.2 -> 4.1 us; fp32 896: 5.7 -> 4.1 us), of up to 6 KB from 2048 on (bf16 3072: 10.2 -> 9.0 us, 1024 rows
-    // 6.8 us either way). Longer rows likewise, but for bf16, whose registers leave 16 warps an SM (fp16: 20), only up to the
-    // one wave that is resident and again where the second is well filled: just above 2368 rows it costs more than the warps
-    // gain (4096: 2368 rows 12.5 -> 11.9 us, 2400 rows 12.5 against 14.1 us, 3600 rows 17.2 against 17.3 us, 3800 rows
-    // 17.9 -> 17.2 us; 3584: 2400 rows 12.1 against 13.0 us, 3400 rows 15.7 -> 15.1 us). fp32 rows of 16 KB leave too few
-    // warps in flight (4093 x 4096: 24.8 against 30.0 us), and with the residual's second stream the CTA per row is not slower.
-    const int64_t resident = (int64_t)sm_count() * 16, refilled = row_bytes <= 7168 ? 3300 : 3750;
-    const bool bf16_tail = std::is_same<T, __nv_bfloat16>::value && row_bytes > 6144 && rows > resident && rows < refilled;
-    if (staged && !delta && D % 8 == 0 && D <= WarpRow<T>::MAX && (!w || aligned(w, 16)) && rows >= (row_bytes <= 4096 ? 1024 : 2048) && !bf16_tail) {
-        const dim3 wgrid((unsigned)((rows + WARP_ROWS - 1) / WARP_ROWS)), wblock(32 * WARP_ROWS);
-        auto kern = w ? rms_norm_warp_kernel<T, true> : rms_norm_warp_kernel<T, false>;
-        launch_overlapped(kern, wgrid, wblock, 0, st, xp, wp, op, (long long)rows, (int)D, eps);
-        return check_launch("bi_rms_norm");
+    // A warp per row once there are rows enough for it, by times over rows that are not in L2. 16-bit rows of up to 16 KB from
+    // 512 on (bf16, 256 / 512 rows: 4096 3.2 / 4.1 -> 3.0 / 3.8 us, 896 2.8 / 3.2 -> 2.9 / 3.0, 8192 5.1 / 7.4 -> 5.2 / 6.1).
+    // fp32 rows of up to 4 KB from 1024 on (896: 5.7 -> 4.1 us); longer ones leave too few warps in flight (4093 x 4096: 26.5
+    // against 34.7 us staged). With the residual's second stream the CTA per row is not slower.
+    if (staged && !delta && D % 8 == 0 && (!w || aligned(w, 16))) {
+        if constexpr (sizeof(T) == 2) {
+            if (row_bytes <= STAGED_ROW_MAX && rows >= 512) {
+                auto kern = w ? rms_norm_staged_warp_kernel<T, true> : rms_norm_staged_warp_kernel<T, false>;
+                const dim3 wgrid((unsigned)((rows + STAGED_ROWS - 1) / STAGED_ROWS)), wblock(32 * STAGED_ROWS);
+                launch_overlapped(kern, wgrid, wblock, STAGED_ROWS * row_bytes, st, xp, wp, op, (long long)rows, (int)D, eps);
+                return check_launch("bi_rms_norm");
+            }
+        } else if (D <= WARP_ROW_MAX && rows >= 1024) {
+            auto kern = w ? rms_norm_warp_kernel<true> : rms_norm_warp_kernel<false>;
+            const dim3 wgrid((unsigned)((rows + WARP_ROWS - 1) / WARP_ROWS)), wblock(32 * WARP_ROWS);
+            launch_overlapped(kern, wgrid, wblock, 0, st, xp, wp, op, (long long)rows, (int)D, eps);
+            return check_launch("bi_rms_norm");
+        }
     }
     dim3 grid((unsigned)rows), block(TG);
 #define BI_RMS_LAUNCH2(ST, HW, HR)                                                                  \

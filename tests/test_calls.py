@@ -29,3 +29,22 @@ def test_arguments(name):
         fn(*[0.5] * len(values))
     with pytest.raises(OverflowError):
         fn(*[2 ** 70] * len(values))
+
+
+SIZES = ["bi_matmul_scratch_bytes", "bi_qmm_scratch_bytes", "bi_attn_decode_workspace_bytes"]
+
+
+@pytest.mark.parametrize("name", ["bi_rms_norm", "bi_add_rms_norm", "bi_matmul", "bi_matmul_bias", "bi_qmm", "bi_attn_decode", "bi_attn_prefill"] + SIZES)
+def test_none_is_a_null_pointer_and_nothing_else(name):
+    """Slot by slot: None and integers where the prototype has a pointer, numbers where it has one, as through ctypes.
+    Integers are zero, so that a call which takes all its arguments does nothing or reports an error."""
+    fn, args = getattr(_lib.calls(), name), _lib.SIGNATURES[name][1]
+    zeros = [None if a is _lib.c_void_p else 0 for a in args]
+    for i, a in enumerate(args):
+        for value, pointer, number in ((None, True, False), (0.0, False, a is _lib.c_float), ("0", False, False)):
+            values = zeros[:i] + [value] + zeros[i + 1:]
+            if pointer if a is _lib.c_void_p else number:
+                assert isinstance(fn(*values), int), (i, value)
+            else:
+                with pytest.raises(TypeError):
+                    fn(*values)

@@ -143,7 +143,7 @@ def calls():
             try:
                 from . import _calls
             except ImportError as e:
-                raise RuntimeError(f"{LIB_PATH.parent / '_calls.so'} is missing: build it with `python -m mlx_batch_invariant_b200.build`") from e
+                raise RuntimeError(f"the _calls module beside {LIB_PATH} is missing: build it with `python -m mlx_batch_invariant_b200.build`") from e
             _calls.bind(lib._handle)
             _bound = _calls
     return _bound

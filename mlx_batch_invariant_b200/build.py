@@ -1,5 +1,5 @@
-"""Build libbi_b200.so (the C-ABI kernel library) in-tree with nvcc for sm_100a, and _calls.so (the CPython face of its
-hot entry points) with the C compiler.
+"""Build libbi_b200.so (the C-ABI kernel library) in-tree with nvcc for sm_100a, and beside it the CPython face of its hot
+entry points (csrc/calls.c) for the interpreter that runs this, named with its ABI tag.
 
     python -m mlx_batch_invariant_b200.build          # rebuild if sources changed
     python -m mlx_batch_invariant_b200.build --force
@@ -22,7 +22,7 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OUT = PKG / "libbi_b200.so"
-CALLS = PKG / "_calls.so"
+CALLS = PKG / ("_calls" + sysconfig.get_config_var("EXT_SUFFIX"))     # another Python version looks for another name
 OBJ = PKG / "build"
 SOURCES = ["abi.cu", "rmsnorm.cu", "attention.cu", "attn_prefill.cu", "attn_decode_static.cu", "matmul_simt.cu", "matmul_tc.cu", "matmul_pair.cu", "dequant.cu", "matmul.cu", "glue.cu", "peer.cu"]
 
@@ -45,20 +45,39 @@ def _sources() -> list[Path]:
     return [CSRC / s for s in SOURCES if (CSRC / s).exists()]
 
 
-def _fingerprint() -> str:
+def _fingerprint(sources: list[Path], *flags: str) -> str:
     h = hashlib.sha256()
-    for p in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.c")) + [PKG.parent / "include" / "bi_abi.h"]):
+    for p in sorted(sources + [PKG.parent / "include" / "bi_abi.h"]):
         h.update(p.name.encode())
         h.update(p.read_bytes())
-    h.update(" ".join(NVCC_FLAGS).encode())
-    h.update(sys.version.encode())
+    h.update(" ".join(flags).encode())
     return h.hexdigest()
 
 
+def _is_fresh(out: Path, stamp: Path, fp: str) -> bool:
+    return out.exists() and stamp.exists() and stamp.read_text() == fp
+
+
+def build_calls(force: bool = False) -> Path:
+    """The CPython module, by nvcc's host compiler (what links the library also compiles this); rebuilt on its own."""
+    src = CSRC / "calls.c"
+    flags = ["-shared", "-cudart", "none", "-O2", "-Xcompiler", "-fPIC,-Wall", "-I", sysconfig.get_paths()["include"]]
+    stamp, fp = OBJ / (CALLS.name + ".txt"), _fingerprint([src], *flags, sys.version)
+    (PKG / "_calls.so").unlink(missing_ok=True)          # without a tag any Python would import it
+    if force or not _is_fresh(CALLS, stamp, fp):
+        OBJ.mkdir(exist_ok=True)
+        r = subprocess.run([_nvcc(), *flags, "-o", str(CALLS), str(src), "-ldl"], capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"nvcc failed for {src.name}:\n{r.stdout}\n{r.stderr}")
+        stamp.write_text(fp)
+    return CALLS
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
+    build_calls(force)
     stamp = OBJ / "fingerprint.txt"
-    fp = _fingerprint()
-    if not force and OUT.exists() and CALLS.exists() and stamp.exists() and stamp.read_text() == fp:
+    fp = _fingerprint(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")), *NVCC_FLAGS)
+    if not force and _is_fresh(OUT, stamp, fp):
         return OUT
     OBJ.mkdir(exist_ok=True)
     nvcc = _nvcc()
@@ -80,11 +99,6 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     r = subprocess.run([nvcc, "-shared", "-o", str(OUT), *map(str, objs)], capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    cc = os.environ.get("CC") or shutil.which("gcc") or shutil.which("cc") or "gcc"
-    r = subprocess.run([cc, "-O2", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], "-o", str(CALLS), str(CSRC / "calls.c"), "-ldl"],
-                       capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"{cc} failed for calls.c:\n{r.stdout}\n{r.stderr}")
     stamp.write_text(fp)
     return OUT
 

@@ -1,5 +1,8 @@
 """The CPython face of the hot entry points: the same functions as through ctypes, and its argument checks."""
 
+import sysconfig
+from pathlib import Path
+
 import pytest
 
 from mlx_batch_invariant_b200 import _lib
@@ -48,3 +51,9 @@ def test_none_is_a_null_pointer_and_nothing_else(name):
             else:
                 with pytest.raises(TypeError):
                     fn(*values)
+
+
+def test_the_module_is_this_interpreters():
+    """Its name carries the interpreter's ABI tag, so that another Python does not import it."""
+    module = Path(_lib.calls().__file__)
+    assert module.name == "_calls" + sysconfig.get_config_var("EXT_SUFFIX") and not (module.parent / "_calls.so").exists()

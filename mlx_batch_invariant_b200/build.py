@@ -59,12 +59,16 @@ def _is_fresh(out: Path, stamp: Path, fp: str) -> bool:
 
 
 def build_calls(force: bool = False) -> Path:
-    """The CPython module, by nvcc's host compiler (what links the library also compiles this); rebuilt on its own."""
+    """The CPython module, by nvcc's host compiler (what links the library also compiles this); rebuilt on its own. Without
+    Python's headers there is none, and _lib.py calls the library through ctypes."""
     src = CSRC / "calls.c"
     flags = ["-shared", "-cudart", "none", "-O2", "-Xcompiler", "-fPIC,-Wall", "-I", sysconfig.get_paths()["include"]]
     stamp, fp = OBJ / (CALLS.name + ".txt"), _fingerprint([src], *flags, sys.version)
     (PKG / "_calls.so").unlink(missing_ok=True)          # without a tag any Python would import it
     if force or not _is_fresh(CALLS, stamp, fp):
+        if not (Path(flags[-1]) / "Python.h").exists():
+            sys.stderr.write(f"no Python.h in {flags[-1]}: {CALLS.name} is not built\n")
+            return CALLS
         OBJ.mkdir(exist_ok=True)
         r = subprocess.run([_nvcc(), *flags, "-o", str(CALLS), str(src), "-ldl"], capture_output=True, text=True)
         if r.returncode != 0:

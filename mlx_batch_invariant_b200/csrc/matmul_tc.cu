@@ -199,7 +199,8 @@ __device__ __forceinline__ void dequant_row64_to_tmem(const uint8_t* raw, int ro
     constexpr int PIECES = BLOCK_K * QBITS / 8 / 16;     // 16-byte pieces behind 64 codes: 2 (4-bit) or 4 (8-bit)
     constexpr int HP = PIECES / 2;                       // pieces behind 32 codes
     constexpr int WORDS = QBITS / 4;                     // words behind eight codes
-    const bool packed = __all_sync(0xffffffffu, dequant_exact<T, QBITS>(scales & 0xffffu, biases & 0xffffu) && dequant_exact<T, QBITS>(scales >> 16, biases >> 16));
+    bool packed = __all_sync(0xffffffffu, dequant_exact<T, QBITS, false>(scales, biases));
+    if (!packed) packed = __all_sync(0xffffffffu, dequant_exact<T, QBITS, true>(scales, biases));
     auto half = [&](int h, auto&& eight) {               // 32 codes -> 16 columns
         uint32_t o[16];
 #pragma unroll
@@ -223,7 +224,7 @@ __device__ __forceinline__ void dequant_row64_to_tmem(const uint8_t* raw, int ro
             half(h, [&](const uint32_t* w) { return dequant8_packed<T, QBITS>(w, sh, bh); });
         }
     } else {
-#pragma unroll 1
+#pragma unroll
         for (int h = 0; h < 2; ++h) {
             const float sf = word16_up<T>(h ? scales >> 16 : scales & 0xffffu), bf = word16_up<T>(h ? biases >> 16 : biases & 0xffffu);
             const uint64_t s2 = ptx::pack2(sf, sf), b2 = ptx::pack2(bf, bf);

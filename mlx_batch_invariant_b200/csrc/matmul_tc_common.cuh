@@ -125,13 +125,17 @@ __device__ __forceinline__ uint4 dequant8(const uint32_t* words, uint64_t s2, ui
 // sequence rounds it to fp32 and then to T. The two agree whenever the fp32 fma is exact, that is when all bits of the
 // product (code bits + the scale's) and of the bias lie within 24 binary places of each other -- a bound on the difference
 // of the two exponents, which every group of an ordinary weight keeps (the bias is a few steps of the scale) -- or when the
-// bias is zero. Groups outside it, scales that are not normal numbers or too large to be shifted as below, infinities and
-// NaN take dequant8.
+// bias or the scale is zero. Groups outside it and scales that are subnormal or too large to be shifted as below (infinities
+// and NaN among them) take dequant8. A bias that is infinite or NaN passes beside a large scale: the products are finite, so
+// either form gives that bias back.
 // Why: eight 4-bit codes take 15 instructions (a shift, two masks, four permutes, four multiplies, four fmas) instead of 23,
-// none of them a conversion and half of them on the FP32 pipe instead of the integer one. The streaming staging is bound by
-// the dequantizers' instructions: 4 bits, group 64, 4096 -> 28672 at 1 / 64 rows 50.4 -> 46.3 / 72.4 -> 65.4 us, 14336 -> 4096
-// 27.6 -> 25.7 / 51.4 -> 48.5 us; the decoder's step at 64 sequences 7.91 -> 7.45 ms. The tile body (more than 64 rows) keeps dequant8: its long layers were up to 8 % slower
-// with this (4096 -> 28672 at 100 rows: 101 against 110 us), its short ones 6 - 12 % faster.
+// none of them a conversion and half of them on the FP32 pipe instead of the integer one. Packed weights of group 64 that are
+// not in L2, without -> with, 1 / 64 rows: 4 bits, 4096 -> 14336 25.3 -> 23.6 / 39.0 -> 35.5 us, 14336 -> 4096 27.8 -> 25.1 /
+// 51.3 -> 47.9 us; 8 bits 26.4 -> 25.2 / 38.8 -> 36.2, 27.7 -> 25.9 / 53.3 -> 51.1 us. The test itself counts: as scalar
+// code for each half it cost 0.5 to 1 us of that. Where every warp meets a group that takes dequant8 a call is 3 - 8 % slower
+// than without all this at 1 and 16 rows (4096 -> 14336, 4 bits 25.7 -> 27.5 us, 8 bits 26.4 -> 28.7 us), and not at 64.
+// The tile body (more than 64 rows) keeps dequant8: its long layers were up to 8 % slower with this (4096 -> 28672 at 100
+// rows: 101 against 110 us), its short ones 6 - 12 % faster.
 template <typename T> struct Half2;
 template <> struct Half2<__nv_bfloat16> {
     static constexpr uint32_t UP = 0x7F007F00u, DOWN = 0x42804280u;    // 2^127 and 2^6: an integer as a bit pattern is itself times 2^-133
@@ -145,13 +149,22 @@ template <> struct Half2<__half> {
     static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) { uint32_t r; asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
     static __device__ __forceinline__ uint32_t fma(uint32_t a, uint32_t b, uint32_t c) { uint32_t r; asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c)); return r; }
 };
-// Scale and bias as the 16-bit words they are in memory. With scale exponent es and bias exponent eb (M = stored mantissa
-// bits, Q = code bits) the sum's bits lie between 2^(min(es, eb) - M) and 2^(max(es + Q + 1, eb + 1) + 1).
-template <typename T, int QBITS>
-__device__ __forceinline__ bool dequant_exact(uint32_t scale, uint32_t bias) {
+// Two scales and two biases as the 16-bit words they are in memory. With scale exponent es and bias exponent eb (M = stored
+// mantissa bits, Q = code bits) the sum's bits lie between 2^(min(es, eb) - M) and 2^(max(es + Q + 1, eb + 1) + 1). Bit 14 of
+// each half says that a difference is not negative. ZEROS: a bias or scale of zero leaves nothing to round, wherever the
+// other lies.
+template <typename T, int QBITS, bool ZEROS>
+__device__ __forceinline__ bool dequant_exact(uint32_t scales, uint32_t biases) {
     using H = Half2<T>;
-    const int es = (int)(scale >> H::MANT) & H::EXP, d = es - ((int)(bias >> H::MANT) & H::EXP);
-    return es >= H::EXP_LO && es <= H::EXP_HI && ((bias & 0x7fffu) == 0u || (d <= 24 - H::MANT - QBITS - 2 && -d <= 24 - H::MANT - 2));
+    constexpr uint32_t BOTH = 0x00010001u, TOP = 0x4000u * BOTH, EXPS = H::EXP * BOTH;
+    constexpr uint32_t BELOW = (24 - H::MANT - QBITS - 2) * BOTH, ABOVE = (24 - H::MANT - 2) * BOTH;     // how far the bias may lie
+    const uint32_t es = (scales >> H::MANT) & EXPS, eb = (biases >> H::MANT) & EXPS;
+    const uint32_t in_range = (es + (TOP - H::EXP_LO * BOTH)) & ((TOP + H::EXP_HI * BOTH) - es);
+    uint32_t near = (eb - es + (TOP + BELOW)) & (es - eb + (TOP + ABOVE));
+    if (!ZEROS) return (in_range & near & TOP) == TOP;
+    const uint32_t magnitudes = 0x7fff7fffu;
+    const uint32_t bias0 = ~((biases & magnitudes) + magnitudes) >> 1, scale0 = ~((scales & magnitudes) + magnitudes) >> 1;
+    return (((in_range & (near | bias0)) | scale0) & TOP) == TOP;
 }
 template <typename T> __device__ __forceinline__ uint32_t dequant_scale(uint32_t scale2) { return Half2<T>::mul(scale2, Half2<T>::DOWN); }
 template <int SEL> __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b) {   // a selector nibble with bit 3 set gives the byte's sign, eight times

@@ -609,18 +609,26 @@ __global__ void __launch_bounds__(32 * MAXW) decode_warp_stream_kernel(
 //     exp(-|s - m|) -- 32 exponentials per instruction instead of one;
 //   * accumulation: lane d owns dims 4d..4d+3 of all NH heads and walks the block's keys in order:
 //     l = fma(l, corr, p), acc = fma(acc, corr, p * v), the factors read back from shared memory.
-// A warp is one work item (batch, kv head, chunk of NH heads, split) at a time; the items that hold keys are dealt to a
-// persistent grid round-robin, full splits first.
+// A warp is one work item (batch, kv head, chunk of NH heads, split) at a time; the items are dealt to a persistent grid
+// round-robin, full splits first (KLDeal).
 // Launch-shape constants, from measurements on B200 (bf16, 32/8 heads): two K blocks per warp beat one (eight and ten
 // warps with one K block: 53.7 / 65.7 us against 50.1 us with seven warps and two at 64 x 560 keys; ten warps cap the
 // kernel at 168 registers). Eight warps with two K blocks fit once the softmax factors of a block live in that
 // block's own K buffer, which nothing reads after the scores.
-constexpr int KL_WARPS = 8;    // most warps per CTA (one CTA per SM): two per scheduler. With few items the launch uses seven:
-                               // each warp is then faster and the tail is what counts (64 x 560 keys: 50.1 us with
-                               // seven, 53.2 with eight; 64 x 4096 keys: 268 against 248 us)
+constexpr int KL_WARPS = 8;    // most warps per CTA (one CTA per SM): two per scheduler
+// Warps for `items` of one size on `ctas` SMs. With few items seven: each is then faster and the tail is what counts (64 x 560
+// keys: 50.1 us with seven, 53.2 with eight; 64 x 4096 keys: 268 against 248 us); eight where each has two items or the eighth
+// saves a round (9 x 4096 keys, 1152 items: 72 us with seven, 46 with eight).
+__host__ __device__ constexpr int kl_warps(long long items, long long ctas) {
+    const long long fit7 = ctas * (KL_WARPS - 1), fit8 = ctas * KL_WARPS;
+    return items >= 2 * fit8 || (items + fit8 - 1) / fit8 < (items + fit7 - 1) / fit7 ? KL_WARPS : KL_WARPS - 1;
+}
 constexpr int KL_KBUFS = 2;    // K blocks in shared memory per warp: the next block is fetched a whole block ahead
 constexpr int KL_UNROLL = 8;   // keys of the accumulation loop in flight
 constexpr int KL_KEYS = 32;
+// Which items there are: those of the capacity, which all sequences fill; those of the capacity, skipping what a sequence's
+// length leaves empty; or only those that hold keys, looked up in the lengths (KLItems).
+enum KLDeal { KL_ALL, KL_CAPACITY, KL_LISTED };
 struct KLCfg {
     static constexpr int ROWB = 256;                       // bytes of a K or V row (128 x 16 bit)
     static constexpr int KPITCH = ROWB + 16;               // lanes read different rows at one column: no bank conflict
@@ -670,59 +678,79 @@ __device__ __forceinline__ void kl_node(const uint8_t* krow, const uint8_t* qs, 
     for (int h = 0; h < NH; ++h) out[h] = ptx::add2_rn(a[h], b[h]);
 }
 
-// The work items of a warp when the sequences differ in length, in ascending order: item i of the launch is (sequence, split,
-// kv head, chunk of query heads), the full splits of all sequences first, then the partly filled ones. Only splits that hold
-// keys are counted, from the lengths in device memory: a warp keeps the inclusive item counts of 32 sequences in its lanes
-// and moves on to the next 32, whose lengths are already on their way, when its index has passed them.
+// The work items of sequences that bring lengths: item i of the launch is (sequence, split, kv head, chunk of query heads),
+// the full splits of all sequences first, then the partly filled ones. Only splits that hold keys are counted, from the
+// lengths in device memory: every warp sums them once, 32 sequences at a time, lane g keeping the items up to and with group
+// g; an item's group is then a vote over the lanes, its sequence a scan over the group's lengths, which were fetched while
+// the item before was worked on.
+constexpr int KL_LISTED_MAX = 1024;                        // most sequences: a group per lane
 struct KLItems {
     const int32_t* kv_lens;
     int B, L, split, per_seq;                              // per_seq: items of one split of a sequence (kv heads x chunks)
-    int phase, b0, len, ahead, incl;                       // this lane: length and inclusive item count of sequence b0 + lane
-    long long before;                                      // items in front of sequence b0
-    __device__ __forceinline__ int fetch(int from) const {
-        const int b = from + (int)(threadIdx.x & 31);
-        return b < B ? kv_lens[b] : 0;
+    int full, part, nfull, nall;                           // inclusive counts of this lane's group; all full ones; all (an item has a partial in the workspace)
+    int len;                                               // of this lane's sequence in the next item's group
+    __device__ __forceinline__ int fetch(int g) const {
+        const int b = g * 32 + (int)(threadIdx.x & 31);
+        return b < B ? max(0, min(kv_lens[b], L)) : 0;
     }
-    __device__ __forceinline__ void count() {
-        const int lane = threadIdx.x & 31;
-        len = min(ahead, L);
-        ahead = fetch(b0 + 32 < B ? b0 + 32 : 0);
-        incl = (phase ? (len > 0 && len % split ? 1 : 0) : max(len, 0) / split) * per_seq;
+    __device__ __forceinline__ int scan(int x) const {
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, off);
-            if (lane >= off) incl += y;
+            const int y = __shfl_up_sync(0xffffffffu, x, off);
+            if ((int)(threadIdx.x & 31) >= off) x += y;
         }
+        return x;
     }
-    __device__ __forceinline__ KLItems(const int32_t* lens, int B_, int L_, int split_, int per_seq_)
-        : kv_lens(lens), B(B_), L(L_), split(split_), per_seq(per_seq_), phase(L_ < split_ ? 1 : 0), b0(0), len(0), ahead(fetch(0)), incl(0), before(0) { count(); }
-    // item `i` (never smaller than in the call before): sequence, split, index among the split's per_seq items, keys
-    __device__ __forceinline__ bool find(long long i, int& b, int& sp, int& sub, int& nk) {
-        while (true) {
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            if (i < before + total) break;
-            before += total;
-            b0 += 32;
-            if (b0 >= B) {
-                if (phase) return false;
-                phase = 1;
-                b0 = 0;
+    __device__ __forceinline__ int group(int i) const {    // of item `i` of nall
+        return __ffs(__ballot_sync(0xffffffffu, i < nfull ? i < full : i - nfull < part)) - 1;
+    }
+    __device__ __forceinline__ void look_ahead(int i) { if (B > 32) len = fetch(group(i)); }
+    __device__ __forceinline__ KLItems(const int32_t* lens, int B_, int L_, int split_, int per_seq_, long long item)
+        : kv_lens(lens), B(B_), L(L_), split(split_), per_seq(per_seq_), full(0), part(0), len(0) {
+        const int lane = threadIdx.x & 31;
+        nfull = nall = 0;
+        for (int g0 = 0; g0 * 32 < B; g0 += 4) {           // four groups' lengths in flight
+            int n[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) n[j] = fetch(g0 + j);
+            if (g0 == 0) len = n[0];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int g = g0 + j;
+                if (g * 32 >= B) break;
+                const int f = n[j] / split, r = n[j] - f * split ? 1 : 0;
+                nfull += __reduce_add_sync(0xffffffffu, f) * per_seq;
+                nall += __reduce_add_sync(0xffffffffu, r) * per_seq;
+                if (lane >= g) { full = nfull; part = nall; }          // the lanes behind the last group hold all
             }
-            count();
         }
-        const int r = (int)(i - before);
+        nall += nfull;
+        if (item < nall) look_ahead((int)item);
+    }
+    // item `i` of nall, the one asked for in the call before (or at the start): sequence, split, index among the split's
+    // per_seq items, keys. `next` is what the next call asks for.
+    __device__ __forceinline__ void find(int i, long long next, int& b, int& sp, int& sub, int& nk) {
+        const bool ph = i >= nfull;
+        int g = 0, r = i - (ph ? nfull : 0);
+        if (B > 32) {
+            g = group(i);
+            const int before = __shfl_sync(0xffffffffu, ph ? part : full, max(g - 1, 0));
+            r -= g ? before : 0;
+        }
+        const int f = len / split;
+        const int incl = scan((ph ? (len - f * split ? 1 : 0) : f) * per_seq);
         const int src = __ffs(__ballot_sync(0xffffffffu, r < incl)) - 1;
         const int prev = __shfl_sync(0xffffffffu, incl, max(src - 1, 0)), n = __shfl_sync(0xffffffffu, len, src);
         const int rel = r - (src ? prev : 0);
-        b = b0 + src;
-        sp = phase ? n / split : rel / per_seq;
-        sub = phase ? rel : rel - sp * per_seq;
-        nk = phase ? n - sp * split : split;
-        return true;
+        b = g * 32 + src;
+        sp = ph ? n / split : rel / per_seq;
+        sub = ph ? rel : rel - sp * per_seq;
+        nk = ph ? n - sp * split : split;
+        if (next < nall) look_ahead((int)next);
     }
 };
 
-template <typename T, int NH, int NW, bool LENS>
+template <typename T, int NH, int NW, KLDeal DEAL>
 __global__ void __launch_bounds__(32 * NW, 1) decode_keylane_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const int32_t* __restrict__ kv_lens,
     float* __restrict__ pm, float* __restrict__ pl, float* __restrict__ pacc, int B, int Hq, int Hkv, int L,
@@ -743,18 +771,23 @@ __global__ void __launch_bounds__(32 * NW, 1) decode_keylane_kernel(
     const long long per_split = (long long)B * Hkv * nchunk;
     const long long items = per_split * nsplit;
 
-    // Where items differ in length, consecutive ones go to different SMs: an SM's share of the keys is then close to the mean
-    // (64 sequences of 1 ... 4096 keys: 168 -> 125 us; 64 x 561 keys, whose last splits hold 49: 48.1 -> 46.4 us). Items of
-    // one length are as many an SM either way; its warps then take neighbours, the kv heads of one sequence (64 x 4096 keys
-    // 240 us, 245 dealt apart).
-    const bool apart = LENS || L % split != 0;
-    long long item = apart ? (long long)wid * gridDim.x + blockIdx.x : (long long)blockIdx.x * NW + wid;
-    KLItems work(kv_lens, LENS ? B : 0, L, split, Hkv * nchunk);
-    for (;; item += (long long)gridDim.x * NW) {
+    // Consecutive items go to different SMs: an SM's share of the keys is then close to the mean where items differ in length
+    // (64 sequences of 1 ... 4096 keys dealt over the capacity: 235 us with neighbours on an SM, 193 so, 141 with only the
+    // items that hold keys; 64 x 561 keys, whose last splits hold 49: 49.3 -> 46.6), and no worse where they do not (64 x
+    // 4096 keys 244 us either way, 256 x 512 146 -> 134).
+    long long item = (long long)wid * gridDim.x + blockIdx.x;
+    KLItems work(kv_lens, DEAL == KL_LISTED ? B : 0, L, split, Hkv * nchunk, item);
+    // all of the listed items full splits: as many warps as for that capacity (8 x 8192 keys 84 us with eight, 82 with seven
+    // of them)
+    const int warps = DEAL == KL_LISTED && NW == KL_WARPS && work.nall == work.nfull ? kl_warps(work.nall, gridDim.x) : NW;
+    if (DEAL == KL_LISTED && wid >= warps) return;
+    const long long stride = (long long)gridDim.x * warps;
+    for (;; item += stride) {
         int b, sp, hk, chunk, nk;                                            // warp-uniform
-        if (LENS) {
+        if (DEAL == KL_LISTED) {
+            if (item >= work.nall) break;
             int sub;
-            if (!work.find(item, b, sp, sub, nk)) break;
+            work.find((int)item, item + stride, b, sp, sub, nk);
             hk = sub / nchunk;
             chunk = sub - hk * nchunk;
         } else {
@@ -764,7 +797,9 @@ __global__ void __launch_bounds__(32 * NW, 1) decode_keylane_kernel(
             chunk = (int)(u % nchunk); u /= nchunk;
             hk = (int)(u % Hkv);
             b = (int)(u / Hkv);
-            nk = min(L, sp * split + split) - sp * split;
+            const int Lb = DEAL == KL_CAPACITY ? min(kv_lens[b], L) : L;
+            if (DEAL == KL_CAPACITY && Lb <= sp * split) continue;
+            nk = min(Lb, sp * split + split) - sp * split;
         }
         const int j0 = sp * split;
         const int h0 = hk * G + chunk * NH;
@@ -990,16 +1025,17 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
                 if (nh > 1 && B * Hkv * ((G + nh - 1) / nh) * nsplit < sms * 4) nh = 1;
                 const int nck = (G + nh - 1) / nh;
                 const int64_t items = B * Hkv * nck * nsplit;
-                // Seven warps where an SM has fewer than two items for each of eight, unless the eighth saves a round: 9 x
-                // 4096 keys, 1152 items, 69 us with seven and 43.5 with eight. How many items sequences of different
-                // length have is known on the device only: more than one round of them if all were full takes eight (8 x
-                // 1 ... 8192 keys: 60 us with seven, 45 with eight; where both are one round eight costs about 2 %).
-                const int64_t fit7 = sms * (KL_WARPS - 1), fit8 = sms * KL_WARPS;
-                const int nw = (kv_lens ? items > fit7 : items >= 2 * fit8 || (items + fit8 - 1) / fit8 < (items + fit7 - 1) / fit7) ? KL_WARPS : KL_WARPS - 1;
+                // Sequences that bring lengths are looked up where a sequence can have more than one split: with one there is
+                // nothing to skip but the sequence (256 x <= 256 keys: 71 us over the capacity, 75 looked up; <= 16 keys each
+                // 22.9 against 26.7). Beyond KL_LISTED_MAX sequences every warp has many items of either kind (4096 x <= 300
+                // keys: 771 us over the capacity, 827 looked up). How many items there are is known on the device only:
+                // the launch has eight warps a CTA unless seven hold all that the capacity can.
+                const bool listed = kv_lens && nsplit > 1 && B <= KL_LISTED_MAX;
+                const int nw = listed ? (items > sms * (KL_WARPS - 1) ? KL_WARPS : KL_WARPS - 1) : kl_warps(items, sms);
                 const int64_t ctas = std::min<int64_t>(sms, (items + nw - 1) / nw);
-#define BI_KL_LAUNCH(NHV, NWV, LENSV)                                                                                         \
+#define BI_KL_LAUNCH(NHV, NWV, DEALV)                                                                                         \
     do {                                                                                                                \
-        auto kern = decode_keylane_kernel<T, NHV, (NWV), LENSV>;                                                              \
+        auto kern = decode_keylane_kernel<T, NHV, (NWV), DEALV>;                                                              \
         static bool attr_set[64] = {false};                                                                             \
         int dev_ = 0;                                                                                                   \
         cudaGetDevice(&dev_);                                                                                           \
@@ -1012,9 +1048,10 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
         launch_overlapped(kern, dim3((unsigned)ctas), dim3(32 * (NWV)), (size_t)((NWV) * KLCfg::WARP_BYTES), st, qp, kp, vp, kv_lens, pm, pl, pacc, \
                           (int)B, (int)Hq, (int)Hkv, (int)L, lay, scale, split, nsplit, nck);                           \
     } while (0)
-#define BI_KL_LAUNCH_NH(NWV, LENSV) do { if (nh == 4) BI_KL_LAUNCH(4, NWV, LENSV); else if (nh == 2) BI_KL_LAUNCH(2, NWV, LENSV); else BI_KL_LAUNCH(1, NWV, LENSV); } while (0)
-                if (kv_lens) { if (nw == KL_WARPS) BI_KL_LAUNCH_NH(KL_WARPS, true); else BI_KL_LAUNCH_NH(KL_WARPS - 1, true); }
-                else { if (nw == KL_WARPS) BI_KL_LAUNCH_NH(KL_WARPS, false); else BI_KL_LAUNCH_NH(KL_WARPS - 1, false); }
+#define BI_KL_LAUNCH_NH(NWV, DEALV) do { if (nh == 4) BI_KL_LAUNCH(4, NWV, DEALV); else if (nh == 2) BI_KL_LAUNCH(2, NWV, DEALV); else BI_KL_LAUNCH(1, NWV, DEALV); } while (0)
+                if (listed) { if (nw == KL_WARPS) BI_KL_LAUNCH_NH(KL_WARPS, KL_LISTED); else BI_KL_LAUNCH_NH(KL_WARPS - 1, KL_LISTED); }
+                else if (kv_lens) { if (nw == KL_WARPS) BI_KL_LAUNCH_NH(KL_WARPS, KL_CAPACITY); else BI_KL_LAUNCH_NH(KL_WARPS - 1, KL_CAPACITY); }
+                else { if (nw == KL_WARPS) BI_KL_LAUNCH_NH(KL_WARPS, KL_ALL); else BI_KL_LAUNCH_NH(KL_WARPS - 1, KL_ALL); }
 #undef BI_KL_LAUNCH_NH
 #undef BI_KL_LAUNCH
                 int rck = check_launch("bi_attn_decode (key per lane)");

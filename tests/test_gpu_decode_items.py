@@ -14,9 +14,10 @@ def bi():
 
 
 # (sequences, capacity, heads, kv heads): one and several groups of 32 sequences, a capacity below, at and above one split
-# and two; few items (a warp per head) and more than a round of them
+# and two; few items (a warp per head) and more than a round of them; the last batch that is looked up and the first that is
+# dealt over the capacity; equal lengths on seven of eight warps
 CASES = [(1, 300, 8, 2), (5, 33, 8, 8), (31, 256, 8, 2), (32, 257, 4, 1), (33, 511, 8, 2), (64, 512, 32, 8), (65, 700, 8, 2),
-         (130, 640, 14, 2), (9, 4096, 32, 8)]
+         (130, 640, 14, 2), (9, 4096, 32, 8), (1024, 257, 2, 1), (1025, 257, 2, 1), (8, 8192, 32, 8)]
 
 
 @pytest.mark.parametrize("B,L,Hq,Hkv", CASES)

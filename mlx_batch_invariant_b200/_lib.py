@@ -136,7 +136,7 @@ _bound = None
 
 def calls():
     """The hot entry points of the loaded library as C functions of a CPython module (csrc/calls.c): same arguments, a
-    quarter of ctypes' cost a call. Where there is no module for this interpreter they are the library's own, through the
+    tenth of ctypes' cost a call. Where there is no module for this interpreter they are the library's own, through the
     prototypes above: the same kernels, a few microseconds of host time more."""
     global _bound
     if _bound is None:

@@ -1,5 +1,7 @@
 /* The entry points a decode loop calls over and over, as CPython functions: the same C calls that ctypes makes from the
- * prototypes in _lib.py, without its conversion of every argument through an object (bi_matmul's sixteen: 3.2 -> 0.25 us; a norm of one row, launch included, 10.1 -> 8.6 us).
+ * prototypes in _lib.py, without its conversion of every argument through an object. On a B200's host, a call that launches
+ * nothing: bi_rms_norm 0.75 -> 0.08 us, bi_matmul 1.43 -> 0.11 us; through the wrappers a norm of one row 9.9 -> 9.0 us, a linear
+ * layer of one row, 4096 -> 4096, 19.6 -> 17.0 us.
  * Pointers are integers or None, the interpreter lock is released around the call, the status comes back as an int.
  * bind() takes the functions from the library that _lib.py has loaded. */
 #define PY_SSIZE_T_CLEAN

@@ -29,7 +29,7 @@
 // For affine-quantized weights the TMA ring carries the packed codes (a deep
 // ring of small stages, so enough bytes are in flight to cover HBM latency)
 // and dequantizer warps turn them into the 16-bit weight operand
-// (fma(float(code), scale, bias) in fp32, one rounding --
+// (the bits of fma(float(code), scale, bias) in fp32 and one rounding --
 // mlx_batch_invariant/kernels/quantized.py:44-67), so the MMA sequence is the
 // dense one. Two stagings of that operand exist:
 //   * tile body (batches above 64 rows): eight warps write the same swizzled
@@ -37,7 +37,8 @@
 //   * streaming (decode, up to 64 rows): sixteen warps, one weight row per
 //     thread, write the operand straight into tensor memory (tcgen05.st) and
 //     the MMA reads its weight operand from there, so the dequantized tile
-//     never crosses shared memory and needs no proxy fence.
+//     never crosses shared memory and needs no proxy fence. Its arithmetic is
+//     packed 16-bit fma where that gives the same bits (dequant_exact).
 //
 // The split path can fold in the producing kernel: a CTA that has stored its
 // group partial bumps a per-tile counter, and the CTA that arrives last reads

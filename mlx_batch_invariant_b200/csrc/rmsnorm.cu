@@ -1,4 +1,4 @@
-// RMSNorm, one CTA of 256 threads per row.
+// RMSNorm: one CTA of 256 threads per row, or, for many rows, a warp that stands for those threads.
 //
 // Canonical order per row (identical to the Metal kernel of the reference,
 // mlx_batch_invariant/kernels/rmsnorm.py:19-47):
@@ -6,7 +6,7 @@
 //   tree:      for s = 128, 64, ..., 1: red[t] = red[t] + red[t+s]  (t < s)
 //   inv  = 1 / sqrt(red[0] / float(D) + eps)
 //   out_i = T((x_i * inv) * w_i)          two fp32 multiplies, one rounding
-// How many rows share the launch never enters: a row sees only its own CTA.
+// How many rows share the launch never enters: a row sees only its own CTA, or its own warp.
 //
 // bi_add_rms_norm is the same kernel with a residual add in front: sum_i = T(x_i + delta_i) (fp32 add, one
 // rounding -- what an elementwise add of two T arrays gives), written out, and the norm runs over the
@@ -196,11 +196,13 @@ __device__ __forceinline__ float warp_tree_sum(const float (&ss)[8], int lane) {
 // 16-bit rows of up to 16 KB: the row waits in shared memory, brought by cp.async in two halves (a lane reads only what it
 // copied itself, so nothing but its own wait stands between the copies and the sums). What bounds it: memory, by the bytes in
 // flight. With the row in registers 16 to 20 warps fit an SM (160 KB in flight, and 2400 rows of bf16 took a second wave);
-// staged, 28 rows of 8 KB do, and longer rows no longer fall back to a CTA per row, which spends its time on load, five
-// barriers and store in series. Rows that are not in L2, bf16: 4093 x 4096 13.8 -> 12.7 us (6000: 20.7 -> 17.5; 2400: 12.0 ->
-// 8.5), 4093 x 896 6.6 -> 4.7 us, 4093 x 8192 35.5 -> 26.0 us. Two rows a CTA: four are up to 5 % slower where the last wave
-// is short; one piece of copies instead of two halves, and loops unrolled by four, 5 to 20 % slower.
-constexpr int STAGED_ROWS = 2;
+// staged, 26 rows of 8 KB do (13 CTAs of 16 KB and the 1 KB that a CTA is charged: 3848 rows a wave), and longer rows no
+// longer fall back to a CTA per row, which spends its time on load, five barriers and store in series. Neither rows nor
+// results in L2, bf16: 4093 x 4096 16.7 -> 14.4 us (6000: 23.8 -> 19.0; 2400: 12.9 -> 9.7, fp16 9.0 -> 9.5), 4093 x 896 7.1 ->
+// 5.1 us, 4093 x 8192 34.9 -> 26.5 us, 32768 x 64 29.8 -> 18.3 us. Two rows a CTA: four are up to 5 % slower from 6144 elements
+// on (4093 x 6144 20.4 against 21.4 us) and up to 25 % faster below 512 (32768 x 128 18.3 against 14.1). With results in L2,
+// one piece of copies instead of two halves, and loops unrolled by four, were 5 to 20 % slower.
+constexpr int STAGED_ROWS = 2;                           // 14 CTAs below: a cap of 72 registers, no occupancy is lost to them
 constexpr size_t STAGED_ROW_MAX = 16 * 1024;
 template <typename T, bool HAS_W>
 __global__ void __launch_bounds__(32 * STAGED_ROWS, 14) rms_norm_staged_warp_kernel(const T* x, const T* __restrict__ w, T* out, long long rows,
@@ -255,7 +257,7 @@ __global__ void __launch_bounds__(32 * STAGED_ROWS, 14) rms_norm_staged_warp_ker
 }
 
 // fp32 rows of up to 1024 elements: the row stays in the lane's registers from the load to the store (two 16-byte words a
-// piece; staged like the 16-bit rows 4093 x 896 takes 7.8 against 6.3 us).
+// piece; 4093 x 896, results in L2: 6.3 us, staged like the 16-bit rows 7.8).
 constexpr int WARP_ROWS = 4;
 constexpr int WARP_ROW_MAX = 1024;                       // longest row kept in registers
 template <bool HAS_W>
@@ -399,10 +401,11 @@ int launch(const void* x, const void* delta, const void* w, void* sum_out, void*
     const T* wp = static_cast<const T*>(w);
     T* sp = static_cast<T*>(sum_out);
     T* op = static_cast<T*>(out);
-    // A warp per row once there are rows enough for it, by times over rows that are not in L2. 16-bit rows of up to 16 KB from
-    // 512 on (bf16, 256 / 512 rows: 4096 3.2 / 4.1 -> 3.0 / 3.8 us, 896 2.8 / 3.2 -> 2.9 / 3.0, 8192 5.1 / 7.4 -> 5.2 / 6.1).
-    // fp32 rows of up to 4 KB from 1024 on (896: 5.7 -> 4.1 us); longer ones leave too few warps in flight (4093 x 4096: 26.5
-    // against 34.7 us staged). With the residual's second stream the CTA per row is not slower.
+    // A warp per row once there are rows enough for it, by times over rows and results that are not in L2. 16-bit rows of up to
+    // 16 KB from 512 on: there it is faster at every width (bf16, 256 / 511 rows by a CTA -> by a warp: 4096 4.0 / 4.9 -> 3.9 /
+    // 4.6 us, 896 3.2 / 3.8 -> 3.4 / 3.5, 8192 5.5 / 7.9 -> 5.6 / 6.7, 6144 4.7 / 6.4 -> 4.9 / 5.8). fp32 rows of up to 4 KB from
+    // 1024 on (results in L2, 896: 5.7 -> 4.1 us); longer ones leave too few warps in flight (4093 x 4096: 26.5 against 34.7 us
+    // staged). With the residual's second stream the CTA per row is not slower.
     if (staged && !delta && D % 8 == 0 && (!w || aligned(w, 16))) {
         if constexpr (sizeof(T) == 2) {
             if (row_bytes <= STAGED_ROW_MAX && rows >= 512) {

@@ -771,11 +771,12 @@ __global__ void __launch_bounds__(32 * NW, 1) decode_keylane_kernel(
     const long long per_split = (long long)B * Hkv * nchunk;
     const long long items = per_split * nsplit;
 
-    // Consecutive items go to different SMs: an SM's share of the keys is then close to the mean where items differ in length
-    // (64 sequences of 1 ... 4096 keys dealt over the capacity: 235 us with neighbours on an SM, 193 so, 141 with only the
-    // items that hold keys; 64 x 561 keys, whose last splits hold 49: 49.3 -> 46.6), and no worse where they do not (64 x
-    // 4096 keys 244 us either way, 256 x 512 146 -> 134).
-    long long item = (long long)wid * gridDim.x + blockIdx.x;
+    // Consecutive items go to different SMs where they differ in length: an SM's share of the keys is then close to the mean
+    // (64 sequences of 1 ... 4096 keys dealt over the capacity: 235 us with neighbours on an SM, 193 apart, 141 with only the
+    // items that hold keys; 64 x 561 keys, whose last splits hold 49: 49.3 -> 46.6). Items of one length are as many an SM
+    // either way; its warps then take neighbours, the kv heads of one sequence (64 x 4096 keys 250.8 us, 253.2 apart).
+    const bool apart = DEAL != KL_ALL || L % split != 0;
+    long long item = apart ? (long long)wid * gridDim.x + blockIdx.x : (long long)blockIdx.x * NW + wid;
     KLItems work(kv_lens, DEAL == KL_LISTED ? B : 0, L, split, Hkv * nchunk, item);
     // all of the listed items full splits: as many warps as for that capacity (8 x 8192 keys 84 us with eight, 82 with seven
     // of them)

@@ -1027,10 +1027,11 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
                 const int nck = (G + nh - 1) / nh;
                 const int64_t items = B * Hkv * nck * nsplit;
                 // Sequences that bring lengths are looked up where a sequence can have more than one split: with one there is
-                // nothing to skip but the sequence (256 x <= 256 keys: 71 us over the capacity, 75 looked up; <= 16 keys each
-                // 22.9 against 26.7). Beyond KL_LISTED_MAX sequences every warp has many items of either kind (4096 x <= 300
-                // keys: 771 us over the capacity, 827 looked up). How many items there are is known on the device only:
-                // the launch has eight warps a CTA unless seven hold all that the capacity can.
+                // nothing to skip but the sequence (256 x <= 256 keys: 70 us over the capacity, 72 looked up; <= 16 keys each
+                // 22.8 against 24.5). With more it pays (16 x <= 1024 keys 39 -> 23.5 us, 256 x <= 1500 236 -> 207, 1024 x <=
+                // 600 393 -> 360; many sequences of two splits are about even: 512 x <= 300 128 -> 127, 1024 x <= 300 218 ->
+                // 229), up to the lanes that hold the counts. How many items there are is known on the device only: the launch
+                // has eight warps a CTA unless seven hold all that the capacity can.
                 const bool listed = kv_lens && nsplit > 1 && B <= KL_LISTED_MAX;
                 const int nw = listed ? (items > sms * (KL_WARPS - 1) ? KL_WARPS : KL_WARPS - 1) : kl_warps(items, sms);
                 const int64_t ctas = std::min<int64_t>(sms, (items + nw - 1) / nw);

@@ -989,6 +989,7 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
                   int64_t B, int64_t Hq, int64_t Hkv, int64_t L, const KvLayout& lay, float scale, int split,
                   cudaStream_t st, const PushSink* sink = nullptr) {
     constexpr int D = 32 * DL;
+    split = std::min(split, 1 << 30);                      // the most keys there are: sums with a split stay in 32 bits
     const int G = (int)(Hq / Hkv);
     const int nsplit = (int)((L + split - 1) / split);
     const int64_t BH = B * Hq;

@@ -494,6 +494,7 @@ int launch_prefill(const void* q, const void* k, const void* v, void* out, int64
     // chain is what counts and shorter row blocks are faster (8 heads x 16 queries over 1000 keys: 119 / 75 / 56 us). Four
     // rows of fp32 with 256 dims would take 240 KB of shared memory.
     const int64_t rows = (Hq / Hkv) * Tq, sms = sm_count();
+    if (split > 1 << 30) split = 1 << 30;                  // the most keys there are: sums with a split stay in 32 bits
     auto ctas = [&](int qb) { return B * Hkv * ((rows + qb - 1) / qb); };
     if constexpr (PF<T, DL, 4>::SMEM <= PF_SMEM_MAX) {
         if (ctas(PF<T, DL, 4>::QB) >= 2 * sms) return launch_prefill_tq<T, DL, 4>(q, k, v, out, B, Hq, Hkv, Tq, L, lay, scale, causal, split, st);

@@ -170,3 +170,18 @@ def test_paged_cache_gives_the_bits_of_the_contiguous_cache(bi, dt, page):
     assert R.bits_of(got) == R.bits_of(want)
     flat = bi.batch_invariant_decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5, kv_lens=torch.tensor(lens))
     assert R.bits_of(got) == R.bits_of(flat)
+
+
+@pytest.mark.parametrize("split", [2 ** 31 - 1, 2 ** 31 - 200, 2 ** 30])
+def test_the_largest_splits_are_one_split(bi, split):
+    """A split longer than any cache is one split, also where adding it to a key's index leaves 32 bits."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q = torch.randn(2, 4, 300, 128, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(2, 2, 300, 128, generator=g, device="cuda").bfloat16() for _ in range(2))
+    lens = torch.tensor([300, 17], dtype=torch.int32, device="cuda")
+    for f in (lambda s: bi.batch_invariant_decode_attention(q[:, :, :1], k, v, scale=0.1, split_size=s),
+              lambda s: bi.batch_invariant_decode_attention(q[:, :, :1], k, v, scale=0.1, split_size=s, kv_lens=lens),
+              lambda s: bi.batch_invariant_decode_attention(q[:, :, :1].float(), k.float(), v.float(), scale=0.1, split_size=s, kv_lens=lens),
+              lambda s: bi.batch_invariant_prefill_attention(q, k, v, scale=0.1, causal=True, split_size=s)):
+        got = f(split)
+        assert got.isfinite().all() and torch.equal(got, f(1024))

@@ -10,11 +10,16 @@
 // totals live in the registers of eight epilogue warps (each thread one weight row, half of the batch tile), while
 // the MMAs of the next group fill the other of two accumulators of 256 tensor-memory columns.
 //
-// What bounds it: the copies into shared memory, then the drain of the accumulators. A K step of 64 takes 0.29 us + 1.2 ns per batch row of the tile, the
-// time of its (128 + bm/2) 128-byte rows at 57 GB/s an SM (the same with a quarter of the MMAs; without the copies it
-// takes 0.42 us at bm = 256, the MMAs alone 0.27). One SM per tile (128 x 128, matmul_tc.cu) takes 0.46 us a step for
-// a quarter of the pair's outputs, its partials on a round trip through tensor memory. fp16 1900 x 4096 -> 14336:
-// 357 -> 233 us (958 TFLOP/s); bf16 1024 x 4096 -> 4096: 61 -> 43 us.
+// The finished tile leaves through shared memory: pieces of 16 batch rows x 128 weight rows in a ring of four for each half,
+// one TMA store each. Stored from the registers, 64 bytes a warp instruction, a tile kept the epilogue warps for 9 us, in
+// which the MMAs stood still after two groups: 1900 x 4096 -> 14336 at bm = 256 248 us so, 212 us staged. Outputs whose rows
+// are no whole 16-byte units are still stored that way.
+//
+// What bounds it: a K step of 64 takes 0.2 us or 0.12 us + 0.9 ns per batch row of the tile, whichever is more (bm = 64 / 128 /
+// 256: 0.20 / 0.22 / 0.35, of which the MMAs alone 0.07 / 0.14 / 0.27): at small tiles the chain commit -> drain -> arrival ->
+// next group of the two accumulators, at 256 rows the tensor pipe under the power cap; 8 - 10 us a launch. One SM per tile
+// (128 x 128, matmul_tc.cu) takes 0.46 us a step for a quarter of the pair's outputs. fp16 1900 x 4096 -> 14336: 241 -> 170 us at
+// bm = 224 (1313 TFLOP/s), bf16 1024 x 4096 -> 4096 60 -> 40 us, 1024 x 14336 -> 4096 179 -> 112 us at bm = 128.
 //
 // Every wait is bounded; a wait that runs out records a code in the status word, raises the CTA's abort flag, and the
 // pair meets at the cluster barrier (which every warp reaches) before tensor memory is freed.
@@ -36,6 +41,10 @@ constexpr int W_BYTES = BLOCK_N * BLOCK_K * 2; // one weight operand tile
 constexpr int EPI0 = 4;                        // warps 0-3 issue (setmaxnreg works on whole warpgroups), 4-11 fold
 constexpr int PAIR_THREADS = 32 * (EPI0 + 8);
 constexpr int PAIR_MAX_BM = 256;
+// Output staging: pieces of 16 batch rows x 128 weight rows, four for each half of the batch tile
+constexpr int OUT_ROWS = 16, OUT_BUFS = 4;
+constexpr int OUT_PIECE = OUT_ROWS * BLOCK_N * 2;
+constexpr int OUT_BYTES = 2 * OUT_BUFS * OUT_PIECE;
 // Registers per thread after the split: 128 x 64 + 256 x 216 = 63488 of the 384 x 168 = 64512 launched.
 constexpr int REGS_LAUNCH = 168, REGS_ISSUE = 64, REGS_EPI = 216;
 static_assert(128 * REGS_ISSUE + 256 * REGS_EPI <= PAIR_THREADS * REGS_LAUNCH, "a split above the launch's registers never completes");
@@ -51,6 +60,7 @@ struct PairParams {
     int box3d;            // K % 64 == 0: the tensor maps are [K/64][rows][64] views (else 2-D, one K step per slot)
     int slots;            // ring depth
     int x_bytes;          // shared-memory bytes of a CTA's activation tile (bm / 2 rows of one K step)
+    int staged;           // the output goes through shared memory and TMA (rows of a multiple of 16 bytes)
 };
 
 __device__ __forceinline__ uint32_t cta_rank() {
@@ -67,8 +77,12 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
+// The accumulator's reads are what this arrival reports: they are complete (tcgen05.wait::ld) and ordered by the tcgen05
+// fences on both sides. Nothing that was written is handed over, so no release at cluster scope, which made every arrival
+// wait for a fence of the whole memory system: 0.5 - 1 us on the way from a drained accumulator to the next group's
+// MMAs (fp16 1900 x 4096 -> 14336: 213 us with it, 178 without; bf16 1024 x 14336 -> 4096 at bm = 128: 166 and 112).
 __device__ __forceinline__ void arrive_cluster(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+        asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // Boxes of this GPU's memory into this CTA's shared memory; completion is signalled on `bar`, which may be the peer's.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap, int c0, int c1, uint32_t bar) {
@@ -101,12 +115,14 @@ __device__ __forceinline__ void commit_pair(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
+__device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory"); }
 template <int R> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 template <int R> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
 
 template <typename T, int KS>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
-pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const PairParams p) {
+pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+                   const __grid_constant__ CUtensorMap tmap_out, const PairParams p) {
     ptx::grid_dep_launch();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -114,7 +130,8 @@ pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // weight tiles, then activation tiles (each a multiple of 1024 bytes), then barriers
     const int S = p.slots;
     const uint32_t x_ring = smem_base + (uint32_t)(S * KS) * W_BYTES;
-    const uint32_t bar_base = x_ring + (uint32_t)(S * KS * p.x_bytes);
+    const uint32_t out_base = x_ring + (uint32_t)(S * KS * p.x_bytes);
+    const uint32_t bar_base = out_base + OUT_BYTES;
     auto bar_full = [&](int s) { return bar_base + 8u * s; };                              // first CTA: both CTAs' tiles landed
     auto bar_empty = [&](int s) { return bar_base + 8u * (PAIR_MAX_SLOTS + s); };          // MMAs of the slot complete
     auto bar_tfull = [&](int b) { return bar_base + 8u * (2 * PAIR_MAX_SLOTS + b); };      // accumulator complete
@@ -287,15 +304,18 @@ pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         // ------------------------------------------------------------ epilogue: totals in registers
         regs_inc<REGS_EPI>();
         constexpr int CH = PAIR_MAX_BM / 2 / 16;                     // 16-column pieces of half a batch tile
-        static_assert(CH % 2 == 0, "taken in twos");
+        static_assert(CH % 4 == 0, "read in blocks of 32 columns, two at a time");
         const int quad = warp & 3, half = (warp - EPI0) >> 2;
         const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * xh);
         T* out = static_cast<T*>(p.out);
         const T* bias = static_cast<const T*>(p.bias);
         const uint32_t tempty0 = map_to_rank(bar_tempty(0), 0), tempty1 = map_to_rank(bar_tempty(1), 0);
+        const uint32_t stage = out_base + (uint32_t)(half * OUT_BUFS * OUT_PIECE);
         int job = 0;
+        uint32_t piece = 0;                                          // pieces this half has staged
         bool ok = true;
-        for (int u = first; u < p.units && ok; u += n_clusters) {
+        // No early exit here either: the four warps of a half meet at a barrier for every piece they store.
+        for (int u = first; u < p.units; u += n_clusters) {
             float tot[CH * 16];
 #pragma unroll
             for (int j = 0; j < CH * 16; ++j) tot[j] = 0.0f;
@@ -303,22 +323,23 @@ pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             const int cols = min(xh, p.M - m0);                      // batch rows that exist (may be <= 0)
             for (int g = 0; g < p.G; ++g, ++job) {
                 const int buf = job & 1;
-                if (!wait_bounded(bar_tfull(buf), (uint32_t)(job >> 1) & 1u, ctl, ROLE_EPI, 16 + buf)) { ok = false; break; }
+                ok = ok && wait_bounded(bar_tfull(buf), (uint32_t)(job >> 1) & 1u, ctl, ROLE_EPI, 16 + buf);
+                if (!ok) continue;
                 ptx::tc_fence_after();
                 const uint32_t acc = lane_base + (uint32_t)(buf * PAIR_ACC_STRIDE);
 #pragma unroll
-                for (int c = 0; c < CH; c += 2) {                    // warp-uniform conditions
-                    if (c * 16 < cols) {
-                        uint32_t v0[16], v1[16];
-                        const bool two = (c + 1) * 16 < cols;
-                        ptx::tmem_ld_32x16(acc + c * 16, v0);
-                        if (two) ptx::tmem_ld_32x16(acc + c * 16 + 16, v1);
+                for (int c = 0; c < CH / 2; c += 2) {                // warp-uniform conditions; two blocks of 32 columns share a wait
+                    if (c * 32 < cols) {
+                        uint32_t v0[32], v1[32];
+                        const bool two = (c + 1) * 32 < cols;
+                        ptx::tmem_ld_32x32(acc + c * 32, v0);
+                        if (two) ptx::tmem_ld_32x32(acc + c * 32 + 32, v1);
                         ptx::tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) tot[c * 16 + j] = add_rn(tot[c * 16 + j], __uint_as_float(v0[j]));
+                        for (int j = 0; j < 32; ++j) tot[c * 32 + j] = add_rn(tot[c * 32 + j], __uint_as_float(v0[j]));
                         if (two) {
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) tot[c * 16 + 16 + j] = add_rn(tot[c * 16 + 16 + j], __uint_as_float(v1[j]));
+                            for (int j = 0; j < 32; ++j) tot[c * 32 + 32 + j] = add_rn(tot[c * 32 + 32 + j], __uint_as_float(v1[j]));
                         }
                     }
                 }
@@ -327,13 +348,31 @@ pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 if (lane == 0) arrive_cluster(buf ? tempty1 : tempty0);
             }
             const int n = unit_n0(u) + quad * 32 + lane;
-            if (ok && n < p.N) {
+            if (p.staged) {
+                const T* b = n < p.N ? bias : nullptr;
+#pragma unroll
+                for (int c = 0; c < CH; ++c) {
+                    if (c * 16 < cols) {                             // the same in the four warps of a half
+                        const uint32_t dst = stage + (piece & (OUT_BUFS - 1)) * OUT_PIECE;
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            ptx::st_shared(dst + (uint32_t)(j * BLOCK_N * 2 + (quad * 32 + lane) * 2), round_out<T>(tot[c * 16 + j], b, n));
+                        ptx::fence_proxy_async_smem();
+                        // before the barrier all but the last two copies have read their piece: the next piece is free after it
+                        if (quad == 0 && lane == 0) ptx::bulk_wait_read<OUT_BUFS - 2>();
+                        half_sync(half);
+                        if (ok && quad == 0 && lane == 0) ptx::tma_store_2d(&tmap_out, unit_n0(u), m0 + c * 16, dst);
+                        ++piece;
+                    }
+                }
+            } else if (ok && n < p.N) {
                 T* dst = out + (long long)m0 * p.N + n;
 #pragma unroll
                 for (int j = 0; j < CH * 16; ++j)
                     if (j < cols) dst[(long long)j * p.N] = round_out<T>(tot[j], bias, n);
             }
         }
+        if (quad == 0 && lane == 0) ptx::bulk_wait_all();
     }
 
     __syncwarp();
@@ -347,7 +386,7 @@ pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 }
 
 template <typename T, int KS>
-int launch_pair_t(const CUtensorMap& mw, const CUtensorMap& mx, const PairParams& p, int smem, cudaStream_t st) {
+int launch_pair_t(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mo, const PairParams& p, int smem, cudaStream_t st) {
     auto kern = pair_matmul_kernel<T, KS>;
     static bool attr_done[64] = {false};
     int dev = 0;
@@ -373,7 +412,7 @@ int launch_pair_t(const CUtensorMap& mw, const CUtensorMap& mx, const PairParams
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, kern, mw, mx, p);
+    cudaLaunchKernelEx(&cfg, kern, mw, mx, mo, p);
     return check_launch("matmul (tensor-core path, SM pairs)");
 }
 
@@ -394,16 +433,19 @@ int launch_pair_matmul(const void* x, int64_t x_ld, const void* w, int64_t w_ld,
     p.units = (int)units;
     p.x_bytes = bm / 2 * BLOCK_K * 2;                       // a multiple of 2 KB
     p.box3d = K % BLOCK_K == 0 ? 1 : 0;
-    const int limit = PAIR_SMEM_LIMIT - 1024 - PAIR_BAR_BYTES;
+    const int limit = PAIR_SMEM_LIMIT - 1024 - PAIR_BAR_BYTES - OUT_BYTES;
     const int ks = p.box3d ? 2 : 1;                         // two K steps per slot: half the handshakes (bm = 128: 349 -> 321 us); four measure the same
     const int slot_bytes = ks * (W_BYTES + p.x_bytes);
     const int fit = limit / slot_bytes;
     p.slots = fit < PAIR_MAX_SLOTS ? fit : PAIR_MAX_SLOTS;
-    const int smem = 1024 + PAIR_BAR_BYTES + p.slots * slot_bytes;
+    const int smem = 1024 + PAIR_BAR_BYTES + OUT_BYTES + p.slots * slot_bytes;
 
     const CUtensorMapDataType dt = dtype == BI_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    CUtensorMap mw, mx;
-    int rc;
+    CUtensorMap mw, mx, mo{};
+    int rc = BI_OK;
+    p.staged = N % 8 == 0 && aligned(out, 16) ? 1 : 0;
+    if (p.staged) rc = make_map(&mo, dt, 2, out, (uint64_t)N, (uint64_t)M, (uint64_t)N, BLOCK_N, OUT_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE);
+    if (rc) return rc;
     if (p.box3d) {
         rc = make_map3(&mx, dt, 2, x, (uint64_t)(K / BLOCK_K), (uint64_t)M, (uint64_t)x_ld, (uint32_t)(bm / 2), (uint32_t)ks);
         if (!rc) rc = make_map3(&mw, dt, 2, w, (uint64_t)(K / BLOCK_K), (uint64_t)N, (uint64_t)w_ld, BLOCK_N, (uint32_t)ks);
@@ -412,7 +454,7 @@ int launch_pair_matmul(const void* x, int64_t x_ld, const void* w, int64_t w_ld,
         if (!rc) rc = make_map(&mw, dt, 2, w, (uint64_t)K, (uint64_t)N, (uint64_t)w_ld, BLOCK_K, BLOCK_N, CU_TENSOR_MAP_SWIZZLE_128B);
     }
     if (rc) return rc;
-#define BI_PAIR_LAUNCH(TT) (ks == 2 ? launch_pair_t<TT, 2>(mw, mx, p, smem, st) : launch_pair_t<TT, 1>(mw, mx, p, smem, st))
+#define BI_PAIR_LAUNCH(TT) (ks == 2 ? launch_pair_t<TT, 2>(mw, mx, mo, p, smem, st) : launch_pair_t<TT, 1>(mw, mx, mo, p, smem, st))
     return dtype == BI_BF16 ? BI_PAIR_LAUNCH(__nv_bfloat16) : BI_PAIR_LAUNCH(__half);
 #undef BI_PAIR_LAUNCH
 }

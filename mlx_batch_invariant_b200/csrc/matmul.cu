@@ -43,28 +43,38 @@ TcShape tc_one_sm_shape(int64_t M, int64_t N, int64_t K, bool quant) {
 constexpr int64_t PAIR_QUANT_ELEMS = 128 << 20;      // largest quantized weight that is unpacked into the workspace (256 MB)
 
 // One SM or a pair of SMs per tile: the cheaper by what a K step of 64 was measured to take, in us, at the batch tile's
-// height (bm), times K steps, times waves of tiles, plus the launch. One SM: 0.17 + 0.0023 bm dense (N = 4096, K = 4096:
-// bm = 32 / 64 / 128 0.23 / 0.29 / 0.46), 0.28 + 0.0039 bm with packed weights, which it unpacks once per batch tile
-// (0.41 / 0.53 / 0.81). A pair: 0.29 + 0.0012 bm (bm = 96 / 128 / 256: 0.41 / 0.44 / 0.60) for 256 weight rows, and with
-// packed weights a pass that unpacks them first (0.45 us per million). The pair's taller tiles win from about 300 rows on;
-// where few tiles fill only part of a wave (small layers, short batches) one SM per tile keeps more SMs busy. Sizes
-// whose one-SM shape splits K keep it. Two limits, from runs over weights that are not in L2: up to 96 rows of a dense
-// batch the pair was nowhere faster (65 rows of 4096 -> 14336 / 28672: 38.9 / 70.7 against 31.7 / 55.3 us; 96 rows of
-// 14336 -> 4096: 88 against 78 us); and over a long K the packed one-SM kernel has a dearer start and cheaper steps, 10 us
-// and 0.27 + 0.003 bm (200 rows of 14336 -> 4096: 4 bits 113, 8 bits 105 us; pairs 114 and 116 us).
-constexpr int64_t PAIR_BM_MAX = 256, PAIR_BM_STEP = 32, PAIR_M_MIN = 97;
+// height (bm), times K steps, times waves of tiles, plus the launch; neither is faster than its weights come from HBM. Sizes
+// whose one-SM shape splits K keep it.
+// One SM: 0.17 + 0.0023 bm dense (N = 4096, K = 4096: bm = 32 / 64 / 128 0.23 / 0.29 / 0.46), 5.2 TB/s of weight beside more
+// than 32 rows (64 x 4096 -> 28672: 49.9 us; half of its ring holds batch rows). A pair: 0.12 + 0.0009 bm and no less than 0.2
+// (bm = 64 / 128 / 192 / 256: 0.20 / 0.22 / 0.29 / 0.35) for 256 weight rows, 6.2 TB/s, 8 us a launch. Weights that are not in
+// L2, one SM and pair: 64 / 128 rows of 4096 -> 28672 49.9 / 62.7 and 46.9 / 49.3 us, 64 of 4096 -> 14336 28.9 and 27.6, 128 of
+// 4096 -> 6144 24.6 and 20.5, 256 of 4096 -> 4096 23.1 and 20.7; 32 rows are the same, 16 of 4096 -> 28672 40 and 44.
+// Packed weights: the tile's height by the same steps; which batches take pairs at all by the sums below, 0.28 + 0.0039 bm a
+// step with one SM, which unpacks once per batch tile (0.41 / 0.53 / 0.81) -- over a long K it has a dearer start and
+// cheaper steps, 10 us and 0.27 + 0.003 bm (200 rows of 14336 -> 4096: 4 bits 113, 8 bits 105 us) -- and 0.29 + 0.0012 bm with a
+// pair behind the pass that unpacks (0.45 us per million), which is more than the pair's steps take now: batches of 97 to
+// 256 rows that this leaves on one SM would be up to 15 % faster, and every larger one is on pairs.
+constexpr int64_t PAIR_BM_MAX = 256, PAIR_BM_STEP = 32, PAIR_M_MIN = 33;
 TcShape tc_auto_shape(int64_t M, int64_t N, int64_t K, bool quant = false) {
     TcShape sh = tc_one_sm_shape(M, N, K, quant);
-    if (sh.split || M <= 64 || (quant ? N * K > PAIR_QUANT_ELEMS : M < PAIR_M_MIN)) return sh;
+    if (sh.split || (quant ? M <= 64 || N * K > PAIR_QUANT_ELEMS : M < PAIR_M_MIN)) return sh;
     const int64_t sms = sm_count(), pairs = sms / 2, steps = (K + 63) / 64;
     auto waves = [](int64_t units, int64_t slots) { return (double)((units + slots - 1) / slots); };
+    auto pair_steps = [&](int64_t bm) { return waves((N + 255) / 256 * ((M + bm - 1) / bm), pairs) * steps; };
     const double one_steps = waves((N + 127) / 128 * ((M + sh.bm - 1) / sh.bm), sms) * steps;
-    const double one = quant ? std::min(4.0 + one_steps * (0.28 + 0.0039 * sh.bm), 10.0 + one_steps * (0.27 + 0.003 * sh.bm))
-                             : 4.0 + one_steps * (0.17 + 0.0023 * sh.bm);
-    double best = 0.95 * one;
+    const double mbytes = 2e-6 * (double)(N * K);
+    bool pair = false;
+    if (quant) {
+        const double one = std::min(4.0 + one_steps * (0.28 + 0.0039 * sh.bm), 10.0 + one_steps * (0.27 + 0.003 * sh.bm));
+        for (int64_t bm = PAIR_BM_STEP; bm <= PAIR_BM_MAX; bm += PAIR_BM_STEP)
+            pair |= 7.0 + 0.225 * mbytes + pair_steps(bm) * (0.29 + 0.0012 * bm) < 0.95 * one;
+        if (!pair) return sh;
+    }
+    double best = quant ? 1e30 : 4.0 + std::max(one_steps * (0.17 + 0.0023 * sh.bm), mbytes / 5.2);
     for (int64_t bm = PAIR_BM_STEP; bm <= PAIR_BM_MAX; bm += PAIR_BM_STEP) {
-        const double cost = 5.0 + (quant ? 2.0 + 0.45e-6 * (double)(N * K) : 0.0) +
-                            waves((N + 255) / 256 * ((M + bm - 1) / bm), pairs) * steps * (0.29 + 0.0012 * bm);
+        const double compute = pair_steps(bm) * std::max(0.2, 0.12 + 0.0009 * bm);
+        const double cost = 8.0 + (quant ? compute : std::max(compute, mbytes / 6.2));
         if (cost < best) { best = cost; sh.pair = true; sh.bm = (int)bm; }
     }
     return sh;

@@ -61,6 +61,25 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const T* __restrict__ gu, T
     out[i] = Cvt<T>::down(swiglu_canon(g, u));
 }
 
+// The same with four 16-bit elements a thread, a block's threads inside one row: 8-byte loads, no 64-bit division. 64 x 14336 in
+// the decoder's step: 5.2 -> 3.9 us (eight a thread 4.3). A row alone has too few threads then: 1.8 us with an element a
+// thread, 2.0 with four; the line lies at the elements that give every SM a block.
+constexpr int64_t SWIGLU_VEC_MIN = 148 * 256 * 4;
+template <typename T>
+__global__ void __launch_bounds__(256) swiglu_vec_kernel(const uint2* __restrict__ gu, uint2* __restrict__ out, int pieces, int blocks_per_row) {
+    ptx::grid_dep_launch();
+    ptx::grid_dep_wait();
+    const int m = blockIdx.x / blocks_per_row, j = (blockIdx.x - m * blocks_per_row) * 256 + threadIdx.x;
+    if (j >= pieces) return;
+    const uint2 g = gu[(int64_t)m * 2 * pieces + j], u = gu[(int64_t)m * 2 * pieces + pieces + j];
+    uint2 o;
+    const T *gv = reinterpret_cast<const T*>(&g), *uv = reinterpret_cast<const T*>(&u);
+    T* ov = reinterpret_cast<T*>(&o);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ov[i] = Cvt<T>::down(swiglu_canon(Cvt<T>::up(gv[i]), Cvt<T>::up(uv[i])));
+    out[(int64_t)m * pieces + j] = o;
+}
+
 }  // namespace
 }  // namespace bi
 
@@ -93,6 +112,15 @@ extern "C" int bi_swiglu(const void* gate_up, void* out, int64_t M, int64_t F, i
     const int64_t blocks = (M * F + 255) / 256;
     if (blocks > 0x7fffffffLL) return fail(BI_ERR_UNSUPPORTED, "bi_swiglu: too large");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int64_t per_row = (F / 4 + 255) / 256;
+    if (dtype != BI_F32 && M * F >= SWIGLU_VEC_MIN && F % 4 == 0 && F < (1LL << 31) && M * per_row < (1LL << 31) && aligned(gate_up, 8) && aligned(out, 8)) {
+        const uint2* g = static_cast<const uint2*>(gate_up);
+        uint2* o = static_cast<uint2*>(out);
+        const dim3 grid((unsigned)(M * per_row));
+        if (dtype == BI_F16) launch_overlapped(swiglu_vec_kernel<__half>, grid, dim3(256), 0, st, g, o, (int)(F / 4), (int)per_row);
+        else launch_overlapped(swiglu_vec_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, g, o, (int)(F / 4), (int)per_row);
+        return check_launch("bi_swiglu");
+    }
     if (dtype == BI_F32) launch_overlapped(swiglu_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const float*>(gate_up), static_cast<float*>(out), M, F);
     else if (dtype == BI_F16) launch_overlapped(swiglu_kernel<__half>, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const __half*>(gate_up), static_cast<__half*>(out), M, F);
     else launch_overlapped(swiglu_kernel<__nv_bfloat16>, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(gate_up), static_cast<__nv_bfloat16*>(out), M, F);

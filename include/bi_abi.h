@@ -110,6 +110,10 @@ enum { BI_MATMUL_AUTO = 0, BI_MATMUL_SPLIT = 1, BI_MATMUL_FUSED = 2, BI_MATMUL_S
 #define BI_MATMUL_BATCH_TILE(n) ((n) << 16)
 #define BI_QMM_STAGE_SMEM 0x1000000
 #define BI_QMM_STAGE_TMEM 0x2000000
+/* The weight (codes, scales and biases with it) is not written by anything that is still running on the stream when the call is
+ * made, apart from kernels that a kernel of another library, a copy or a synchronisation has already waited for: the matmul may
+ * read it before the kernels in front of it have finished. Everything else it still reads and writes after them. */
+#define BI_MATMUL_STATIC_WEIGHT 0x4000000
 #define BI_MATMUL_COUNTER_BYTES 16384
 
 size_t bi_matmul_workspace_bytes(int64_t M, int64_t N, int64_t K, int dtype);

@@ -23,6 +23,7 @@ BI_F32, BI_F16, BI_BF16 = 0, 1, 2
 PATH_AUTO, PATH_SPLIT, PATH_FUSED, PATH_SPLIT_FOLD, PATH_PAIR = 0, 1, 2, 3, 4
 WS_ZEROED = 0x100                 # BI_MATMUL_WS_ZEROED
 QMM_STAGE_SMEM, QMM_STAGE_TMEM = 0x1000000, 0x2000000
+STATIC_WEIGHT = 0x4000000         # BI_MATMUL_STATIC_WEIGHT
 COUNTER_BYTES = 16384             # BI_MATMUL_COUNTER_BYTES
 
 

@@ -13,12 +13,10 @@ std::atomic<unsigned long long> g_launches{0};
 
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
-// Off unless BI_PDL=1: measured on the decoder step (418 kernels in one CUDA graph) it changed nothing for 16-bit
-// weights (6.07 against 6.04 ms) and cost 5 % with 4-bit weights (8.36 against 7.98 ms): inside a graph the gaps
-// between kernels are already short, and CTAs of the next kernel that sit resident take room from the running one.
-bool pdl_enabled() {
+// On for kernels of one GPU; those that shake hands with peers are launched the plain way. BI_PDL=0 / 1 switches all of them.
+bool pdl_enabled(bool peers) {
     const char* v = getenv("BI_PDL");      // read per launch: a test can switch it for one call
-    return v && v[0] == '1';
+    return v ? v[0] == '1' : !peers;
 }
 
 int fail(int code, const char* fmt, ...) {

@@ -949,8 +949,7 @@ __global__ void __launch_bounds__(256) decode_combine_kernel(const float* __rest
                                                              const int32_t* __restrict__ kv_lens, T* __restrict__ out,
                                                              int64_t BH, int Hq, int D, int L, int split, int nsplit,
                                                              PushSink sink) {
-    ptx::grid_dep_launch();   // the next kernel of the stream may start its set-up
-    ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
+    ptx::grid_dep_wait_and_launch();
     constexpr int AHEAD = 4;
     const int per_row = D / VEC, rows = 256 / per_row;               // threads of a row, rows of a block
     const int r0 = (int)threadIdx.x / per_row, d = ((int)threadIdx.x - r0 * per_row) * VEC;
@@ -1011,7 +1010,7 @@ int launch_decode_combine(const float* pm, const float* pl, const float* pacc, c
     const dim3 grid((unsigned)((BH + rows - 1) / rows)), block(256);
 #define BI_DECODE_COMBINE(VEC)                                                                                                          \
     do {                                                                                                                                \
-        if (sink) launch_overlapped(decode_combine_kernel<T, VEC, true>, grid, block, 0, st, pm, pl, pacc, kv_lens, (T*)nullptr, BH, Hq, D, L, split, nsplit, *sink); \
+        if (sink) launch_overlapped_unless(true, decode_combine_kernel<T, VEC, true>, grid, block, 0, st, pm, pl, pacc, kv_lens, (T*)nullptr, BH, Hq, D, L, split, nsplit, *sink); \
         else launch_overlapped(decode_combine_kernel<T, VEC, false>, grid, block, 0, st, pm, pl, pacc, kv_lens, static_cast<T*>(out), BH, Hq, D, L, split, nsplit, PushSink{}); \
     } while (0)
     if (wide) BI_DECODE_COMBINE(4); else BI_DECODE_COMBINE(1);

@@ -30,15 +30,18 @@ inline int fail_cuda(const char* what, cudaError_t e) {
     return fail(BI_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
-// Defined in abi.cu: whether kernels are launched with programmatic dependent launch (BI_PDL=1 turns it on).
-bool pdl_enabled();
+// Defined in abi.cu: whether a kernel is launched with programmatic dependent launch; `peers`: it waits for or signals
+// other ranks.
+bool pdl_enabled(bool peers = false);
 
 // Launch `kernel` so that it may begin (block scheduling, barrier and tensor-memory set-up) while the kernel before it
 // on the stream is still draining; the kernel itself waits (ptx::grid_dep_wait) before it touches global memory.
 // Every kernel launched through here MUST execute ptx::grid_dep_wait() in every CTA: completion of this kernel then
 // implies completion of everything before it, which is what the kernel after it relies on.
+// When the kernel after this one may begin is this kernel's to say (ptx::grid_dep_launch): short ones say so at once, matmuls
+// when their last loads are on their way -- CTAs that sit resident from the start took room from them.
 template <typename... KArgs, typename... Args>
-inline void launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+inline void launch_kernel(bool overlapped, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -48,8 +51,17 @@ inline void launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = overlapped ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);     // errors are picked up by check_launch()
+}
+template <typename... KArgs, typename... Args>
+inline void launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    launch_kernel(pdl_enabled(), kernel, grid, block, smem, st, static_cast<Args&&>(args)...);
+}
+// The same for kernels that take part in a handshake with other ranks where `peers` is set.
+template <typename... KArgs, typename... Args>
+inline void launch_overlapped_unless(bool peers, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    launch_kernel(pdl_enabled(peers), kernel, grid, block, smem, st, static_cast<Args&&>(args)...);
 }
 
 inline bool aligned(const void* p, size_t n) { return (reinterpret_cast<uintptr_t>(p) % n) == 0; }

@@ -67,8 +67,7 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const T* __restrict__ gu, T
 constexpr int64_t SWIGLU_VEC_MIN = 148 * 256 * 4;
 template <typename T>
 __global__ void __launch_bounds__(256) swiglu_vec_kernel(const uint2* __restrict__ gu, uint2* __restrict__ out, int pieces, int blocks_per_row) {
-    ptx::grid_dep_launch();
-    ptx::grid_dep_wait();
+    ptx::grid_dep_wait_and_launch();
     const int m = blockIdx.x / blocks_per_row, j = (blockIdx.x - m * blocks_per_row) * 256 + threadIdx.x;
     if (j >= pieces) return;
     const uint2 g = gu[(int64_t)m * 2 * pieces + j], u = gu[(int64_t)m * 2 * pieces + pieces + j];

@@ -26,7 +26,7 @@ int64_t ngroups(int64_t K) { return (K + GROUP_K - 1) / GROUP_K; }
 // they want every SM: with fewer weight tiles than SMs they split (the partials of <= 8 rows are tiny) -- 4096 ->
 // 14336 at M = 1: 26.4 us split over 148 CTAs against 27.5 us fused on 112.
 TcShape tc_one_sm_shape(int64_t M, int64_t N, int64_t K, bool quant) {
-    TcShape sh{false, 128, nullptr, TcShape::STAGE_AUTO, Await{nullptr, nullptr, 0, 0}, nullptr, false};
+    TcShape sh{false, 128, nullptr, TcShape::STAGE_AUTO, Await{nullptr, nullptr, 0, 0}, nullptr, false, false};
     const int64_t G = ngroups(K);
     const int64_t nt = (N + 127) / 128;
     if (quant && M <= 8 && G > 1 && nt < sm_count()) { sh.split = true; return sh; }
@@ -102,11 +102,13 @@ struct PathArg {
     bool zeroed;    // BI_MATMUL_WS_ZEROED
     int bm;         // 0 = choose
     int stage;      // TcShape::STAGE_*
+    bool static_w;  // BI_MATMUL_STATIC_WEIGHT
 };
 int parse_path(const char* op, int path, PathArg* pa) {
     pa->kind = path & 0xff;
     pa->zeroed = (path & BI_MATMUL_WS_ZEROED) != 0;
     pa->bm = (path >> 16) & 0xff;
+    pa->static_w = (path & BI_MATMUL_STATIC_WEIGHT) != 0;
     pa->stage = (path & BI_QMM_STAGE_SMEM) ? TcShape::STAGE_SMEM : ((path & BI_QMM_STAGE_TMEM) ? TcShape::STAGE_TMEM : TcShape::STAGE_AUTO);
     if (pa->kind > BI_MATMUL_PAIR) return fail(BI_ERR_BAD_ARG, "%s: unknown path %d", op, pa->kind);
     if (pa->kind == BI_MATMUL_PAIR) {
@@ -263,6 +265,7 @@ int matmul_impl(const void* a, const void* b, void* out, void* workspace, size_t
         if (rc) return rc;
         sh.await = aw;
         sh.bias = bias;
+        sh.static_w = pa.static_w;
         const int64_t w_ld = N == 1 ? K : b_sn;
         if (sh.pair) return launch_pair_matmul(a, x_ld, b, w_ld, out, M, N, K, dtype, sh, status, st);
         rc = launch_tc_matmul(a, x_ld, b, w_ld, nullptr, out, part, M, N, K, dtype, sh, status, st);
@@ -347,6 +350,7 @@ int qmm_impl(const void* x, const uint32_t* w, const void* scales, const void* b
             rc = launch_dequant(q, part, N, K, dtype, st);
             return rc ? rc : launch_pair_matmul(x, x_ld, part, K, out, M, N, K, dtype, sh, status, st);
         }
+        sh.static_w = pa.static_w;       // not for a pair: its weight is what launch_dequant has just written
         rc = launch_tc_matmul(x, x_ld, nullptr, 0, &q, out, part, M, N, K, dtype, sh, status, st);
         if (rc || !sh.split || sh.counters) return rc;
         if (rope) return launch_combine_rope(part, (int)ngroups(K), M * N, dtype, st, *rope);

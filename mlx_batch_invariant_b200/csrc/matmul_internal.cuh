@@ -76,6 +76,7 @@ struct TcShape {
     Await await;
     const void* bias;     // optional [N] bias in the output dtype, added after the output's rounding
     bool pair;
+    bool static_w;        // the weight (with its scales and biases) may be read before the kernels in front have finished
 };
 int launch_tc_matmul(const void* x, int64_t x_ld, const void* w, int64_t w_ld, const TcQuant* q, void* out,
                      float* part, int64_t M, int64_t N, int64_t K, int dtype, const TcShape& shape, int32_t* status,

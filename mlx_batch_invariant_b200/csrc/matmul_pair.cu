@@ -60,6 +60,7 @@ struct PairParams {
     int box3d;            // K % 64 == 0: the tensor maps are [K/64][rows][64] views (else 2-D, one K step per slot)
     int slots;            // ring depth
     int x_bytes;          // shared-memory bytes of a CTA's activation tile (bm / 2 rows of one K step)
+    int static_w;         // no kernel still in flight writes the weight: it is read before they are done
     int staged;           // the output goes through shared memory and TMA (rows of a multiple of 16 bytes)
 };
 
@@ -123,7 +124,6 @@ template <typename T, int KS>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                    const __grid_constant__ CUtensorMap tmap_out, const PairParams p) {
-    ptx::grid_dep_launch();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - ptx::smem_u32(smem_raw));
@@ -166,7 +166,7 @@ pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     __syncthreads();
     cluster_sync_all();                    // both CTAs' barriers exist before either signals the other's
     ptx::tc_fence_after();
-    ptx::grid_dep_wait();
+    if (!p.static_w) ptx::grid_dep_wait();
     const uint32_t tmem_base = 0;          // the whole of tensor memory was allocated: it starts at column 0
 
     const int n_clusters = (int)(gridDim.x >> 1), first = (int)(blockIdx.x >> 1);
@@ -206,27 +206,42 @@ pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         const uint32_t full0 = map_to_rank(bar_full(0), 0);
         int s = 0, filled = 0;
         uint32_t ph = 1;                                             // an untouched barrier passes the odd phase
+        auto load_w = [&](int sl, int n0, int k) {                   // all K steps of a slot in one box per operand
+            const uint32_t wt = smem_base + (uint32_t)(sl * KS) * W_BYTES, bar = full0 + 8u * (uint32_t)sl;
+            if (rank == 0) ptx::mbar_expect_tx(bar_full(sl), tx);
+            if (KS > 1 || p.box3d) tma_load_3d_pair(wt, &tmap_w, 0, n0, k >> 6, bar);
+            else tma_load_2d_pair(wt, &tmap_w, k, n0, bar);
+        };
+        auto load_x = [&](int sl, int m0, int k) {
+            const uint32_t xt = x_ring + (uint32_t)(sl * KS * p.x_bytes), bar = full0 + 8u * (uint32_t)sl;
+            if (KS > 1 || p.box3d) tma_load_3d_pair(xt, &tmap_x, 0, m0, k >> 6, bar);
+            else tma_load_2d_pair(xt, &tmap_x, k, m0, bar);
+        };
+        // The kernels in front may still be running: the slots of the first unit get their weights, then those kernels are
+        // waited for, and the loop below finds so many weights there.
+        int ahead = 0;
+        if (p.static_w) {
+            ahead = min(S, (p.K + KS * BLOCK_K - 1) / (KS * BLOCK_K));
+            if (ok && leader)
+                for (int i = 0; i < ahead; ++i) load_w(i, unit_n0(first), i * KS * BLOCK_K);
+            __syncwarp();
+            ptx::grid_dep_wait();
+        }
         for (int u = first; u < p.units; u += n_clusters) {
             const int n0 = unit_n0(u), m0 = unit_m0(u) + (int)rank * xh;
             for (int k = 0; k < p.K; k += KS * BLOCK_K) {
                 ok = ok && wait_bounded(bar_empty(s), ph, ctl, ROLE_TMA, 8 + s);
-                const uint32_t wt = smem_base + (uint32_t)(s * KS) * W_BYTES, xt = x_ring + (uint32_t)(s * KS * p.x_bytes);
-                const uint32_t bar = full0 + 8u * (uint32_t)s;
                 if (ok && leader) {
-                    if (rank == 0) ptx::mbar_expect_tx(bar_full(s), tx);
-                    if (KS > 1 || p.box3d) {                                   // all K steps of the slot in one box per operand
-                        tma_load_3d_pair(wt, &tmap_w, 0, n0, k >> 6, bar);
-                        tma_load_3d_pair(xt, &tmap_x, 0, m0, k >> 6, bar);
-                    } else {
-                        tma_load_2d_pair(wt, &tmap_w, k, n0, bar);
-                        tma_load_2d_pair(xt, &tmap_x, k, m0, bar);
-                    }
+                    if (ahead <= 0) load_w(s, n0, k);
+                    load_x(s, m0, k);
                 }
+                --ahead;
                 __syncwarp();
                 filled += ok ? 1 : 0;
                 if (++s == S) { s = 0; ph ^= 1u; }
             }
         }
+        ptx::grid_dep_launch();                                      // the last loads are on their way: the next kernel may start
         // Every slot's last use has to be over before this CTA may go away: the copies have landed (also after an
         // abort, when no MMA will read them) and no commit is still to arrive here.
         const int from = max(0, filled - S);
@@ -303,6 +318,7 @@ pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     } else if (warp >= EPI0) {
         // ------------------------------------------------------------ epilogue: totals in registers
         regs_inc<REGS_EPI>();
+        if (p.static_w) ptx::grid_dep_wait();                        // before the first store
         constexpr int CH = PAIR_MAX_BM / 2 / 16;                     // 16-column pieces of half a batch tile
         static_assert(CH % 4 == 0, "read in blocks of 32 columns, two at a time");
         const int quad = warp & 3, half = (warp - EPI0) >> 2;
@@ -411,7 +427,7 @@ int launch_pair_t(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMa
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    cfg.numAttrs = pdl_enabled(p.await.flags != nullptr) ? 2 : 1;
     cudaLaunchKernelEx(&cfg, kern, mw, mx, mo, p);
     return check_launch("matmul (tensor-core path, SM pairs)");
 }
@@ -426,6 +442,7 @@ int launch_pair_matmul(const void* x, int64_t x_ld, const void* w, int64_t w_ld,
     p.out = out; p.bias = shape.bias; p.status = status; p.await = shape.await;
     p.M = (int)M; p.N = (int)N; p.K = (int)K;
     p.G = (int)((K + GROUP_K - 1) / GROUP_K);
+    p.static_w = shape.static_w && !shape.await.flags ? 1 : 0;
     p.bm = bm;
     p.m_tiles = (int)((M + bm - 1) / bm);
     const int64_t units = (N + 2 * BLOCK_N - 1) / (2 * BLOCK_N) * p.m_tiles;

@@ -344,7 +344,7 @@ int combine_t(const float* part, void* out, int G, int64_t MN, cudaStream_t st, 
 #define BI_COMBINE(VEC, THREADS_)                                                                                        \
     do {                                                                                                                 \
         const unsigned blocks_ = (unsigned)(((THREADS_) + 255) / 256);                                                  \
-        if (sink) launch_overlapped(combine_kernel<T, VEC, true>, dim3(blocks_), dim3(256), 0, st, part, (T*)nullptr, G, MN, bias, N, *sink); \
+        if (sink) launch_overlapped_unless(true, combine_kernel<T, VEC, true>, dim3(blocks_), dim3(256), 0, st, part, (T*)nullptr, G, MN, bias, N, *sink); \
         else launch_overlapped(combine_kernel<T, VEC, false>, dim3(blocks_), dim3(256), 0, st, part, static_cast<T*>(out), G, MN, bias, N, none); \
     } while (0)
     if (vec_ok && MN >= (1 << 20)) {

@@ -118,6 +118,7 @@ struct Params {
     int uniform;        // every chunk is a whole K group (K % 256 == 0 and four K steps per chunk)
     int raw_span;       // quantized: bytes of one weight row in one box of packed codes (32, 64 or 128)
     int raw_boxes;      // quantized: boxes of packed codes per chunk (1 or 2)
+    int static_w;       // no kernel still in flight writes the weight (codes, scales, biases): it may be read before they are done
     int gs;
     long long units;
 };
@@ -240,7 +241,6 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                  const Params p) {
     using C = Cfg<QBITS, TSA>;
     static_assert(!TSA || QBITS != 0, "the tensor-memory weight operand exists for quantized weights only");
-    ptx::grid_dep_launch();   // the next kernel of the stream may start its set-up
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - ptx::smem_u32(smem_raw));
@@ -289,8 +289,8 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     __syncthreads();
     ptx::tc_fence_after();
     // Barriers, tensor memory and the tensor maps were set up while the kernel before this one was still draining;
-    // from here on global memory is touched.
-    ptx::grid_dep_wait();
+    // from here on global memory is touched -- the weight alone before that wait where nothing in flight writes it.
+    if (!p.static_w) ptx::grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_total = 2u * (uint32_t)p.acc_stride;
 
@@ -351,7 +351,15 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 }
             };
             ChunkIter it(p, ub, ue);
-            if (p.await.flags != nullptr && it.valid()) {
+            if (p.static_w) {
+                // The kernels in front may still be running: fill the ring with weights, then wait for them.
+                ChunkIter first(it);
+                int n = 0;
+                for (; it.valid() && n < LS; it.next(), ++n) issue_w(it);
+                ptx::grid_dep_wait();
+                for (int i = 0; i < n; ++i, first.next()) issue_x(first);
+                __syncwarp();
+            } else if (p.await.flags != nullptr && it.valid()) {
                 // The activation is still arriving from the other ranks. Fill the ring with weights first, then wait
                 // (bounded) for every peer's flag, then fetch the activation tiles of those chunks.
                 ChunkIter first(it);
@@ -384,6 +392,10 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 issue_x(it);
                 __syncwarp();
             }
+            // The last loads are on their way: the next kernel of the stream may start. Behind more rows its blocks are many
+            // and stand in the way of what is left here; the MMA warp lets them in (decoder step, 16-bit / 4-bit weights, from
+            // here and from there: one sequence 3556 / 3831 and 3600 / 3882 us, 16 sequences 4353 / 4647 and 4263 / 4619).
+            if (p.M <= 8) ptx::grid_dep_launch();
             if (!ok) {
                 // Let the copies already in flight land before the CTA goes away.
                 const int ci = it.ci;
@@ -514,8 +526,10 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             if (leader) ptx::umma_commit(bar_done(it.d));
             __syncwarp();
         }
+        ptx::grid_dep_launch();   // the last MMAs are on their way: the next kernel of the stream may start
     } else if (warp >= WARP_EPI0 && warp < WARP_EPI0 + 4) {
         // ------------------------------------------------------------ epilogue
+        if (p.static_w) ptx::grid_dep_wait();                        // before the first store
         const int quad = warp & 3;  // TMEM lanes this warp may touch: 32*quad .. 32*quad+31
         const int row = quad * 32 + lane;
         const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
@@ -904,7 +918,7 @@ int launch_t(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, cuda
     long long grid = p.units < sms ? p.units : sms;
     const long long waves = (p.units + sms - 1) / sms;
     if (waves >= 2 && waves <= 16) grid = (p.units + waves - 1) / waves;
-    launch_overlapped(kern, dim3((unsigned)grid), dim3(C::THREADS), p.smem_bytes, st, mw, mx, p);
+    launch_overlapped_unless(p.await.flags != nullptr, kern, dim3((unsigned)grid), dim3(C::THREADS), p.smem_bytes, st, mw, mx, p);
     return check_launch("matmul (tensor-core path)");
 }
 
@@ -935,6 +949,7 @@ int launch_tc_matmul(const void* x, int64_t x_ld, const void* w, int64_t w_ld, c
     Params p{};
     p.out = out; p.part = part; p.status = status;
     p.await = shape.await;
+    p.static_w = shape.static_w && !shape.await.flags ? 1 : 0;
     p.bias = shape.bias;
     p.counters = split ? shape.counters : nullptr;
     p.scales = quant ? q->scales : nullptr; p.biases = quant ? q->biases : nullptr;

@@ -142,7 +142,7 @@ extern "C" int bi_push_gather(const void* local, void* const* dst, void* const* 
     long long blocks = (total + 256 * 4 - 1) / (256 * 4);   // four 16-byte pieces per thread
     if (blocks > 128) blocks = 128;
     if (blocks < 1) blocks = 1;
-    launch_overlapped(push_gather_kernel, dim3((unsigned)blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+    launch_overlapped_unless(true, push_gather_kernel, dim3((unsigned)blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
         static_cast<const uint4*>(local), rows, (int)f16, rank, world, d, f, counters, status, wait);
     return check_launch("bi_push_gather");
 }
@@ -171,7 +171,7 @@ extern "C" int bi_push_gather_swiglu(const void* gate_up, void* const* dst, void
     if (blocks > 128) blocks = 128;
     if (blocks < 1) blocks = 1;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-#define BI_PGS(TT) launch_overlapped(push_gather_swiglu_kernel<TT>, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const TT*>(gate_up), rows, (int)F, rank, world, d, f, counters, status, wait)
+#define BI_PGS(TT) launch_overlapped_unless(true, push_gather_swiglu_kernel<TT>, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const TT*>(gate_up), rows, (int)F, rank, world, d, f, counters, status, wait)
     if (dtype == BI_F32) BI_PGS(float); else if (dtype == BI_F16) BI_PGS(__half); else BI_PGS(__nv_bfloat16);
 #undef BI_PGS
     return check_launch("bi_push_gather_swiglu");

@@ -62,8 +62,7 @@ struct NormAwait {
 template <typename T, bool STAGED, bool HAS_W, bool HAS_RES>
 __global__ void __launch_bounds__(TG) rms_norm_kernel(const T* x, const T* __restrict__ delta, const T* __restrict__ w,
                                                       T* sum_out, T* __restrict__ out, int D, float eps, NormAwait aw) {
-    ptx::grid_dep_launch();   // the next kernel of the stream may start its set-up
-    ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
+    ptx::grid_dep_wait_and_launch();
     extern __shared__ uint4 stage_raw[];
     __shared__ float red[TG];
     const int t = threadIdx.x;
@@ -448,7 +447,7 @@ int launch(const void* x, const void* delta, const void* w, void* sum_out, void*
                                                  (int)smem);                                        \
             if (e != cudaSuccess) return fail_cuda("rms_norm smem attr", e);                               \
         }                                                                                           \
-        launch_overlapped(kern, grid, block, smem, st, xp, dp, wp, sp, op, (int)D, eps, aw);                       \
+        launch_overlapped_unless(aw.flags != nullptr, kern, grid, block, smem, st, xp, dp, wp, sp, op, (int)D, eps, aw);                       \
     } while (0)
 #define BI_RMS_LAUNCH(ST, HW) do { if (delta) BI_RMS_LAUNCH2(ST, HW, true); else BI_RMS_LAUNCH2(ST, HW, false); } while (0)
     if (staged) { if (w) BI_RMS_LAUNCH(true, true); else BI_RMS_LAUNCH(true, false); }

@@ -45,7 +45,7 @@ def _weight_is_tensor_core(b: torch.Tensor, K: int) -> bool:
 
 
 def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None = None, awaiting=None, bias=None, push=None,
-                           rope=None):
+                           rope=None, static_weight: bool = False):
     """``a @ b`` with a batch-invariant reduction order.
 
     ``a`` may have extra leading dims (flattened into M); ``b`` must be 2-D (a transposed
@@ -62,6 +62,8 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
     ``rope`` (the arguments of ``bi_rope_append`` after ``qkv``, up to ``capacity``): the product is a decoder's qkv
     projection; the fold kernel rotates q and k and appends k and v to the cache itself (``bi_matmul_rope``);
     nothing is returned.
+    ``static_weight``: nothing that is still running on the stream writes ``b`` (a model's weights; not the result of the call
+    before): the kernel starts on it while the kernels in front of it finish (``BI_MATMUL_STATIC_WEIGHT``).
     """
     at, foreign = adopt(a)
     bt, _ = adopt(b)
@@ -80,6 +82,7 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
     a2 = at if at.ndim == 2 and K else at.reshape(-1, K)
     if a2.dtype != out_dtype:
         a2 = a2.to(out_dtype)
+    early = _lib.STATIC_WEIGHT if static_weight and bt.dtype == out_dtype else 0
     if bt.dtype != out_dtype:
         bt = bt.to(out_dtype)
     M = a2.shape[0]
@@ -94,7 +97,7 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
         with _lib.on_device(dev):
             word, ws, nbytes = _launch_shape("split", batch_tile, M, N, K, 0, dev)
             _lib.check(lib.bi_matmul_rope(a2.data_ptr(), bt.data_ptr(), _lib.ptr(ws), nbytes, M, N, K,
-                                          a2.stride(0) if M > 1 else K, a2.stride(1), bt.stride(0), bt.stride(1), code, word,
+                                          a2.stride(0) if M > 1 else K, a2.stride(1), bt.stride(0), bt.stride(1), code, word | early,
                                           _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev), *rope))
         return None
     if push is not None:
@@ -113,7 +116,7 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
         word, ws, nbytes = _launch_shape(path, batch_tile, M, N, K, calls.bi_matmul_scratch_bytes(M, N, K, code), dev)
         sm, sk = a2.stride()
         args = (a2.data_ptr(), bt.data_ptr(), out.data_ptr(), _lib.ptr(ws), nbytes, M, N, K, sm if M > 1 else K, sk, *bt.stride(), code,
-                word, _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev))
+                word | early, _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev))
         if bias is not None:
             bias_t = adopt(bias)[0]
             if bias_t.shape != (N,) or bias_t.dtype != out_dtype or not bias_t.is_cuda or awaiting is not None:

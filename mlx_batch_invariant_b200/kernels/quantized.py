@@ -43,10 +43,10 @@ _STAGES = {None: 0, "smem": _lib.QMM_STAGE_SMEM, "tmem": _lib.QMM_STAGE_TMEM}
 
 def batch_invariant_quantized_matmul(x, w, scales, biases, *, group_size: int, bits: int, path: str = "auto",
                                      batch_tile: int | None = None, stage: str | None = None, awaiting=None, push=None,
-                                     rope=None):
+                                     rope=None, static_weight: bool = False):
     """``x @ dequant(w).T``. ``path`` / ``batch_tile`` force a launch shape as for the dense matmul; ``stage``
     ("smem", "tmem") forces how the dequantized weight reaches the tensor core. All give the same bits.
-    ``awaiting`` / ``push`` / ``rope``: as for ``batch_invariant_matmul`` (``bi_qmm_awaiting`` / ``bi_qmm_push`` /
+    ``awaiting`` / ``push`` / ``rope`` / ``static_weight`` (of ``w``, ``scales`` and ``biases``): as for ``batch_invariant_matmul`` (``bi_qmm_awaiting`` / ``bi_qmm_push`` /
     ``bi_qmm_rope``)."""
     xt, foreign = adopt(x)
     wt, st, bt = adopt(w)[0], adopt(scales)[0], adopt(biases)[0]
@@ -64,9 +64,11 @@ def batch_invariant_quantized_matmul(x, w, scales, biases, *, group_size: int, b
     code = dtype_code(dt)
     x2 = rows_16b(xt if xt.ndim == 2 and K else xt.reshape(-1, K))
     M = x2.shape[0]
+    given = (wt, st, bt)
     st = st.to(dt).contiguous()
     bt = bt.to(dt).contiguous()
     wt = wt.contiguous()
+    early = _lib.STATIC_WEIGHT if static_weight and wt is given[0] and st is given[1] and bt is given[2] else 0      # none was just copied
     lib = _lib.load()
     if rope is not None:
         if push is not None or awaiting is not None or M == 0:
@@ -74,7 +76,7 @@ def batch_invariant_quantized_matmul(x, w, scales, biases, *, group_size: int, b
         with _lib.on_device(dev):
             word, ws, nbytes = _launch_shape("split", batch_tile, M, N, K, 0, dev)
             _lib.check(lib.bi_qmm_rope(x2.data_ptr(), wt.data_ptr(), st.data_ptr(), bt.data_ptr(), _lib.ptr(ws), nbytes, M, N, K,
-                                       x2.stride(0) if M > 1 else K, group_size, bits, code, word | _STAGES[stage],
+                                       x2.stride(0) if M > 1 else K, group_size, bits, code, word | early | _STAGES[stage],
                                        _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev), *rope))
         return None
     if push is not None:
@@ -94,6 +96,6 @@ def batch_invariant_quantized_matmul(x, w, scales, biases, *, group_size: int, b
                                        _lib.COUNTER_BYTES + 2 * N * K)
         args = (x2.data_ptr(), wt.data_ptr(), st.data_ptr(), bt.data_ptr(), out.data_ptr(),
                 _lib.ptr(ws), nbytes, M, N, K, x2.stride(0) if M > 1 else K, group_size, bits, code,
-                word | _STAGES[stage], _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev))
+                word | early | _STAGES[stage], _lib.status_word(dev).data_ptr(), _lib.stream_ptr(dev))
         _lib.check(calls.bi_qmm(*args) if awaiting is None else lib.bi_qmm_awaiting(*args, *awaiting))
     return give_back(out if xt.ndim == 2 else out.reshape(*lead, N), x, foreign)

@@ -101,18 +101,20 @@ class KernelBackend(TorchGlue):
                                          _lib.stream_ptr(gu.device)))
         return out
 
+    static_weights = True   # the linears can be told that their weight is at rest
+
     fused_rope = True       # the fold of the qkv projection can rotate and append itself (bi_matmul_rope / bi_qmm_rope)
 
-    def linear_rope(self, x, w, quant, cos, sin, pos0, B, T, hq, hkv, D, kc, vc):
+    def linear_rope(self, x, w, quant, cos, sin, pos0, B, T, hq, hkv, D, kc, vc, static_weight=False):
         """rope_append(linear(x, w)) in the matmul's own two launches: returns the rotated q [B, hq, T, D]."""
         q = torch.empty(B, hq, T, D, dtype=x.dtype, device=x.device)
         rope = (cos.data_ptr(), sin.data_ptr(), pos0.data_ptr(), q.data_ptr(), kc.data_ptr(), vc.data_ptr(), B, T, hq, hkv, D,
                 kc.stride(0), kc.stride(1), kc.stride(2), min(kc.shape[2], cos.shape[0]))
         if quant is None:
-            K.batch_invariant_matmul(x, w.T, rope=rope)
+            K.batch_invariant_matmul(x, w.T, rope=rope, static_weight=static_weight)
         else:
             p, s, b = w
-            K.batch_invariant_quantized_matmul(x, p, s, b, group_size=quant[1], bits=quant[0], rope=rope)
+            K.batch_invariant_quantized_matmul(x, p, s, b, group_size=quant[1], bits=quant[0], rope=rope, static_weight=static_weight)
         return q
 
     fused_wait = True       # the kernels can wait for a peer gather themselves (the *_awaiting entry points)
@@ -131,12 +133,12 @@ class KernelBackend(TorchGlue):
             _lib.check(_lib.load().bi_add_rms_norm_awaiting(*args, *awaiting, _lib.status_word(x.device).data_ptr()))
         return s, out
 
-    def linear(self, x, w, awaiting=None, push=None):       # x[M, K] @ W[N, K]^T
-        return K.batch_invariant_matmul(x, w.T, awaiting=awaiting, push=push)
+    def linear(self, x, w, awaiting=None, push=None, static_weight=False):       # x[M, K] @ W[N, K]^T
+        return K.batch_invariant_matmul(x, w.T, awaiting=awaiting, push=push, static_weight=static_weight)
 
-    def qlinear(self, x, packed, group_size, bits, awaiting=None, push=None):
+    def qlinear(self, x, packed, group_size, bits, awaiting=None, push=None, static_weight=False):
         p, s, b = packed
-        return K.batch_invariant_quantized_matmul(x, p, s, b, group_size=group_size, bits=bits, awaiting=awaiting, push=push)
+        return K.batch_invariant_quantized_matmul(x, p, s, b, group_size=group_size, bits=bits, awaiting=awaiting, push=push, static_weight=static_weight)
 
     def rms_norm(self, x, w, eps):
         return K.batch_invariant_rms_norm(x, w, eps)
@@ -237,8 +239,13 @@ class ShardedDecoder:
             return self.ops.add_rms_norm(x, delta, w, self.cfg.eps)
         return self.ops.add_rms_norm(x, delta, w, self.cfg.eps, awaiting=awaiting)
 
+    def _static(self):
+        """The decoder's weights are at rest: between whatever wrote them last and the first linear of a pass stands the
+        embedding lookup, a kernel of another library, which is launched behind them and which the first norm waits for."""
+        return {"static_weight": True} if getattr(self.ops, "static_weights", False) else {}
+
     def _lin(self, x, w, awaiting=None):
-        kw = {} if awaiting is None else {"awaiting": awaiting}
+        kw = self._static() if awaiting is None else {"awaiting": awaiting}
         if self.quant is None:
             return self.ops.linear(x, w, **kw)
         return self.ops.qlinear(x, w, self.quant[1], self.quant[0], **kw)
@@ -284,7 +291,7 @@ class ShardedDecoder:
                  and ((Kdim + 255) // 256) * M * n * 4 <= PUSH_PARTIALS_MAX and vc.stride() == kc.stride()
                  and 256 % D == 0)
         if fused:
-            return self.ops.linear_rope(h, w, self.quant, self.cos, self.sin, pos0, B, T, self.hq, self.hkv, D, kc, vc)
+            return self.ops.linear_rope(h, w, self.quant, self.cos, self.sin, pos0, B, T, self.hq, self.hkv, D, kc, vc, **self._static())
         return self.ops.rope_append(self._lin(h, w), self.cos, self.sin, pos0, B, T, self.hq, self.hkv, D, kc, vc)
 
     def _fused_push(self) -> bool:

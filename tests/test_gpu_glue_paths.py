@@ -32,7 +32,7 @@ def test_split_merge(B, Hq, D, L):
     lib = _lib.load()
     nbytes = lib.bi_attn_decode_workspace_bytes(B, Hq, L, D, 256)
     ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device="cuda")
-    for shift in (0, 1):                                                    # an output that is not aligned for four
+    for shift in (0, D // 32):                    # elements: for 32 and 64 dims an output that is not aligned for four
         out = torch.empty(shift + q.numel(), device="cuda")[shift:]
         _lib.check(lib.bi_attn_decode(qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), lc.data_ptr(), ws.data_ptr(), nbytes, B, Hq, Hq, L, D,
                                       Hq * L * D, L * D, D, D ** -0.5, 256, _lib.BI_F32, _lib.stream_ptr(qc.device)))

@@ -1,0 +1,48 @@
+"""Matmuls that start on a weight at rest while the kernels in front of them still run: the bits of plain launches, eagerly and
+from a graph, for every kernel and ring (rings deeper than K, several tiles a CTA, K that ends inside a step)."""
+
+import pytest
+import torch
+
+import mlx_batch_invariant_b200 as bi
+from mlx_batch_invariant_b200 import _lib
+from mlx_batch_invariant_b200.runner.decoder import quantize_rows
+
+pytestmark = pytest.mark.gpu
+
+
+def weights(dims, packed):
+    g = torch.Generator(device="cuda").manual_seed(sum(dims))
+    ws = [(torch.randn(n, k, device="cuda", generator=g) * k ** -0.5).bfloat16() for k, n in zip(dims, dims[1:])]
+    return [quantize_rows(w, 64, packed) for w in ws] if packed else ws
+
+
+def chain(x, ws, packed, path, static):
+    """Linear, norm, linear, norm, ...: every matmul follows a kernel that writes its activation."""
+    for w in ws:
+        h = bi.batch_invariant_rms_norm(x, None, 1e-5)
+        if packed:
+            x = bi.batch_invariant_quantized_matmul(h, *w, group_size=64, bits=packed, path=path, static_weight=static)
+        else:
+            x = bi.batch_invariant_matmul(h, w.T, path=path, static_weight=static)
+    return x
+
+
+@pytest.mark.parametrize("M,path", [(1, "auto"), (1, "fused"), (16, "auto"), (64, "split"), (64, "fused"), (70, "pair"), (300, "auto")])
+@pytest.mark.parametrize("dims,packed", [((256, 4096, 320, 22000, 512), 0), ((1000, 136, 2056, 1000), 0), ((256, 4096, 320, 22016, 512), 4), ((512, 2048, 512), 8)])
+def test_bits_of_plain_launches(M, path, dims, packed, monkeypatch):
+    ws = weights(dims, packed)
+    x = torch.randn(M, dims[0], device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).bfloat16()
+    monkeypatch.setenv("BI_PDL", "0")
+    want = chain(x, ws, packed, path, False)
+    monkeypatch.delenv("BI_PDL")
+    for _ in range(3):
+        assert torch.equal(chain(x, ws, packed, path, True), want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(x, ws, packed, path, True)
+    for _ in range(3):
+        got.zero_()
+        graph.replay()
+        assert torch.equal(got, want)
+    _lib.check_device_status()

@@ -52,7 +52,7 @@ __device__ __forceinline__ float div_canon(float a, float b) { return __fdiv_rn(
 __device__ __forceinline__ float swiglu_canon(float g, float u) {
     const float e = expf_canon(-fabsf(g));
     const float den = add_rn(1.0f, e);
-    const float sig = g >= 0.0f ? div_canon(1.0f, den) : div_canon(e, den);
+    const float sig = div_canon(g >= 0.0f ? 1.0f : e, den);      // the numerator is selected: of two divisions a warp would do both (1024 x 14336: 40.7 -> 33.5 us)
     return mul_rn(mul_rn(g, sig), u);
 }
 

@@ -37,3 +37,19 @@ def test_split_merge(B, Hq, D, L):
         _lib.check(lib.bi_attn_decode(qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), lc.data_ptr(), ws.data_ptr(), nbytes, B, Hq, Hq, L, D,
                                       Hq * L * D, L * D, D, D ** -0.5, 256, _lib.BI_F32, _lib.stream_ptr(qc.device)))
         assert R.bits_of(out.view_as(qc)) == R.bits_of(ref)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,hq,hkv,D", [(1, 1, 2, 1, 16), (2, 37, 14, 2, 64), (1, 300, 32, 8, 128), (3, 5, 3, 1, 96)])      # a head a thread ... blocks that a token does not fill
+def test_rope_by_quads_of_pieces_has_the_bits_of_elements(B, T, hq, hkv, D, dtype):
+    g = torch.Generator(device="cuda").manual_seed(T)
+    cap, pos0 = T + 3, torch.tensor([2], dtype=torch.long, device="cuda")
+    qkv = torch.randn(B * T, (hq + 2 * hkv) * D, device="cuda", generator=g).to(dtype)
+    cos, sin = (torch.randn(cap, D, device="cuda", generator=g) for _ in range(2))
+    shifted = torch.empty(qkv.numel() + 1, device="cuda", dtype=dtype)[1:].view_as(qkv).copy_(qkv)        # not aligned: an element a thread
+    got = []
+    for x in (qkv, shifted):
+        kc, vc = (torch.full((B + 1, hkv, cap, D), 7.0, device="cuda", dtype=dtype) for _ in range(2))
+        got.append((KernelBackend().rope_append(x, cos, sin, pos0, B, T, hq, hkv, D, kc, vc), kc, vc))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    _lib.check_device_status()

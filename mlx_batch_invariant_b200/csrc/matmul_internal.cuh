@@ -76,6 +76,8 @@ struct TcShape {
     Await await;
     const void* bias;     // optional [N] bias in the output dtype, added after the output's rounding
     bool pair;
+    int per_tile, first_run;   // split: CTAs of a tile and the groups the first of them folds itself (0: equal shares of all units, no run);
+                               // the fold then starts at partial first_run - 1
     bool static_w;        // the weight (with its scales and biases) may be read before the kernels in front have finished
 };
 int launch_tc_matmul(const void* x, int64_t x_ld, const void* w, int64_t w_ld, const TcQuant* q, void* out,

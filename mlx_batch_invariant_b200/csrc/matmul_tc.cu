@@ -40,6 +40,10 @@
 //     never crosses shared memory and needs no proxy fence. Its arithmetic is
 //     packed 16-bit fma where that gives the same bits (dequant_exact).
 //
+// The split path deals the K groups of a long dense tile to a few CTAs of its own (Params::per_tile); the first of them folds
+// its groups as they come and stores one total in the place of the last one's partial: the partials are bytes beside the
+// weight's (64 rows of 14336 -> 4096: 59 MB beside 117, 30.7 us with their stores and 22.9 without).
+//
 // The split path can fold in the producing kernel: a CTA that has stored its
 // group partial bumps a per-tile counter, and the CTA that arrives last reads
 // the G partials of the tile back in ascending g and writes T(total) -- the adds
@@ -105,6 +109,8 @@ struct Params {
     int n_tiles, m_tiles;
     int bm;             // batch rows per tile: 16, 32, 64 or 128 (launch shape; an output column's bits do not depend on it)
     int split;          // 1: split jobs, 0: fused units
+    int per_tile;       // split, dense: CTAs of a tile, which share its K groups; 0: the units are dealt in equal contiguous shares
+    int first_run;      // with per_tile: the groups of a tile's first CTA, which stores only their total, in the place of the last one's partial
     int x_rows;         // rows of the activation TMA box
     int box3d;          // 1: one TMA box holds a whole chunk (all K steps of a slot) of an operand
     int smem_bytes;     // dynamic shared memory of the launch
@@ -129,7 +135,18 @@ struct Params {
 // shared-memory budget allows), and everyone who needs "the MMAs of chunk c are done" -- the TMA
 // thread before it refills a slot, the dequantizers before they overwrite a weight slot, the
 // epilogue before it reads an accumulator -- waits on the same barrier done[c % 8].
-struct ChunkIter {
+// What of the kernel a launch needs. A decoder's step goes through some 390 kernels, and each begins with its instructions in
+// no cache: code that a launch does not reach still lies between what it does, and the registers of the widest loop are
+// everyone's (168; now 45 - 112). Decoder step, one kernel for all -> one for each: 64 / 16 / 1 sequences 5539 / 4308 / 3559 ->
+// 5383 / 4067 / 3514 us, 4-bit weights 7115 / 4645 / 3830 -> 6392 / 4349 / 3567. ANY decides at run time: the in-kernel fold, and
+// packed weights of more than 64 rows.
+enum { SHAPE_ANY, SHAPE_FUSED, SHAPE_SPLIT, SHAPE_RUNS };
+enum { ROWS_ANY, ROWS_FEW, ROWS_MANY };      // FEW: every tile has at most 8 batch rows; MANY: up to 8 are treated like more
+template <int SHAPE> __device__ __forceinline__ bool is_split(const Params& p) { return SHAPE == SHAPE_ANY ? p.split != 0 : SHAPE != SHAPE_FUSED; }
+template <int ROWS> __device__ __forceinline__ bool few_rows(int ncols) { return ROWS == ROWS_ANY ? ncols <= 8 : ROWS == ROWS_FEW; }
+
+template <int SHAPE>
+struct ChunkIterT {
     // Enumerates (unit, group, chunk) in the one order every role follows, and keeps the ring
     // positions of the current chunk. Only the constructor divides; stepping is increments.
     const Params& p;
@@ -140,12 +157,12 @@ struct ChunkIter {
     int ci;                   // CTA-local running chunk index
     int l, w, d;              // load slot, weight slot, completion barrier of the chunk
     uint32_t lph, wph, dph;   // phase parities of those rings
-    __device__ __forceinline__ ChunkIter(const Params& pp, int ub, int ue) : p(pp), left(ue - ub) {
+    __device__ __forceinline__ ChunkIterT(const Params& pp, int ub, int ue) : p(pp), left(ue - ub) {
         ci = 0; l = w = d = 0; lph = wph = dph = 0;
         nt = mt = g = g1 = nst = c = nchunk = 0;
         if (left <= 0) return;
         int tile;
-        if (p.split) { tile = ub / p.G; g = ub - tile * p.G; g1 = g + 1; }
+        if (is_split<SHAPE>(p)) { tile = ub / p.G; g = ub - tile * p.G; g1 = g + 1; }
         else         { tile = ub; g = 0; g1 = p.G; }
         nt = tile / p.m_tiles; mt = tile - nt * p.m_tiles;
         start_group();
@@ -176,13 +193,13 @@ struct ChunkIter {
         const int c1 = c + 1, gn = g + 1, mt1 = mt + 1;
         const bool stay = c1 < nchunk;                              // next chunk of the same K group
         const bool unit_end = !stay && gn >= g1;                    // else: next group of the same unit
-        const bool tile_adv = unit_end && (!p.split || gn == p.G);  // a split unit is one (tile, group)
+        const bool tile_adv = unit_end && (!is_split<SHAPE>(p) || gn == p.G);  // a split unit is one (tile, group)
         const bool mwrap = mt1 == p.m_tiles;
         left -= unit_end ? 1 : 0;
         mt = tile_adv ? (mwrap ? 0 : mt1) : mt;
         nt += (tile_adv && mwrap) ? 1 : 0;
         g = stay ? g : (tile_adv ? 0 : gn);
-        g1 = (unit_end && p.split) ? g + 1 : g1;
+        g1 = (unit_end && is_split<SHAPE>(p)) ? g + 1 : g1;
         const int kw = min(p.K - g * GROUP_K, GROUP_K);
         const int nst_n = (kw + BLOCK_K - 1) >> 6;
         static_assert(BLOCK_K == 64, "shift above");
@@ -235,11 +252,13 @@ __device__ __forceinline__ void dequant_row64_to_tmem(const uint8_t* raw, int ro
     }
 }
 
-template <typename T, int QBITS, bool TSA>
+template <typename T, int QBITS, bool TSA, int SHAPE, int ROWS>
 __global__ void __launch_bounds__((Cfg<QBITS, TSA>::THREADS), 1)
 tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                  const Params p) {
     using C = Cfg<QBITS, TSA>;
+    using ChunkIter = ChunkIterT<SHAPE>;
+    const bool split = is_split<SHAPE>(p);
     static_assert(!TSA || QBITS != 0, "the tensor-memory weight operand exists for quantized weights only");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -294,8 +313,16 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_total = 2u * (uint32_t)p.acc_stride;
 
-    const int ub = (int)(p.units * blockIdx.x / gridDim.x);
-    const int ue = (int)(p.units * (blockIdx.x + 1) / gridDim.x);
+    int ub = (int)(p.units * blockIdx.x / gridDim.x);
+    int ue = (int)(p.units * (blockIdx.x + 1) / gridDim.x);
+    bool run_cta = false;                                            // this CTA folds its groups as they come
+    if (SHAPE == SHAPE_RUNS) {
+        const int tile = (int)blockIdx.x / p.per_tile, j = (int)blockIdx.x - tile * p.per_tile;
+        auto start = [&](int i) { return i ? p.first_run + (p.G - p.first_run) * (i - 1) / (p.per_tile - 1) : 0; };
+        ub = tile * p.G + start(j);
+        ue = tile * p.G + start(j + 1);
+        run_cta = j == 0;
+    }
     // wait until the MMAs of chunk `ci` (CTA-local running index) have completed
     auto wait_done = [&](int ci, int role) {   // MAX_SLOTS is a power of two: mask and shift, no division
         return wait_bounded(bar_done(ci & (MAX_SLOTS - 1)), (uint32_t)(ci >> 3) & 1u, ctl, role, 16 + (ci & (MAX_SLOTS - 1)));
@@ -428,7 +455,7 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         uint32_t tmem_d = tmem_base;
         if (p.uniform) {
             // Every chunk is one whole K group with its own accumulator: nothing to enumerate but ring positions.
-            const int nch = (ue - ub) * (p.split ? 1 : p.G);
+            const int nch = (ue - ub) * (split ? 1 : p.G);
             int l = 0, w = 0, d = 0;
             uint32_t lph = 0, wph = 0;
             const int wring = QBITS ? WS : LS;
@@ -543,6 +570,45 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             epi_ph ^= 1u;
             return r;
         };
+        if (SHAPE == SHAPE_RUNS && run_cta) {
+            // The groups of a tile's first run: their total in registers (the tile has at most 64 batch rows), stored as the last
+            // group's partial. A loop of its own: beside the one below the compiler gave that one slower stores.
+            constexpr int RUN_ROWS = SHAPE == SHAPE_RUNS ? 64 : 1;
+            float total[RUN_ROWS];
+#pragma unroll
+            for (int j = 0; j < RUN_ROWS; ++j) total[j] = 0.0f;
+            ChunkIter it(p, ub, ue);
+            const int n = it.n0() + row, m0 = it.m0(), ncols = min(p.bm, p.M - m0);
+            for (; it.valid() && ok; it.next()) {
+                if (it.first_in_group()) ++job;
+                if (!it.last_in_group()) continue;
+                const int buf = job & 1;
+                if (!wait_bounded(bar_done(it.d), it.dph, ctl, ROLE_EPI, 16 + it.d)) { ok = false; break; }
+                ptx::tc_fence_after();
+                const uint32_t acc = lane_base + (uint32_t)(buf * p.acc_stride);
+                uint32_t v0[32], v1[32];
+                const bool two = ncols > 32;
+                ptx::tmem_ld_32x32(acc, v0);
+                if (two) ptx::tmem_ld_32x32(acc + 32, v1);
+                ptx::tmem_ld_wait();
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar_tempty(buf));
+#pragma unroll
+                for (int j = 0; j < 32; ++j) total[j % RUN_ROWS] = add_rn(total[j % RUN_ROWS], __uint_as_float(v0[j]));
+                if (two) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) total[(32 + j) % RUN_ROWS] = add_rn(total[(32 + j) % RUN_ROWS], __uint_as_float(v1[j]));
+                }
+            }
+            if (ok && n < p.N) {
+                float* dst = p.part + ((long long)(p.first_run - 1) * p.M + m0) * p.N + n;
+#pragma unroll
+                for (int j = 0; j < RUN_ROWS; ++j)
+                    if (j < ncols) dst[(long long)j * p.N] = total[j];
+            }
+            ue = ub;                                                 // nothing is left for the loop below
+        }
         T* out = static_cast<T*>(p.out);
         const T* bias = static_cast<const T*>(p.bias);
         float small_total[8];                                        // running totals of a tile of at most 8 batch rows (fused)
@@ -560,7 +626,8 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             const int ncols = min(p.bm, p.M - m0);
             const uint32_t acc = lane_base + (uint32_t)(buf * p.acc_stride);
             const bool first = g == 0, last = g == p.G - 1;
-            if (ncols <= 8) {
+            const bool few = few_rows<ROWS>(ncols);
+            if (few) {
                 // Few batch rows (decode): a narrow accumulator read, and in the fused shape the running totals
                 // stay in registers from group to group -- no round trip through tensor memory.
                 {
@@ -571,7 +638,7 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                     ptx::tc_fence_before();
                     __syncwarp();
                     if (lane == 0) ptx::mbar_arrive(bar_tempty(buf));          // the accumulator is in registers
-                    if (p.split) {
+                    if (split) {
                         if (n < p.N) {
                             float* dst = p.part + ((long long)g * p.M + m0) * p.N + n;
 #pragma unroll
@@ -588,7 +655,7 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                         }
                     }
                 }
-            } else if (p.split) {
+            } else if (split) {
                 // A TMEM load queues behind the MMAs already issued for the next unit, so the loads of two
                 // column blocks go out together and pay that wait once (the streaming variant, short of
                 // registers with its sixteen dequantizer warps, takes one block at a time).
@@ -621,7 +688,7 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                     }
                 }
             }
-            if (p.split && p.counters) {
+            if (SHAPE == SHAPE_ANY && split && p.counters) {
                 // In-kernel fold. Every thread's partial stores are fenced device-wide, the four warps meet,
                 // one thread counts this unit in; the CTA that counts in last (all G partials of the tile are
                 // then visible) folds them in ascending g and writes the output. The counter goes back to 0.
@@ -663,7 +730,7 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             // (16 in the streaming variant, which is short of registers).
             constexpr int EW = TSA ? 16 : 32;
 #pragma unroll 1
-            for (int c = 0; !p.split && ncols > 8 && c * EW < ncols; ++c) {  // warp-uniform trip count
+            for (int c = 0; !split && !few && c * EW < ncols; ++c) {  // warp-uniform trip count
                 uint32_t v[EW], t[EW];
                 if constexpr (TSA) {
                     ptx::tmem_ld_32x16(acc + c * EW, v);
@@ -689,7 +756,7 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                     else ptx::tmem_st_32x32(lane_base + tmem_total + c * EW, t);
                 }
             }
-            if (!p.split && ncols > 8) {
+            if (!split && !few) {
                 if (!last) ptx::tmem_st_wait();
                 ptx::tc_fence_before();
                 __syncwarp();
@@ -898,10 +965,10 @@ bool pick_rings(Params& p, int raw_bytes, bool tsa) {
     return true;
 }
 
-template <typename T, int QBITS, bool TSA>
-int launch_t(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, cudaStream_t st) {
+template <typename T, int QBITS, bool TSA, int SHAPE, int ROWS>
+int launch_v(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, cudaStream_t st) {
     using C = Cfg<QBITS, TSA>;
-    auto kern = tc_matmul_kernel<T, QBITS, TSA>;
+    auto kern = tc_matmul_kernel<T, QBITS, TSA, SHAPE, ROWS>;
     static bool attr_done[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -918,8 +985,20 @@ int launch_t(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, cuda
     long long grid = p.units < sms ? p.units : sms;
     const long long waves = (p.units + sms - 1) / sms;
     if (waves >= 2 && waves <= 16) grid = (p.units + waves - 1) / waves;
+    if (p.per_tile) grid = p.units / p.G * p.per_tile;
     launch_overlapped_unless(p.await.flags != nullptr, kern, dim3((unsigned)grid), dim3(C::THREADS), p.smem_bytes, st, mw, mx, p);
     return check_launch("matmul (tensor-core path)");
+}
+
+template <typename T, int QBITS, bool TSA>
+int launch_t(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, cudaStream_t st) {
+    if constexpr (QBITS != 0 && !TSA) return launch_v<T, QBITS, TSA, SHAPE_ANY, ROWS_ANY>(mw, mx, p, st);
+    if (p.counters) return launch_v<T, QBITS, TSA, SHAPE_ANY, ROWS_ANY>(mw, mx, p, st);
+    if constexpr (QBITS == 0) {
+        if (p.per_tile) return launch_v<T, QBITS, TSA, SHAPE_RUNS, ROWS_MANY>(mw, mx, p, st);
+    }
+    if (p.M <= 8) return p.split ? launch_v<T, QBITS, TSA, SHAPE_SPLIT, ROWS_FEW>(mw, mx, p, st) : launch_v<T, QBITS, TSA, SHAPE_FUSED, ROWS_FEW>(mw, mx, p, st);
+    return p.split ? launch_v<T, QBITS, TSA, SHAPE_SPLIT, ROWS_MANY>(mw, mx, p, st) : launch_v<T, QBITS, TSA, SHAPE_FUSED, ROWS_MANY>(mw, mx, p, st);
 }
 
 }  // namespace
@@ -959,6 +1038,8 @@ int launch_tc_matmul(const void* x, int64_t x_ld, const void* w, int64_t w_ld, c
     p.n_tiles = (int)((N + BLOCK_N - 1) / BLOCK_N);
     p.m_tiles = (int)((M + bm - 1) / bm);
     p.split = split ? 1 : 0;
+    p.per_tile = split && !quant ? shape.per_tile : 0;
+    p.first_run = shape.first_run;
     p.gs = quant ? q->gs : 0;
     p.units = (long long)p.n_tiles * p.m_tiles * (split ? p.G : 1);
     if (p.units >= (1LL << 31)) return fail(BI_ERR_UNSUPPORTED, "matmul: %lld work units exceed the kernel's 32-bit unit index", p.units);

@@ -241,8 +241,9 @@ class ShardedDecoder:
 
     def _static(self):
         """The decoder's weights are at rest: between whatever wrote them last and the first linear of a pass stands the
-        embedding lookup, a kernel of another library, which is launched behind them and which the first norm waits for."""
-        return {"static_weight": True} if getattr(self.ops, "static_weights", False) else {}
+        embedding lookup, a kernel of another library, which is launched behind them and which the first norm waits for. A
+        block hook may put work of its own between two blocks."""
+        return {"static_weight": True} if getattr(self.ops, "static_weights", False) and self.block_hook is None else {}
 
     def _lin(self, x, w, awaiting=None):
         kw = self._static() if awaiting is None else {"awaiting": awaiting}

@@ -46,3 +46,42 @@ def test_bits_of_plain_launches(M, path, dims, packed, monkeypatch):
         graph.replay()
         assert torch.equal(got, want)
     _lib.check_device_status()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_behind_copies_memsets_and_joined_streams(captured):
+    """What stands in front of an overlapped launch need not be a kernel, nor on its stream."""
+    w = weights((512, 4096, 512), 0)
+    src = torch.randn(16, 512, device="cuda").bfloat16()
+    want = bi.batch_invariant_matmul(bi.batch_invariant_matmul(src, w[0].T), w[1].T)
+    x, side = torch.empty_like(src), torch.cuda.Stream()
+
+    def work():
+        outs = []
+        x.copy_(src)                                                       # a copy
+        outs.append(bi.batch_invariant_matmul(bi.batch_invariant_matmul(x, w[0].T, static_weight=True), w[1].T))
+        x.zero_()                                                          # a memset
+        outs.append(bi.batch_invariant_matmul(x, w[0].T))
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):                                      # a kernel of the library and a copy on another stream
+            y = bi.batch_invariant_matmul(src, w[0].T)
+            x.copy_(src)
+        z = bi.batch_invariant_rms_norm(src, None, 1e-5)
+        torch.cuda.current_stream().wait_stream(side)
+        outs += [bi.batch_invariant_matmul(y, w[1].T, static_weight=True), bi.batch_invariant_matmul(bi.batch_invariant_matmul(x, w[0].T), w[1].T), z]
+        return outs
+
+    torch.cuda.synchronize()
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            outs = work()
+        for o in outs:
+            o.fill_(7.0)
+        graph.replay()
+    else:
+        outs = work()
+    torch.cuda.synchronize()
+    a, zero, b, c, z = outs
+    assert torch.equal(a, want) and torch.equal(b, want) and torch.equal(c, want) and not zero.any()
+    assert torch.equal(z, bi.batch_invariant_rms_norm(src, None, 1e-5))

@@ -704,8 +704,7 @@ struct KLItems {
     __device__ __forceinline__ int group(int i) const {    // of item `i` of nall
         return __ffs(__ballot_sync(0xffffffffu, i < nfull ? i < full : i - nfull < part)) - 1;
     }
-    __device__ __forceinline__ void look_ahead(int i) { if (B > 32) len = fetch(group(i)); }
-    __device__ __forceinline__ KLItems(const int32_t* lens, int B_, int L_, int split_, int per_seq_, long long item)
+    __device__ __forceinline__ KLItems(const int32_t* lens, int B_, int L_, int split_, int per_seq_)
         : kv_lens(lens), B(B_), L(L_), split(split_), per_seq(per_seq_), full(0), part(0), len(0) {
         const int lane = threadIdx.x & 31;
         nfull = nall = 0;
@@ -725,15 +724,15 @@ struct KLItems {
             }
         }
         nall += nfull;
-        if (item < nall) look_ahead((int)item);
     }
     // item `i` of nall, the one asked for in the call before (or at the start): sequence, split, index among the split's
     // per_seq items, keys. `next` is what the next call asks for.
-    __device__ __forceinline__ void find(int i, long long next, int& b, int& sp, int& sub, int& nk) {
+    __device__ __forceinline__ void find(int i, int& b, int& sp, int& sub, int& nk) {
         const bool ph = i >= nfull;
         int g = 0, r = i - (ph ? nfull : 0);
         if (B > 32) {
             g = group(i);
+            len = fetch(g);
             const int before = __shfl_sync(0xffffffffu, ph ? part : full, max(g - 1, 0));
             r -= g ? before : 0;
         }
@@ -746,7 +745,6 @@ struct KLItems {
         sp = ph ? n / split : rel / per_seq;
         sub = ph ? rel : rel - sp * per_seq;
         nk = ph ? n - sp * split : split;
-        if (next < nall) look_ahead((int)next);
     }
 };
 
@@ -777,18 +775,45 @@ __global__ void __launch_bounds__(32 * NW, 1) decode_keylane_kernel(
     // either way; its warps then take neighbours, the kv heads of one sequence (64 x 4096 keys 250.8 us, 253.2 apart).
     const bool apart = DEAL != KL_ALL || L % split != 0;
     long long item = apart ? (long long)wid * gridDim.x + blockIdx.x : (long long)blockIdx.x * NW + wid;
-    KLItems work(kv_lens, DEAL == KL_LISTED ? B : 0, L, split, Hkv * nchunk, item);
+    // (behind the warps' buffers: 16 bytes of static shared memory in front of them cost the main loop 15 %)
+    int* const taken = reinterpret_cast<int*>(dec_smem + NW * C::WARP_BYTES);
+    if (threadIdx.x == 0) *taken = 0;
+    __syncthreads();
+    KLItems work(kv_lens, DEAL == KL_LISTED ? B : 0, L, split, Hkv * nchunk);
     // all of the listed items full splits: as many warps as for that capacity (8 x 8192 keys 84 us with eight, 82 with seven
     // of them)
     const int warps = DEAL == KL_LISTED && NW == KL_WARPS && work.nall == work.nfull ? kl_warps(work.nall, gridDim.x) : NW;
     if (DEAL == KL_LISTED && wid >= warps) return;
     const long long stride = (long long)gridDim.x * warps;
-    for (;; item += stride) {
+    // A CTA's first items and its full splits go round its warps. Where the short ones fit beside the last round of full splits,
+    // or are as many as the warps, the others of them go to whichever warp is done: one that has no full split left takes
+    // several while the others are at theirs (64 x 561 keys 46.5 -> 43.5 us with their lengths, 96 x up to 600 53.6 -> 47.4, 1024 x
+    // up to 300 210 -> 196, 200 x 600 128 -> 120). Round otherwise, because neighbours are on different schedulers: with the full
+    // splits, too, for whoever is done the last of them meet on one, 96 x 600 keys 67 -> 73 us; so do a few more short ones than
+    // fit, 64 x 640 50 -> 55. (An item has partials in the workspace: their number is an int.)
+    const int ctas = (int)gridDim.x, first = (int)blockIdx.x;
+    const int nfull = DEAL == KL_LISTED ? work.nfull : (int)per_split * (L / split);
+    const int nshort = DEAL == KL_LISTED ? work.nall - work.nfull : (L % split ? (int)per_split : 0);
+    const int mine = nfull > first ? (nfull - first + ctas - 1) / ctas : 0;                                 // full splits of this CTA
+    bool whoever = apart && DEAL != KL_CAPACITY;
+    if (NH > 1 && whoever) {             // a head a warp: few items, and the sums below would cost them 0.7 us
+        // keys of all short ones; of sequences with lengths the first 32 stand for all
+        const long long rest = DEAL == KL_LISTED ? (long long)__reduce_add_sync(0xffffffffu, work.len % split) * (Hkv * nchunk) * ((B + 31) / 32) : per_split * (L % split);
+        whoever = nshort >= warps * ctas || rest <= (long long)((warps - mine % warps) % warps * ctas) * split;
+    }
+    auto following = [&](long long i) {
+        if (!whoever || i + stride < nfull) return i + stride;
+        int t = 0;
+        if (lane == 0) t = atomicAdd(taken, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        return (long long)(max(mine, warps) + t) * ctas + first;
+    };
+    for (;; item = following(item)) {
         int b, sp, hk, chunk, nk;                                            // warp-uniform
         if (DEAL == KL_LISTED) {
             if (item >= work.nall) break;
             int sub;
-            work.find((int)item, item + stride, b, sp, sub, nk);
+            work.find((int)item, b, sp, sub, nk);
             hk = sub / nchunk;
             chunk = sub - hk * nchunk;
         } else {
@@ -874,25 +899,42 @@ __global__ void __launch_bounds__(32 * NW, 1) decode_keylane_kernel(
             kl_node<T, NH, 1, 0>(kcur + lane * C::KPITCH, qs, dd);
             uint8_t* const cps = C::CP_IN_KBUF ? kcur : cps_own;
             if (C::CP_IN_KBUF) __syncwarp();                                 // every lane has read its K row: the buffer is free
-            // ---- softmax scalars of the block
+            // ---- softmax scalars of the block, the heads' chains side by side
+            float sc[NH], before[NH];
+            bool rise = false;
 #pragma unroll
             for (int h = 0; h < NH; ++h) {
                 float d0, d1;
                 ptx::unpack2(dd[h], d0, d1);
-                const float s = add_rn(d0, d1);
-                float x = valid ? s : -INFINITY;                              // inclusive prefix maximum over the lanes
+                sc[h] = add_rn(d0, d1);
+                before[h] = m[h];                                             // running maximum before this key
+                rise |= valid && sc[h] > m[h];
+            }
+            if (__any_sync(0xffffffffu, rise)) {                              // else no key of the block moves a maximum
+                float x[NH];                                                  // inclusive prefix maxima over the lanes
+#pragma unroll
+                for (int h = 0; h < NH; ++h) x[h] = valid ? sc[h] : -INFINITY;
 #pragma unroll
                 for (int off = 1; off < 32; off <<= 1) {
-                    const float y = __shfl_up_sync(0xffffffffu, x, off);
-                    if (lane >= off) x = fmaxf(x, y);
+                    float y[NH];
+#pragma unroll
+                    for (int h = 0; h < NH; ++h) y[h] = __shfl_up_sync(0xffffffffu, x[h], off);
+#pragma unroll
+                    for (int h = 0; h < NH; ++h) if (lane >= off) x[h] = fmaxf(x[h], y[h]);
                 }
-                float before = __shfl_up_sync(0xffffffffu, x, 1);
-                before = fmaxf(m[h], lane == 0 ? -INFINITY : before);         // running maximum before this key
-                const float e = expf_canon(-fabsf(sub_rn(s, before)));
-                const bool rises = s >= before;
+#pragma unroll
+                for (int h = 0; h < NH; ++h) {
+                    const float up = __shfl_up_sync(0xffffffffu, x[h], 1);
+                    before[h] = fmaxf(m[h], lane == 0 ? -INFINITY : up);
+                    m[h] = fmaxf(m[h], __shfl_sync(0xffffffffu, x[h], 31));
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+                const float e = expf_canon(-fabsf(sub_rn(sc[h], before[h])));
+                const bool rises = sc[h] >= before[h];
                 const float corr = rises ? e : 1.0f, p = rises ? 1.0f : e;
                 *reinterpret_cast<float4*>(cps + (lane * NH + h) * 16) = make_float4(corr, corr, p, p);
-                m[h] = fmaxf(m[h], __shfl_sync(0xffffffffu, x, 31));
             }
             if (KL_KBUFS == 2) {
                 asm volatile("cp.async.wait_group 0;" ::: "memory");        // V rows (and the next K rows) have landed
@@ -1068,7 +1110,10 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
                 // 229), up to the lanes that hold the counts. How many items there are is known on the device only: the launch
                 // has eight warps a CTA unless seven hold all that the capacity can.
                 const bool listed = kv_lens && nsplit > 1 && B <= KL_LISTED_MAX;
-                const int nw = listed ? (items > sms * (KL_WARPS - 1) ? KL_WARPS : KL_WARPS - 1) : kl_warps(items, sms);
+                // Without lengths eight as well where seven hold the full splits and the eighth the short ones.
+                const int64_t one = items / nsplit, rest = L % split;
+                const bool eighth = rest && items > sms * (KL_WARPS - 1) && one * (nsplit - 1) <= sms * (KL_WARPS - 1) && one * rest <= sms * split;
+                const int nw = listed ? (items > sms * (KL_WARPS - 1) ? KL_WARPS : KL_WARPS - 1) : (eighth ? KL_WARPS : kl_warps(items, sms));
                 const int64_t ctas = std::min<int64_t>(sms, (items + nw - 1) / nw);
 #define BI_KL_LAUNCH(NHV, NWV, DEALV)                                                                                         \
     do {                                                                                                                \
@@ -1078,11 +1123,11 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
         cudaGetDevice(&dev_);                                                                                           \
         if (dev_ < 0 || dev_ >= 64) dev_ = 0;                                                                           \
         if (!attr_set[dev_]) {                                                                                          \
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (NWV) * KLCfg::WARP_BYTES); \
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (NWV) * KLCfg::WARP_BYTES + 16); \
             if (e != cudaSuccess) return fail_cuda("bi_attn_decode smem attr", e);      \
             attr_set[dev_] = true;                                                                                      \
         }                                                                                                               \
-        launch_overlapped(kern, dim3((unsigned)ctas), dim3(32 * (NWV)), (size_t)((NWV) * KLCfg::WARP_BYTES), st, qp, kp, vp, kv_lens, pm, pl, pacc, \
+        launch_overlapped(kern, dim3((unsigned)ctas), dim3(32 * (NWV)), (size_t)((NWV) * KLCfg::WARP_BYTES + 16), st, qp, kp, vp, kv_lens, pm, pl, pacc, \
                           (int)B, (int)Hq, (int)Hkv, (int)L, lay, scale, split, nsplit, nck);                           \
     } while (0)
 #define BI_KL_LAUNCH_NH(NWV, DEALV) do { if (nh == 4) BI_KL_LAUNCH(4, NWV, DEALV); else if (nh == 2) BI_KL_LAUNCH(2, NWV, DEALV); else BI_KL_LAUNCH(1, NWV, DEALV); } while (0)

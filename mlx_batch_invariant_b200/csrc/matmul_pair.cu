@@ -61,7 +61,6 @@ struct PairParams {
     int slots;            // ring depth
     int x_bytes;          // shared-memory bytes of a CTA's activation tile (bm / 2 rows of one K step)
     int static_w;         // no kernel still in flight writes the weight: it is read before they are done
-    int staged;           // the output goes through shared memory and TMA (rows of a multiple of 16 bytes)
 };
 
 __device__ __forceinline__ uint32_t cta_rank() {
@@ -120,7 +119,7 @@ __device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0,
 template <int R> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 template <int R> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
 
-template <typename T, int KS>
+template <typename T, int KS, bool STAGED>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                    const __grid_constant__ CUtensorMap tmap_out, const PairParams p) {
@@ -364,7 +363,7 @@ pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 if (lane == 0) arrive_cluster(buf ? tempty1 : tempty0);
             }
             const int n = unit_n0(u) + quad * 32 + lane;
-            if (p.staged) {
+            if (STAGED) {                                            // outputs whose rows are whole 16-byte units: through shared memory and TMA
                 const T* b = n < p.N ? bias : nullptr;
 #pragma unroll
                 for (int c = 0; c < CH; ++c) {
@@ -401,9 +400,9 @@ pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     }
 }
 
-template <typename T, int KS>
+template <typename T, int KS, bool STAGED>
 int launch_pair_t(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mo, const PairParams& p, int smem, cudaStream_t st) {
-    auto kern = pair_matmul_kernel<T, KS>;
+    auto kern = pair_matmul_kernel<T, KS, STAGED>;
     static bool attr_done[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -460,8 +459,8 @@ int launch_pair_matmul(const void* x, int64_t x_ld, const void* w, int64_t w_ld,
     const CUtensorMapDataType dt = dtype == BI_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     CUtensorMap mw, mx, mo{};
     int rc = BI_OK;
-    p.staged = N % 8 == 0 && aligned(out, 16) ? 1 : 0;
-    if (p.staged) rc = make_map(&mo, dt, 2, out, (uint64_t)N, (uint64_t)M, (uint64_t)N, BLOCK_N, OUT_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE);
+    const bool staged = N % 8 == 0 && aligned(out, 16);
+    if (staged) rc = make_map(&mo, dt, 2, out, (uint64_t)N, (uint64_t)M, (uint64_t)N, BLOCK_N, OUT_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
     if (p.box3d) {
         rc = make_map3(&mx, dt, 2, x, (uint64_t)(K / BLOCK_K), (uint64_t)M, (uint64_t)x_ld, (uint32_t)(bm / 2), (uint32_t)ks);
@@ -471,8 +470,10 @@ int launch_pair_matmul(const void* x, int64_t x_ld, const void* w, int64_t w_ld,
         if (!rc) rc = make_map(&mw, dt, 2, w, (uint64_t)K, (uint64_t)N, (uint64_t)w_ld, BLOCK_K, BLOCK_N, CU_TENSOR_MAP_SWIZZLE_128B);
     }
     if (rc) return rc;
-#define BI_PAIR_LAUNCH(TT) (ks == 2 ? launch_pair_t<TT, 2>(mw, mx, mo, p, smem, st) : launch_pair_t<TT, 1>(mw, mx, mo, p, smem, st))
+#define BI_PAIR_LAUNCH_KS(TT, STAGED) (ks == 2 ? launch_pair_t<TT, 2, STAGED>(mw, mx, mo, p, smem, st) : launch_pair_t<TT, 1, STAGED>(mw, mx, mo, p, smem, st))
+#define BI_PAIR_LAUNCH(TT) (staged ? BI_PAIR_LAUNCH_KS(TT, true) : BI_PAIR_LAUNCH_KS(TT, false))
     return dtype == BI_BF16 ? BI_PAIR_LAUNCH(__nv_bfloat16) : BI_PAIR_LAUNCH(__half);
+#undef BI_PAIR_LAUNCH_KS
 #undef BI_PAIR_LAUNCH
 }
 

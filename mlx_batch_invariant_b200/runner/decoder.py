@@ -45,6 +45,7 @@ class DecoderConfig:
 LLAMA3_8B = DecoderConfig()
 
 PUSH_TESTED_WORLDS = (2, 4, 8)  # world sizes at which the peer-memory all-gather has run on hardware
+FUSED_ROPE_ROWS = 64            # the qkv projection folds with its rotation up to here: beyond, the split it forces is dearer than a launch (300 rows: 75 us against 35)
 PUSH_PARTIALS_MAX = 256 << 20   # a matmul pushes its own output only while its split partials stay below this many bytes
 
 
@@ -289,7 +290,7 @@ class ShardedDecoder:
         fused = (getattr(self.ops, "fused_rope", False) and self.dt != torch.float32
                  and os.environ.get("BI_FUSED_ROPE", "1") != "0"
                  and Kdim % (64 if self.quant is not None else 8) == 0
-                 and ((Kdim + 255) // 256) * M * n * 4 <= PUSH_PARTIALS_MAX and vc.stride() == kc.stride()
+                 and M <= FUSED_ROPE_ROWS and ((Kdim + 255) // 256) * M * n * 4 <= PUSH_PARTIALS_MAX and vc.stride() == kc.stride()
                  and 256 % D == 0)
         if fused:
             return self.ops.linear_rope(h, w, self.quant, self.cos, self.sin, pos0, B, T, self.hq, self.hkv, D, kc, vc, **self._static())

@@ -399,10 +399,10 @@ int launch_layer_norm(const void* x, const void* w, const void* b, void* out, in
     const T* bp = static_cast<const T*>(b);
     T* op = static_cast<T*>(out);
     dim3 grid((unsigned)rows), block(TG);
-    if (w && b) layer_norm_kernel<T, true, true><<<grid, block, 0, st>>>(xp, wp, bp, op, (int)D, eps);
-    else if (w) layer_norm_kernel<T, true, false><<<grid, block, 0, st>>>(xp, wp, bp, op, (int)D, eps);
-    else if (b) layer_norm_kernel<T, false, true><<<grid, block, 0, st>>>(xp, wp, bp, op, (int)D, eps);
-    else layer_norm_kernel<T, false, false><<<grid, block, 0, st>>>(xp, wp, bp, op, (int)D, eps);
+    if (w && b) launch_overlapped(layer_norm_kernel<T, true, true>, grid, block, 0, st, xp, wp, bp, op, (int)D, eps);
+    else if (w) launch_overlapped(layer_norm_kernel<T, true, false>, grid, block, 0, st, xp, wp, bp, op, (int)D, eps);
+    else if (b) launch_overlapped(layer_norm_kernel<T, false, true>, grid, block, 0, st, xp, wp, bp, op, (int)D, eps);
+    else launch_overlapped(layer_norm_kernel<T, false, false>, grid, block, 0, st, xp, wp, bp, op, (int)D, eps);
     return check_launch("bi_layer_norm");
 }
 

@@ -63,8 +63,9 @@ constexpr int64_t PAIR_QUANT_ELEMS = 128 << 20;      // largest quantized weight
 // Packed weights: the tile's height by the same steps; which batches take pairs at all by the sums below, 0.28 + 0.0039 bm a
 // step with one SM, which unpacks once per batch tile (0.41 / 0.53 / 0.81) -- over a long K it has a dearer start and
 // cheaper steps, 10 us and 0.27 + 0.003 bm (200 rows of 14336 -> 4096: 4 bits 113, 8 bits 105 us) -- and 0.29 + 0.0012 bm with a
-// pair behind the pass that unpacks (0.45 us per million), which is more than the pair's steps take now: batches of 97 to
-// 256 rows that this leaves on one SM would be up to 15 % faster, and every larger one is on pairs.
+// pair behind the pass that unpacks (0.45 us per million), which is more than the pair's steps take now. Where that line is
+// early, 200 and 256 rows of 4096 -> 4096 take 28.4 us on one SM and would take 24.3 on pairs; elsewhere the two are within 7 %
+// on both sides of it (128 rows of 4096 -> 14336 55.4 and 51.7, 200 of 14336 -> 4096 75.2 and 73.5, 4-bit weights).
 constexpr int64_t PAIR_BM_MAX = 256, PAIR_BM_STEP = 32, PAIR_M_MIN = 33;
 TcShape tc_auto_shape(int64_t M, int64_t N, int64_t K, bool quant = false) {
     TcShape sh = tc_one_sm_shape(M, N, K, quant);

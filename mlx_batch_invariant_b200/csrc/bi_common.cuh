@@ -40,6 +40,7 @@ bool pdl_enabled(bool peers = false);
 // implies completion of everything before it, which is what the kernel after it relies on.
 // When the kernel after this one may begin is this kernel's to say (ptx::grid_dep_launch): short ones say so at once, matmuls
 // when their last loads are on their way -- CTAs that sit resident from the start took room from them.
+// Kernels that need an even spread of a few CTAs over the SMs are launched plainly (matmul_simt.cu).
 template <typename... KArgs, typename... Args>
 inline void launch_kernel(bool overlapped, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
     cudaLaunchConfig_t cfg = {};

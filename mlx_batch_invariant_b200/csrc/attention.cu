@@ -122,8 +122,6 @@ __global__ void __launch_bounds__(128) decode_kernel(const T* __restrict__ q, co
                                                      float* __restrict__ pm, float* __restrict__ pl,
                                                      float* __restrict__ pacc, int B, int Hq, int Hkv, int L,
                                                      KvLayout lay, float scale, int split, int nsplit, int nchunk) {
-    ptx::grid_dep_launch();   // the next kernel of the stream may start its set-up
-    ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
     constexpr int D = 32 * DL;
     constexpr int NL = NCHUNK * DL;
     const int lane = threadIdx.x & 31;
@@ -263,8 +261,6 @@ __global__ void __launch_bounds__(32 * DEC2_WARPS) decode_stream_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const int32_t* __restrict__ kv_lens,
     float* __restrict__ pm, float* __restrict__ pl, float* __restrict__ pacc, int B, int Hq, int Hkv, int L,
     KvLayout lay, float scale, int split, int nsplit, int nchunk) {
-    ptx::grid_dep_launch();   // the next kernel of the stream may start its set-up
-    ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
     using C = Dec2Cfg<T, DL>;
     constexpr int D = 32 * DL;
     constexpr int SEGS = C::ROWB / 16;                 // 16-byte segments per row
@@ -460,8 +456,6 @@ __global__ void __launch_bounds__(32 * MAXW) decode_warp_stream_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const int32_t* __restrict__ kv_lens,
     float* __restrict__ pm, float* __restrict__ pl, float* __restrict__ pacc, int B, int Hq, int Hkv, int L,
     KvLayout lay, float scale, int split, int nsplit, int nchunk) {
-    ptx::grid_dep_launch();   // the next kernel of the stream may start its set-up
-    ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
     using C = DecWCfg<T, DL>;
     constexpr int D = 32 * DL;
     constexpr int SEGS = C::ROWB / 16;
@@ -753,7 +747,9 @@ __global__ void __launch_bounds__(32 * NW, 1) decode_keylane_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const int32_t* __restrict__ kv_lens,
     float* __restrict__ pm, float* __restrict__ pl, float* __restrict__ pacc, int B, int Hq, int Hkv, int L,
     KvLayout lay, float scale, int split, int nsplit, int nchunk) {
-    ptx::grid_dep_launch();   // the next kernel of the stream may start its set-up
+    // The merge behind this kernel has little to set up; its blocks beside the last items cost 8 x 8192 keys 72.9 -> 78.9 us. A few
+    // CTAs leave room for it: decoder step of 4 sequences 3552 -> 3522 us.
+    if (gridDim.x < 64) ptx::grid_dep_launch();
     ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
     using C = KLCfg;
     constexpr int D = 128;
@@ -1089,6 +1085,8 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
     const T* kp = static_cast<const T*>(k);
     const T* vp = static_cast<const T*>(v);
     dim3 grid((unsigned)blocks), block(32 * warps);
+    // The octet-lane kernels below are launched plainly: several CTAs an SM, less than a wave of them as a rule, which must be
+    // spread evenly (64 x 561 keys of 14 / 2 heads of 64 in a chain of calls: 36 us so, 52 let in beside the merge in front).
     // Streamed kernel when every K/V row starts on a 16-byte boundary (cp.async granularity);
     // otherwise the register-prefetch kernel. Same arithmetic, the choice depends on layout only.
     if constexpr (DL < 8) {
@@ -1179,7 +1177,7 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
             if (e != cudaSuccess) return fail_cuda("bi_attn_decode smem attr", e);      \
             attr_set[dev_] = true;                                                                                      \
         }                                                                                                               \
-        launch_overlapped(kern, dim3((unsigned)blocksw), dim3(32 * wpc), smem_w, st, qp, kp, vp, kv_lens, pm, pl, pacc, (int)B, (int)Hq, (int)Hkv, \
+        launch_kernel(false, kern, dim3((unsigned)blocksw), dim3(32 * wpc), smem_w, st, qp, kp, vp, kv_lens, pm, pl, pacc, (int)B, (int)Hq, (int)Hkv, \
                                                           (int)L, lay, scale, split, nsplit, nchunk4);                  \
     } while (0)
             if (wpc <= 4) BI_DECW_LAUNCH(4);
@@ -1201,7 +1199,7 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES); \
             if (e != cudaSuccess) return fail_cuda("bi_attn_decode smem attr", e); \
         }                                                                                                        \
-        launch_overlapped(kern, dim3((unsigned)blocks2), dim3(32 * DEC2_WARPS), C::SMEM_BYTES, st, qp, kp, vp, kv_lens, pm, pl, pacc, (int)B, \
+        launch_kernel(false, kern, dim3((unsigned)blocks2), dim3(32 * DEC2_WARPS), C::SMEM_BYTES, st, qp, kp, vp, kv_lens, pm, pl, pacc, (int)B, \
                                                                           (int)Hq, (int)Hkv, (int)L, lay, scale, split, nsplit, nchunk); \
     } while (0)
             if (GU == 4) BI_DECODE2_LAUNCH(4); else if (GU == 2) BI_DECODE2_LAUNCH(2); else BI_DECODE2_LAUNCH(1);
@@ -1215,7 +1213,7 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
     if (lay.table != nullptr)
         return fail(BI_ERR_UNSUPPORTED, "bi_attn_decode_paged: paged caches are read by the 16-bit head_dim-128 kernel only");
 #define BI_DECODE_LAUNCH(GUV)                                                                              \
-    launch_overlapped(decode_kernel<T, DL, GUV>, grid, block, 0, st, qp, kp, vp, kv_lens, pm, pl, pacc, (int)B, (int)Hq, \
+    launch_kernel(false, decode_kernel<T, DL, GUV>, grid, block, 0, st, qp, kp, vp, kv_lens, pm, pl, pacc, (int)B, (int)Hq, \
                                                       (int)Hkv, (int)L, lay, scale, split, nsplit, nchunk)
     if (GU == 4) {
         if constexpr (DL < 8) BI_DECODE_LAUNCH(4);

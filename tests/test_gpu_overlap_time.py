@@ -32,6 +32,16 @@ def _behind_another_linear(M, K, N):
     return lambda: (other(), call())
 
 
+def _decode(B, L, dtype, heads=14, kv_heads=2, dim=64):
+    q, k, v = _rand(B, heads, 1, dim, dtype=dtype), *(_rand(B, kv_heads, L, dim, dtype=dtype) for _ in range(2))
+    return lambda: bi.batch_invariant_decode_attention(q, k, v, scale=dim ** -0.5)
+
+
+def _decode_behind_a_linear():
+    x, w, attend = _rand(64, 896, dtype=torch.bfloat16), _rand(896, 896, dtype=torch.bfloat16).T, _decode(64, 561, torch.bfloat16)
+    return lambda: (bi.batch_invariant_matmul(bi.batch_invariant_rms_norm(x, None, 1e-5), w), attend())
+
+
 CHAINS = {
     "fp32 few rows": lambda: _linear(2, 2048, 2048),
     "fp32 9 x 4096 -> 4096": lambda: _linear(9, 4096, 4096),
@@ -41,6 +51,9 @@ CHAINS = {
     "fp32 behind a 16-bit linear": lambda: _behind_another_linear(64, 2048, 2048),
     "bf16 in element-wise fetches": lambda: _linear(16, 4092, 4096, torch.bfloat16),
     "bf16 norm and row-major linear": lambda: _norm_linears(16, torch.bfloat16, True),
+    "bf16 decode attention": lambda: _decode(64, 561, torch.bfloat16),
+    "fp32 decode attention": lambda: _decode(64, 561, torch.float32),
+    "bf16 decode attention behind a linear": _decode_behind_a_linear,
 }
 
 

@@ -244,7 +244,6 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
     float* const ms = reinterpret_cast<float*>(sm + C::MOFF);
     int* const ns = reinterpret_cast<int*>(sm + C::NOFF);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
 
     const RowBlock block(B, Hkv, G, Tq, QB);
     const long long R = block.R, r0 = block.r0;
@@ -481,7 +480,10 @@ int launch_prefill_tq(const void* q, const void* k, const void* v, void* out, in
         if (e != cudaSuccess) return fail_cuda("bi_attn_prefill smem attr", e);
         attr_set[dev] = true;
     }
-    launch_overlapped(kern, dim3((unsigned)blocks), dim3(PF_THREADS), C::SMEM, st,
+    // Plainly: two or three CTAs an SM, which lie unevenly when they are let in beside a running kernel, for long prompts too, whose
+    // blocks differ in keys. Linear and attention of 512 tokens, 32 / 8 heads of 128: 143 us so, 119 plainly (and 1400 tokens 675
+    // and 684); norm, linear and 512 tokens of 14 / 2 heads of 64 89 and 64; prompts in a row gain 0.4 us by it.
+    kern<<<(unsigned)blocks, PF_THREADS, C::SMEM, st>>>(
         static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), static_cast<T*>(out), (int)B, (int)Hkv,
         (int)G, (int)Tq, (int)L, lay, scale, causal, split, rows16);
     return check_launch("bi_attn_prefill");

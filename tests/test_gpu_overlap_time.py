@@ -42,6 +42,12 @@ def _decode_behind_a_linear():
     return lambda: (bi.batch_invariant_matmul(bi.batch_invariant_rms_norm(x, None, 1e-5), w), attend())
 
 
+def _prefill_behind_a_linear(T):
+    x, w = _rand(T, 896, dtype=torch.bfloat16), _rand(896, 896, dtype=torch.bfloat16).T
+    q, k, v = _rand(1, 14, T, 64, dtype=torch.bfloat16), *(_rand(1, 2, T, 64, dtype=torch.bfloat16) for _ in range(2))
+    return lambda: (bi.batch_invariant_matmul(x, w), bi.batch_invariant_attention(q, k, v, scale=0.125, mask="causal"))
+
+
 CHAINS = {
     "fp32 few rows": lambda: _linear(2, 2048, 2048),
     "fp32 9 x 4096 -> 4096": lambda: _linear(9, 4096, 4096),
@@ -54,6 +60,7 @@ CHAINS = {
     "bf16 decode attention": lambda: _decode(64, 561, torch.bfloat16),
     "fp32 decode attention": lambda: _decode(64, 561, torch.float32),
     "bf16 decode attention behind a linear": _decode_behind_a_linear,
+    "bf16 prefill attention behind a linear": lambda: _prefill_behind_a_linear(512),
 }
 
 

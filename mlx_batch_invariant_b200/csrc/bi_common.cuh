@@ -35,11 +35,13 @@ inline int fail_cuda(const char* what, cudaError_t e) {
 bool pdl_enabled(bool peers = false);
 
 // Launch `kernel` so that it may begin (block scheduling, barrier and tensor-memory set-up) while the kernel before it
-// on the stream is still draining; the kernel itself waits (ptx::grid_dep_wait) before it touches global memory.
+// on the stream is still draining; the kernel itself waits (ptx::grid_dep_wait) before it reads what earlier kernels wrote or
+// writes anything. (A weight that its caller vouches for is read before that.)
 // Every kernel launched through here MUST execute ptx::grid_dep_wait() in every CTA: completion of this kernel then
 // implies completion of everything before it, which is what the kernel after it relies on.
-// When the kernel after this one may begin is this kernel's to say (ptx::grid_dep_launch): short ones say so at once, matmuls
-// when their last loads are on their way -- CTAs that sit resident from the start took room from them.
+// When the kernel after this one may begin is this kernel's to say (ptx::grid_dep_launch): matmuls say so when their last loads
+// or MMAs are on their way, most others behind their own wait -- CTAs that sit resident from the start take room from
+// them. A kernel that says nothing lets the next one in when its last CTAs leave.
 // Kernels that need an even spread of a few CTAs over the SMs are launched plainly (matmul_simt.cu).
 template <typename... KArgs, typename... Args>
 inline void launch_kernel(bool overlapped, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {

@@ -18,8 +18,7 @@ template <typename T, int QBITS>
 __global__ void __launch_bounds__(DQ_THREADS)
 dequant_kernel(const uint32_t* __restrict__ codes, const T* __restrict__ scales, const T* __restrict__ biases, uint4* __restrict__ out,
                unsigned pieces, unsigned group_shift) {
-    ptx::grid_dep_launch();
-    ptx::grid_dep_wait();
+    ptx::grid_dep_wait_and_launch();
     constexpr int WORDS = QBITS / 4;                          // 32-bit words behind eight codes
     const unsigned i0 = blockIdx.x * (DQ_THREADS * DQ_PIECES) + threadIdx.x;
     uint32_t w[DQ_PIECES][WORDS];

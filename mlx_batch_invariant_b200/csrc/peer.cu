@@ -29,8 +29,7 @@ namespace {
 __global__ void __launch_bounds__(256) push_gather_kernel(const uint4* __restrict__ local, long long rows, int f16, int rank,
                                                           int R, PeerPtrs dst, PeerPtrs flags, unsigned* counters,
                                                           int32_t* status, int wait) {
-    ptx::grid_dep_launch();   // the next kernel of the stream may start its set-up
-    ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
+    ptx::grid_dep_wait_and_launch();
     const long long total = rows * f16;
     const long long pitch = (long long)R * f16;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -50,8 +49,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) push_gather_swiglu_kernel(const T* __restrict__ gu, long long rows, int F, int rank, int R,
                                                                  PeerPtrs dst, PeerPtrs flags, unsigned* counters,
                                                                  int32_t* status, int wait) {
-    ptx::grid_dep_launch();   // the next kernel of the stream may start its set-up
-    ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
+    ptx::grid_dep_wait_and_launch();
     constexpr int V = 16 / (int)sizeof(T);
     const int f16 = F / V;
     const long long total = rows * f16;

@@ -48,6 +48,11 @@ def _prefill_behind_a_linear(T):
     return lambda: (bi.batch_invariant_matmul(x, w), bi.batch_invariant_attention(q, k, v, scale=0.125, mask="causal"))
 
 
+def _norm(rows, dim, dtype, op=bi.batch_invariant_rms_norm):
+    x, w = _rand(rows, dim, dtype=dtype), torch.ones(dim, device="cuda", dtype=dtype)
+    return (lambda: op(x, w, w, 1e-5)) if op is bi.batch_invariant_layer_norm else (lambda: op(x, w, 1e-5))
+
+
 CHAINS = {
     "fp32 few rows": lambda: _linear(2, 2048, 2048),
     "fp32 9 x 4096 -> 4096": lambda: _linear(9, 4096, 4096),
@@ -60,6 +65,9 @@ CHAINS = {
     "bf16 decode attention": lambda: _decode(64, 561, torch.bfloat16),
     "fp32 decode attention": lambda: _decode(64, 561, torch.float32),
     "bf16 decode attention behind a linear": _decode_behind_a_linear,
+    "bf16 norm of 1200 rows": lambda: _norm(1200, 4096, torch.bfloat16),
+    "fp32 norm of 1200 rows": lambda: _norm(1200, 896, torch.float32),
+    "bf16 LayerNorm of 300 rows": lambda: _norm(300, 4096, torch.bfloat16, bi.batch_invariant_layer_norm),
     "bf16 prefill attention behind a linear": lambda: _prefill_behind_a_linear(512),
 }
 

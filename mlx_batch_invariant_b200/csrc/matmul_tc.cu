@@ -438,6 +438,7 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         // The whole warp runs the loop, so that control flow and descriptor arithmetic are warp-uniform (a
         // single-lane branch forces them onto per-thread registers, each instruction waiting for the one
         // before: measured ~200 cycles per MMA); one elected lane issues the MMAs and the commit.
+        if (p.static_w) ptx::grid_dep_wait();                        // no bounded wait counts the time of the kernels in front
         const bool leader = ptx::elect_one();
         constexpr uint32_t FMT = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
         // The MMA's N is the batch rows that were loaded, rounded up to the 16 the instruction wants
@@ -823,6 +824,7 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             if (first.valid()) fetch(first.n0() + row, first.g, sw_n, bw_n);
             else { for (int i = 0; i < 4; ++i) { sw_n[i] = 0u; bw_n[i] = 0u; } }
         }
+        if (p.static_w) ptx::grid_dep_wait();                        // as above: a slot is full when its batch rows are there too
         bool ok = true;
         for (ChunkIter it(p, ub, ue); it.valid() && ok; it.next()) {
             if (it.first_in_group()) {
@@ -899,6 +901,7 @@ tc_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         ChunkIter pf(p, ub, ue);
 #pragma unroll
         for (int i = 0; i < DEPTH; ++i) { fetch(pf, qs[i], qb[i]); pf.next(); }
+        if (p.static_w) ptx::grid_dep_wait();                        // as above: a slot is full when its batch rows are there too
         const uint32_t a_lane = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)p.a_col0;
         bool ok = true;
         ChunkIter it(p, ub, ue);

@@ -85,3 +85,27 @@ def test_behind_copies_memsets_and_joined_streams(captured):
     a, zero, b, c, z = outs
     assert torch.equal(a, want) and torch.equal(b, want) and torch.equal(c, want) and not zero.any()
     assert torch.equal(z, bi.batch_invariant_rms_norm(src, None, 1e-5))
+
+
+@pytest.mark.parametrize("M,path,packed", [(16, "split", 0), (16, "fused", 4), (48, "pair", 0)])
+def test_time_of_the_kernels_in_front_is_no_timeout(M, path, packed):
+    """The norm in front lets the matmul in and then waits out its limit for a flag that nothing raises (2 s): the matmul's own
+    limits begin when that is over."""
+    from mlx_batch_invariant_b200.runner.decoder import KernelBackend
+    (w,), ones = weights((512, 4096), packed), torch.ones(512, device="cuda").bfloat16()
+    x = torch.randn(M, 512, device="cuda").bfloat16()
+    flags, epoch = torch.zeros(8, dtype=torch.int32, device="cuda"), torch.tensor([3], dtype=torch.int32, device="cuda")
+
+    def work(static, **kw):
+        h = KernelBackend().add_rms_norm(x, x, ones, 1e-5, **kw)[1]
+        if packed:
+            return bi.batch_invariant_quantized_matmul(h, *w, group_size=64, bits=packed, path=path, static_weight=static)
+        return bi.batch_invariant_matmul(h, w.T, path=path, static_weight=static)
+
+    want = work(False)
+    _lib.check_device_status()
+    got = work(True, awaiting=(flags.data_ptr(), epoch.data_ptr(), 0, 2))
+    torch.cuda.synchronize()
+    with pytest.raises(_lib.KernelError, match="0x20103"):                # the norm's: 0x20000 | peer 1 << 8 | epoch 3
+        _lib.check_device_status()
+    assert torch.equal(got, want)

@@ -995,13 +995,16 @@ int launch_v(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, cuda
 
 template <typename T, int QBITS, bool TSA>
 int launch_t(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, cudaStream_t st) {
-    if constexpr (QBITS != 0 && !TSA) return launch_v<T, QBITS, TSA, SHAPE_ANY, ROWS_ANY>(mw, mx, p, st);
-    if (p.counters) return launch_v<T, QBITS, TSA, SHAPE_ANY, ROWS_ANY>(mw, mx, p, st);
-    if constexpr (QBITS == 0) {
-        if (p.per_tile) return launch_v<T, QBITS, TSA, SHAPE_RUNS, ROWS_MANY>(mw, mx, p, st);
+    if constexpr (QBITS != 0 && !TSA) {
+        return launch_v<T, QBITS, TSA, SHAPE_ANY, ROWS_ANY>(mw, mx, p, st);
+    } else {
+        if (p.counters) return launch_v<T, QBITS, TSA, SHAPE_ANY, ROWS_ANY>(mw, mx, p, st);
+        if constexpr (QBITS == 0) {
+            if (p.per_tile) return launch_v<T, QBITS, TSA, SHAPE_RUNS, ROWS_MANY>(mw, mx, p, st);
+        }
+        if (p.M <= 8) return p.split ? launch_v<T, QBITS, TSA, SHAPE_SPLIT, ROWS_FEW>(mw, mx, p, st) : launch_v<T, QBITS, TSA, SHAPE_FUSED, ROWS_FEW>(mw, mx, p, st);
+        return p.split ? launch_v<T, QBITS, TSA, SHAPE_SPLIT, ROWS_MANY>(mw, mx, p, st) : launch_v<T, QBITS, TSA, SHAPE_FUSED, ROWS_MANY>(mw, mx, p, st);
     }
-    if (p.M <= 8) return p.split ? launch_v<T, QBITS, TSA, SHAPE_SPLIT, ROWS_FEW>(mw, mx, p, st) : launch_v<T, QBITS, TSA, SHAPE_FUSED, ROWS_FEW>(mw, mx, p, st);
-    return p.split ? launch_v<T, QBITS, TSA, SHAPE_SPLIT, ROWS_MANY>(mw, mx, p, st) : launch_v<T, QBITS, TSA, SHAPE_FUSED, ROWS_MANY>(mw, mx, p, st);
 }
 
 }  // namespace

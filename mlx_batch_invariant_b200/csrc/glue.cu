@@ -111,7 +111,6 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const T* __restrict__ gu, T
 // The same with four 16-bit elements a thread, a block's threads inside one row: 8-byte loads, no 64-bit division. 64 x 14336 in
 // the decoder's step: 5.2 -> 3.9 us (eight a thread 4.3). A row alone has too few threads then: 1.8 us with an element a
 // thread, 2.0 with four; the line lies at the elements that give every SM a block.
-constexpr int64_t SWIGLU_VEC_MIN = 148 * 256 * 4;
 template <typename T>
 __global__ void __launch_bounds__(256) swiglu_vec_kernel(const uint2* __restrict__ gu, uint2* __restrict__ out, int pieces, int blocks_per_row) {
     ptx::grid_dep_wait_and_launch();
@@ -170,7 +169,7 @@ extern "C" int bi_swiglu(const void* gate_up, void* out, int64_t M, int64_t F, i
     if (blocks > 0x7fffffffLL) return fail(BI_ERR_UNSUPPORTED, "bi_swiglu: too large");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int64_t per_row = (F / 4 + 255) / 256;
-    if (dtype != BI_F32 && M * F >= SWIGLU_VEC_MIN && F % 4 == 0 && F < (1LL << 31) && M * per_row < (1LL << 31) && aligned(gate_up, 8) && aligned(out, 8)) {
+    if (dtype != BI_F32 && M * F >= (int64_t)sm_count() * 256 * 4 && F % 4 == 0 && F < (1LL << 31) && M * per_row < (1LL << 31) && aligned(gate_up, 8) && aligned(out, 8)) {
         const uint2* g = static_cast<const uint2*>(gate_up);
         uint2* o = static_cast<uint2*>(out);
         const dim3 grid((unsigned)(M * per_row));

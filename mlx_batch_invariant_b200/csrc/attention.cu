@@ -456,6 +456,7 @@ __global__ void __launch_bounds__(32 * MAXW) decode_warp_stream_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const int32_t* __restrict__ kv_lens,
     float* __restrict__ pm, float* __restrict__ pl, float* __restrict__ pacc, int B, int Hq, int Hkv, int L,
     KvLayout lay, float scale, int split, int nsplit, int nchunk) {
+    ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
     using C = DecWCfg<T, DL>;
     constexpr int D = 32 * DL;
     constexpr int SEGS = C::ROWB / 16;
@@ -1085,8 +1086,6 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
     const T* kp = static_cast<const T*>(k);
     const T* vp = static_cast<const T*>(v);
     dim3 grid((unsigned)blocks), block(32 * warps);
-    // The octet-lane kernels below are launched plainly: several CTAs an SM, less than a wave of them as a rule, which must be
-    // spread evenly (64 x 561 keys of 14 / 2 heads of 64 in a chain of calls: 36 us so, 52 let in beside the merge in front).
     // Streamed kernel when every K/V row starts on a 16-byte boundary (cp.async granularity);
     // otherwise the register-prefetch kernel. Same arithmetic, the choice depends on layout only.
     if constexpr (DL < 8) {
@@ -1162,22 +1161,16 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
             // Below nine warps per SM a warp runs alone on its scheduler most of the time and the 4-warp
             // instantiation (more registers, more loads in flight per warp) is the faster code: measured 55 us
             // against 64 us at 768 streams, 40 against 54 us at 32.
+            // The launch holds the CTAs to that spread: 64 x 561 keys of 14 / 2 heads of 64 in a chain of calls 34.5 us, 36 launched
+            // plainly, 52 let in without regard.
             if (wpc < 9) wpc = 4;
             const size_t smem_w = (size_t)wpc * CW::WARP_BYTES;
             const int64_t blocksw = (streams + wpc - 1) / wpc;
 #define BI_DECW_LAUNCH(MW)                                                                                              \
     do {                                                                                                                \
-        auto kern = decode_warp_stream_kernel<T, DL, MW>;                                                               \
-        static bool attr_set[64] = {false}; /* per instantiation and device: the attribute is per device */            \
-        int dev_ = 0;                                                                                                   \
-        cudaGetDevice(&dev_);                                                                                           \
-        if (dev_ < 0 || dev_ >= 64) dev_ = 0;                                                                           \
-        if (!attr_set[dev_] && MW * CW::WARP_BYTES > 40 * 1024) {                                                       \
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MW * CW::WARP_BYTES); \
-            if (e != cudaSuccess) return fail_cuda("bi_attn_decode smem attr", e);      \
-            attr_set[dev_] = true;                                                                                      \
-        }                                                                                                               \
-        launch_kernel(false, kern, dim3((unsigned)blocksw), dim3(32 * wpc), smem_w, st, qp, kp, vp, kv_lens, pm, pl, pacc, (int)B, (int)Hq, (int)Hkv, \
+        constexpr auto kern = decode_warp_stream_kernel<T, DL, MW>;                                                     \
+        if (!opt_in_smem<kern>()) return fail_cuda("bi_attn_decode smem attr", cudaErrorInvalidValue);                  \
+        launch_overlapped(kern, dim3((unsigned)blocksw), dim3(32 * wpc), spread_smem<kern>(blocksw, smem_w), st, qp, kp, vp, kv_lens, pm, pl, pacc, (int)B, (int)Hq, (int)Hkv, \
                                                           (int)L, lay, scale, split, nsplit, nchunk4);                  \
     } while (0)
             if (wpc <= 4) BI_DECW_LAUNCH(4);
@@ -1199,6 +1192,7 @@ int launch_decode(const void* q, const void* k, const void* v, void* out, const 
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES); \
             if (e != cudaSuccess) return fail_cuda("bi_attn_decode smem attr", e); \
         }                                                                                                        \
+        /* plainly: many CTAs, several an SM */                                                                   \
         launch_kernel(false, kern, dim3((unsigned)blocks2), dim3(32 * DEC2_WARPS), C::SMEM_BYTES, st, qp, kp, vp, kv_lens, pm, pl, pacc, (int)B, \
                                                                           (int)Hq, (int)Hkv, (int)L, lay, scale, split, nsplit, nchunk); \
     } while (0)

@@ -244,6 +244,7 @@ __global__ void __launch_bounds__(PF_THREADS, TQ == 4 && (DL == 2 || DL == 4) &&
     float* const ms = reinterpret_cast<float*>(sm + C::MOFF);
     int* const ns = reinterpret_cast<int*>(sm + C::NOFF);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    ptx::grid_dep_wait();     // everything before this kernel has completed and is visible
 
     const RowBlock block(B, Hkv, G, Tq, QB);
     const long long R = block.R, r0 = block.r0;
@@ -470,20 +471,14 @@ int launch_prefill_tq(const void* q, const void* k, const void* v, void* out, in
     if (blocks > 0x7fffffffLL) return fail(BI_ERR_UNSUPPORTED, "bi_attn_prefill: grid too large");
     const int64_t per16 = 16 / (int64_t)sizeof(T);
     const int rows16 = aligned(k, 16) && aligned(v, 16) && aligned(out, 16) && lay.sb % per16 == 0 && lay.sh % per16 == 0 && lay.sl % per16 == 0;
-    auto kern = prefill_kernel<T, DL, TQ>;
-    static bool attr_set[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) dev = 0;
-    if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-        if (e != cudaSuccess) return fail_cuda("bi_attn_prefill smem attr", e);
-        attr_set[dev] = true;
-    }
-    // Plainly: two or three CTAs an SM, which lie unevenly when they are let in beside a running kernel, for long prompts too, whose
-    // blocks differ in keys. Linear and attention of 512 tokens, 32 / 8 heads of 128: 143 us so, 119 plainly (and 1400 tokens 675
-    // and 684); norm, linear and 512 tokens of 14 / 2 heads of 64 89 and 64; prompts in a row gain 0.4 us by it.
-    kern<<<(unsigned)blocks, PF_THREADS, C::SMEM, st>>>(
+    constexpr auto kern = prefill_kernel<T, DL, TQ>;
+    if (!opt_in_smem<kern>()) return fail_cuda("bi_attn_prefill smem attr", cudaErrorInvalidValue);
+    // More CTAs than SMs are launched plainly: two or three lie on an SM, unevenly when they are let in beside a running kernel, in
+    // long prompts too, whose blocks differ in keys. Linear and attention of 512 tokens, 32 / 8 heads of 128: 143 us so, 120 plainly
+    // (1400 tokens 675 and 683); norm, linear and 512 tokens of 14 / 2 heads of 64 89 and 63, held to two an SM 75. Held to one,
+    // 100 tokens of 32 / 8 heads in a row take 18.1 us, 18.5 plainly (eagerly 18.9 and 21.0).
+    const bool overlapped = pdl_enabled() && blocks <= sm_count();
+    launch_kernel(overlapped, kern, dim3((unsigned)blocks), dim3(PF_THREADS), overlapped ? spread_smem<kern>(blocks, C::SMEM) : C::SMEM, st,
         static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), static_cast<T*>(out), (int)B, (int)Hkv,
         (int)G, (int)Tq, (int)L, lay, scale, causal, split, rows16);
     return check_launch("bi_attn_prefill");

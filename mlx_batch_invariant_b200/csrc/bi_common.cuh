@@ -2,6 +2,8 @@
 // error message, and launch checking.
 #pragma once
 #include <cuda_runtime.h>
+#include <algorithm>
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdint>
@@ -42,7 +44,7 @@ bool pdl_enabled(bool peers = false);
 // When the kernel after this one may begin is this kernel's to say (ptx::grid_dep_launch): matmuls say so when their last loads
 // or MMAs are on their way, most others behind their own wait -- CTAs that sit resident from the start take room from
 // them. A kernel that says nothing lets the next one in when its last CTAs leave.
-// Kernels that need an even spread of a few CTAs over the SMs are launched plainly (matmul_simt.cu).
+// Kernels of several CTAs an SM need an even spread of them (spread_smem below) or are launched plainly.
 template <typename... KArgs, typename... Args>
 inline void launch_kernel(bool overlapped, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
@@ -82,6 +84,35 @@ inline int sm_count() {
     if (dev < 0 || dev >= 64) dev = 0;
     if (!cached[dev]) cudaDeviceGetAttribute(&cached[dev], cudaDevAttrMultiProcessorCount, dev);
     return cached[dev] > 0 ? cached[dev] : 148;
+}
+
+// An SM's shared memory, of which every CTA takes 1 KB besides its own, and what a CTA may have.
+constexpr size_t SM_SMEM = 228 << 10, CTA_SMEM = 227 << 10;
+
+// The dynamic shared memory that a launch of KERNEL may ask for; the opt-in to it is made once per device. 0: refused.
+template <auto KERNEL> size_t opt_in_smem() {
+    static std::atomic<int> cached[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    int most = cached[dev].load(std::memory_order_relaxed);
+    if (!most) {
+        cudaFuncAttributes a;
+        cudaError_t e = cudaFuncGetAttributes(&a, KERNEL);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, most = (int)(CTA_SMEM - a.sharedSizeBytes));
+        if (e != cudaSuccess) { cudaGetLastError(); return 0; }                // not the next launch's error
+        cached[dev].store(most, std::memory_order_relaxed);
+    }
+    return (size_t)most;
+}
+
+// CTAs that are let in beside a running kernel land where room comes free first, four on some SMs and none on others; a grid of
+// less than a wave then takes as long as the fullest SM. A launch that asks for this much dynamic shared memory (`smem` is what
+// KERNEL uses) leaves an SM no room for more CTAs than an even spread gives it.
+template <auto KERNEL> size_t spread_smem(int64_t ctas, size_t smem) {
+    const size_t fixed = CTA_SMEM - opt_in_smem<KERNEL>(), per_sm = (size_t)((ctas + sm_count() - 1) / sm_count());
+    const size_t share = SM_SMEM / (per_sm + 1);                     // one CTA more would need more than all
+    return share > fixed ? std::max(smem, (share - fixed + 127) / 128 * 128) : smem;
 }
 
 // Canonical constants of the arithmetic contract.

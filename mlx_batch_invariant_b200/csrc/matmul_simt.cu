@@ -425,14 +425,29 @@ struct SimtArgs {
     cudaStream_t st;
 };
 
-// Less than a wave of CTAs is launched plainly. Let in beside a running kernel, CTAs land where room comes free first, four on
-// some SMs and none on others, and a grid that never fills them takes as long as the fullest SM. fp32 128 x 2048 -> 2048 in a
-// chain of calls 52.5 us so, 31 plainly; 64 x 2048 -> 2048 behind a 16-bit linear 60 and 26. Grids of a wave up gain a launch's
-// latency: 100 x 4096 -> 4096 97.1 -> 93.0 us a call.
-template <typename Kernel> bool overlaps(Kernel kernel, const dim3& grid, int threads, size_t smem) {
+// How a grid lies on the SMs decides its time where it is less than a wave (spread_smem). Up to a CTA an SM it is held to that;
+// of two CTAs an SM up the fullest ones were slower than an idle machine's spread, so these are launched plainly, and grids of
+// a wave up again beside the kernel in front; so are packed weights, whose codes come through the L1 that the hold takes from (64 x
+// 896 -> 4864, 4 bits 70.0 us, held 71.6). us a call in chains, let in without regard / plainly / so: fp32 128 x 2048 -> 2048
+// 52.5 / 31 / 30.4, 9 x 2048 -> 2048 19.5 / 14.7 / 13.8, 64 x 2048 -> 2048 behind a 16-bit linear 60 / 26 / 23.8; eagerly 100 x 4096 ->
+// 4096 93 / 97 / 93.
+template <auto KERNEL, bool HOLD, typename... Args>
+void launch_simt(dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    const int64_t ctas = (int64_t)grid.x * grid.y * grid.z;
+    bool overlapped = pdl_enabled();
     int resident = 0;
-    return pdl_enabled() && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, threads, smem) == cudaSuccess &&
-           (int64_t)grid.x * grid.y * grid.z >= (int64_t)resident * sm_count();
+    if (HOLD && overlapped && ctas <= sm_count()) smem = spread_smem<KERNEL>(ctas, smem);
+    else if (overlapped) overlapped = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, KERNEL, threads, smem) == cudaSuccess && ctas >= (int64_t)resident * sm_count();
+    launch_kernel(overlapped, KERNEL, grid, dim3(threads), smem, st, args...);
+}
+
+template <int TM, bool SPLIT>
+int simt_columns(dim3 grid, size_t smem, const SimtArgs& p) {
+    constexpr auto kern = simt_stream_kernel<TM, SPLIT>;
+    if (!opt_in_smem<kern>()) return fail_cuda("matmul (cuda-core path) smem attr", cudaErrorInvalidValue);
+    launch_simt<kern, true>(grid, STREAM_N, smem, p.st, static_cast<const float*>(p.a), static_cast<const float*>(p.b), p.qa, static_cast<float*>(p.dst), (int)p.M,
+                      (int)p.N, (int)p.K, p.a_sm, p.b_sn);
+    return check_launch("matmul (cuda-core path)");
 }
 
 template <int TM>
@@ -441,12 +456,13 @@ int simt_stream(const SimtArgs& p) {
     if (p.split && G > 65535) return fail(BI_ERR_UNSUPPORTED, "matmul (cuda-core path): K=%lld too large", (long long)p.K);
     dim3 grid((unsigned)((p.N + STREAM_N - 1) / STREAM_N), 1, p.split ? (unsigned)G : 1u);
     constexpr size_t smem = (size_t)STREAM_STAGES * (TM + STREAM_N) * STREAM_PITCH * sizeof(float);
-    auto kern = p.split ? simt_stream_kernel<TM, true> : simt_stream_kernel<TM, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return fail_cuda("matmul (cuda-core path) smem attr", e);
-    launch_kernel(overlaps(kern, grid, STREAM_N, smem), kern, grid, dim3(STREAM_N), smem, p.st, static_cast<const float*>(p.a),
-                  static_cast<const float*>(p.b), p.qa, static_cast<float*>(p.dst), (int)p.M, (int)p.N, (int)p.K, p.a_sm, p.b_sn);
-    return check_launch("matmul (cuda-core path)");
+    return p.split ? simt_columns<TM, true>(grid, smem, p) : simt_columns<TM, false>(grid, smem, p);
+}
+
+template <typename T, int TM, int TN, int MG, int NL, bool SPLIT, bool QUANT, bool VEC>
+void simt_tiles(dim3 grid, const SimtArgs& p) {
+    launch_simt<simt_matmul_kernel<T, TM, TN, MG, NL, SPLIT, QUANT, VEC>, !QUANT>(grid, MG * NL, 0, p.st, static_cast<const T*>(p.a), static_cast<const T*>(p.b),
+                                                                                  p.qa, p.dst, (int)p.M, (int)p.N, (int)p.K, p.a_sm, p.a_sk, p.b_sk, p.b_sn);
 }
 
 template <typename T, bool QUANT, bool VEC, int I>
@@ -458,9 +474,8 @@ int simt_launch(int tile, const SimtArgs& p) {
         const int64_t G = (p.K + GROUP_K - 1) / GROUP_K, gy = (p.M + bm - 1) / bm;
         if (gy > 65535 || (p.split && G > 65535)) return fail(BI_ERR_UNSUPPORTED, "matmul (cuda-core path): M=%lld K=%lld too large", (long long)p.M, (long long)p.K);
         dim3 grid((unsigned)((p.N + bn - 1) / bn), (unsigned)gy, p.split ? (unsigned)G : 1u);
-        auto kern = p.split ? simt_matmul_kernel<T, t.tm, t.tn, t.mg, t.nl, true, QUANT, VEC> : simt_matmul_kernel<T, t.tm, t.tn, t.mg, t.nl, false, QUANT, VEC>;
-        launch_kernel(overlaps(kern, grid, t.mg * t.nl, 0), kern, grid, dim3(t.mg * t.nl), 0, p.st,
-                      static_cast<const T*>(p.a), static_cast<const T*>(p.b), p.qa, p.dst, (int)p.M, (int)p.N, (int)p.K, p.a_sm, p.a_sk, p.b_sk, p.b_sn);
+        if (p.split) simt_tiles<T, t.tm, t.tn, t.mg, t.nl, true, QUANT, VEC>(grid, p);
+        else simt_tiles<T, t.tm, t.tn, t.mg, t.nl, false, QUANT, VEC>(grid, p);
         return check_launch("matmul (cuda-core path)");
     }
     return fail(BI_ERR_UNSUPPORTED, "matmul (cuda-core path): no tile %d", tile);

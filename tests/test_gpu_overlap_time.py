@@ -69,6 +69,8 @@ CHAINS = {
     "fp32 norm of 1200 rows": lambda: _norm(1200, 896, torch.float32),
     "bf16 LayerNorm of 300 rows": lambda: _norm(300, 4096, torch.bfloat16, bi.batch_invariant_layer_norm),
     "bf16 prefill attention behind a linear": lambda: _prefill_behind_a_linear(512),
+    "short bf16 prefill attention behind a linear": lambda: _prefill_behind_a_linear(100),
+    "fp32 16 x 2048 -> 2048": lambda: _linear(16, 2048, 2048),
 }
 
 

@@ -3,7 +3,7 @@ on the way (world of one: the destination is local memory), the *_awaiting entry
 flags already raised they give the bits of the plain entry points; with a flag that nothing raises the bounded
 wait runs out, the status word says so, and the context stays usable --, the *_push entry points (matmul,
 quantized matmul, decode attention) as one rank of a world of two whose destinations both live on this GPU, and
-the kernels launched with programmatic dependent launch. (The exchange between GPUs itself is covered by
+chains of kernels that start while the one before finishes. (The exchange between GPUs itself is covered by
 tests/test_gpu_multi.py.)"""
 
 import ctypes
@@ -135,38 +135,50 @@ def test_ops_that_push_their_own_output(bi):
     bi.check_device_status()
 
 
-def test_programmatic_dependent_launch_gives_the_same_bits(bi, monkeypatch):
-    """BI_PDL=1 launches the kernels so that each may start while the one before it drains (every kernel waits
-    for its predecessors before it touches global memory). A chain of dependent ops, eagerly and from a replayed
-    CUDA graph, must give the bits of the plain launches."""
+@pytest.mark.parametrize("rows", [16, 80])        # fewer than 64 rows let the next kernel in ahead of their own wait
+def test_overlapped_launches_give_the_bits_of_plain_ones(bi, monkeypatch, rows):
+    """Kernels of one GPU are launched so that each may start while the one before it drains (every kernel waits for its
+    predecessors before it reads what they wrote, or writes). A chain of dependent ops, eagerly and from a replayed CUDA graph,
+    must give the bits of plain launches."""
     from mlx_batch_invariant_b200.runner.decoder import KernelBackend
     dt = torch.bfloat16
     g = torch.Generator().manual_seed(4)
-    x = torch.randn(16, 1024, generator=g).to(dt).cuda()
+    x = torch.randn(rows, 1024, generator=g).to(dt).cuda()
     w1 = (torch.randn(1024, 1024, generator=g) / 32).to(dt).cuda()
-    w2 = (torch.randn(2048, 1024, generator=g) / 32).to(dt).cuda()
+    wqkv = (torch.randn(1536, 1024, generator=g) / 32).to(dt).cuda()
+    wup = (torch.randn(4096, 1024, generator=g) / 32).to(dt).cuda()
+    wdown = (torch.randn(1024, 2048, generator=g) / 45).to(dt).cuda()
     nw = torch.ones(1024, dtype=dt, device="cuda")
-    q = torch.randn(16, 8, 1, 128, generator=g).to(dt).cuda()
-    k = torch.randn(16, 2, 300, 128, generator=g).to(dt).cuda()
-    v = torch.randn(16, 2, 300, 128, generator=g).to(dt).cuda()
+    k = torch.randn(rows, 2, 300, 128, generator=g).to(dt).cuda()
+    v = torch.randn(rows, 2, 300, 128, generator=g).to(dt).cuda()
+    cos, sin = (torch.randn(rows, 128, generator=g).cuda() for _ in range(2))
+    pos0 = torch.zeros(1, dtype=torch.int64, device="cuda")
+    kc, vc = (torch.empty(1, 2, rows, 128, dtype=dt, device="cuda") for _ in range(2))
     ops = KernelBackend()
 
     def chain():
         h = bi.batch_invariant_matmul(x, w1.T, path="split")
         s, h = ops.add_rms_norm(x, h, nw, 1e-5)
-        h = ops.swiglu(bi.batch_invariant_matmul(h, w2.T))
-        a = bi.batch_invariant_decode_attention(q, k, v, scale=0.09).reshape(16, 1024)
-        return bi.batch_invariant_matmul(h + a, w1.T, path="fused"), s
+        q = ops.rope_append(bi.batch_invariant_matmul(h, wqkv.T, static_weight=True), cos, sin, pos0, 1, rows, 8, 2, 128, kc, vc)
+        h = bi.batch_invariant_attention(q, kc, vc, scale=0.09, mask="causal").reshape(rows, 1024)
+        h = bi.batch_invariant_layer_norm(bi.batch_invariant_matmul(h, w1.T, static_weight=True), nw, nw, 1e-5)
+        h = ops.swiglu(bi.batch_invariant_matmul(h, wup.T, static_weight=True))                    # 80 rows: four elements a thread
+        h = bi.batch_invariant_matmul(h, wdown.T, path="fused", static_weight=True)
+        h = bi.batch_invariant_decode_attention(h.reshape(rows, 8, 1, 128), k, v, scale=0.09).reshape(rows, 1024)
+        f = bi.batch_invariant_rms_norm(h.float(), nw.float(), 1e-5)
+        return bi.batch_invariant_matmul(h, w1.T, static_weight=True), s, q, kc.clone(), vc.clone(), bi.batch_invariant_matmul(f, w1.float().T)
 
+    monkeypatch.setenv("BI_PDL", "0")
     want = [R.bits_of(t) for t in chain()]
-    monkeypatch.setenv("BI_PDL", "1")
-    assert [R.bits_of(t) for t in chain()] == want
-    torch.cuda.synchronize()
+    monkeypatch.delenv("BI_PDL")
+    for _ in range(3):
+        assert [R.bits_of(t) for t in chain()] == want
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         outs = chain()
     for _ in range(3):
+        for t in (*outs, kc, vc):
+            t.zero_()
         graph.replay()
-    torch.cuda.synchronize()
-    assert [R.bits_of(t) for t in outs] == want
+        assert [R.bits_of(t) for t in outs] == want
     bi.check_device_status()

@@ -676,14 +676,14 @@ __device__ __forceinline__ void kl_node(const uint8_t* krow, const uint8_t* qs, 
 // The work items of sequences that bring lengths: item i of the launch is (sequence, split, kv head, chunk of query heads),
 // the full splits of all sequences first, then the partly filled ones. Only splits that hold keys are counted, from the
 // lengths in device memory: every warp sums them once, 32 sequences at a time, lane g keeping the items up to and with group
-// g; an item's group is then a vote over the lanes, its sequence a scan over the group's lengths, which were fetched while
-// the item before was worked on.
+// g; an item's group is then a vote over the lanes, its sequence a scan over the group's lengths (up to 32 sequences stay in a
+// register, of more they are fetched when the item is looked up).
 constexpr int KL_LISTED_MAX = 1024;                        // most sequences: a group per lane
 struct KLItems {
     const int32_t* kv_lens;
     int B, L, split, per_seq;                              // per_seq: items of one split of a sequence (kv heads x chunks)
     int full, part, nfull, nall;                           // inclusive counts of this lane's group; all full ones; all (an item has a partial in the workspace)
-    int len;                                               // of this lane's sequence in the next item's group
+    int len;                                               // of this lane's sequence in the group looked up last (at first: the first group)
     __device__ __forceinline__ int fetch(int g) const {
         const int b = g * 32 + (int)(threadIdx.x & 31);
         return b < B ? max(0, min(kv_lens[b], L)) : 0;
@@ -720,8 +720,7 @@ struct KLItems {
         }
         nall += nfull;
     }
-    // item `i` of nall, the one asked for in the call before (or at the start): sequence, split, index among the split's
-    // per_seq items, keys. `next` is what the next call asks for.
+    // item `i` of nall: sequence, split, index among the split's per_seq items, keys
     __device__ __forceinline__ void find(int i, int& b, int& sp, int& sub, int& nk) {
         const bool ph = i >= nfull;
         int g = 0, r = i - (ph ? nfull : 0);

@@ -41,7 +41,7 @@ TcShape tc_one_sm_shape(int64_t M, int64_t N, int64_t K, bool quant) {
     return sh;
 }
 // Split, dense: the same number of CTAs for every tile, the first of which folds its run of groups itself, so that a tile
-// writes and the fold reads G - run + 1 partials: 64 rows of 14336 -> 4096, 43 of 56, 35.0 -> 33.5 us a call. For 33 to 64 rows
+// writes and the fold reads G - run + 1 partials: 64 rows of 14336 -> 4096, 43 of 56, 35.2 -> 32.4 us a call. For 33 to 64 rows
 // and runs of eight groups up: shorter ones give nothing (64 of 4096 -> 4096, run of four: 14.4 us either way), nor do fewer
 // rows, whose partials are small (16 of 14336 -> 4096: 27.9 and 27.8).
 void split_runs(int64_t M, int64_t N, int64_t K, TcShape* sh) {

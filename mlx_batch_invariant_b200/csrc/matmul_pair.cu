@@ -82,7 +82,7 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
 // wait for a fence of the whole memory system: 0.5 - 1 us on the way from a drained accumulator to the next group's
 // MMAs (fp16 1900 x 4096 -> 14336: 213 us with it, 178 without; bf16 1024 x 14336 -> 4096 at bm = 128: 166 and 112).
 __device__ __forceinline__ void arrive_cluster(uint32_t bar) {
-        asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // Boxes of this GPU's memory into this CTA's shared memory; completion is signalled on `bar`, which may be the peer's.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap, int c0, int c1, uint32_t bar) {

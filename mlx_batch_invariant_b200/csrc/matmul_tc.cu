@@ -137,7 +137,7 @@ struct Params {
 // epilogue before it reads an accumulator -- waits on the same barrier done[c % 8].
 // What of the kernel a launch needs. A decoder's step goes through some 390 kernels, and each begins with its instructions in
 // no cache: code that a launch does not reach still lies between what it does, and the registers of the widest loop are
-// everyone's (168; now 45 - 112). Decoder step, one kernel for all -> one for each: 64 / 16 / 1 sequences 5539 / 4308 / 3559 ->
+// everyone's (168; now 45 - 128, with runs 154; the in-kernel fold still 168). Decoder step, one kernel for all -> one for each: 64 / 16 / 1 sequences 5539 / 4308 / 3559 ->
 // 5383 / 4067 / 3514 us, 4-bit weights 7115 / 4645 / 3830 -> 6392 / 4349 / 3567. ANY decides at run time: the in-kernel fold, and
 // packed weights of more than 64 rows.
 enum { SHAPE_ANY, SHAPE_FUSED, SHAPE_SPLIT, SHAPE_RUNS };

@@ -62,8 +62,8 @@ def batch_invariant_matmul(a, b, *, path: str = "auto", batch_tile: int | None =
     ``rope`` (the arguments of ``bi_rope_append`` after ``qkv``, up to ``capacity``): the product is a decoder's qkv
     projection; the fold kernel rotates q and k and appends k and v to the cache itself (``bi_matmul_rope``);
     nothing is returned.
-    ``static_weight``: nothing that is still running on the stream writes ``b`` (a model's weights; not the result of the call
-    before): the kernel starts on it while the kernels in front of it finish (``BI_MATMUL_STATIC_WEIGHT``).
+    ``static_weight``: nothing that is still running on the stream writes ``b`` (a model's weights; not the result of one of the
+    calls before): the kernel starts on it while the kernels in front of it finish (``BI_MATMUL_STATIC_WEIGHT``).
     """
     at, foreign = adopt(a)
     bt, _ = adopt(b)

@@ -106,6 +106,20 @@ template <auto KERNEL> size_t opt_in_smem() {
     return (size_t)most;
 }
 
+// CTAs of KERNEL that an SM holds, which is always launched with the same threads and shared memory; asked once per device.
+template <auto KERNEL> int resident_ctas(int threads, size_t smem) {
+    static std::atomic<int> cached[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    int n = cached[dev].load(std::memory_order_relaxed);
+    if (!n) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, KERNEL, threads, smem) != cudaSuccess || n < 1) { cudaGetLastError(); return 32; }
+        cached[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 // CTAs that are let in beside a running kernel land where room comes free first, four on some SMs and none on others; a grid of
 // less than a wave then takes as long as the fullest SM. A launch that asks for this much dynamic shared memory (`smem` is what
 // KERNEL uses) leaves an SM no room for more CTAs than an even spread gives it.

@@ -435,9 +435,8 @@ template <auto KERNEL, bool HOLD, typename... Args>
 void launch_simt(dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
     const int64_t ctas = (int64_t)grid.x * grid.y * grid.z;
     bool overlapped = pdl_enabled();
-    int resident = 0;
     if (HOLD && overlapped && ctas <= sm_count()) smem = spread_smem<KERNEL>(ctas, smem);
-    else if (overlapped) overlapped = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, KERNEL, threads, smem) == cudaSuccess && ctas >= (int64_t)resident * sm_count();
+    else if (overlapped) overlapped = ctas >= (int64_t)resident_ctas<KERNEL>(threads, smem) * sm_count();
     launch_kernel(overlapped, KERNEL, grid, dim3(threads), smem, st, args...);
 }
 

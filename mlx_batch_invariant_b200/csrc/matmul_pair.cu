@@ -176,6 +176,7 @@ pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     auto unit_m0 = [&](int u) { return (u % p.m_tiles) * p.bm; };
 
     if (warp < EPI0) regs_dec<REGS_ISSUE>();
+    if (warp == 1 && p.static_w) ptx::grid_dep_wait();               // no bounded wait counts the time of the kernels in front
     if (warp == 0) {
         // ------------------------------------------------------------ TMA: weight and activation tiles
         const bool leader = ptx::elect_one();
@@ -257,7 +258,6 @@ pair_matmul_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer (first CTA of the pair)
         if (rank == 0) {
-            if (p.static_w) ptx::grid_dep_wait();                    // no bounded wait counts the time of the kernels in front
             const bool leader = ptx::elect_one();
             constexpr uint32_t FMT = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
             const uint32_t IDESC = (1u << 4) | (FMT << 7) | (FMT << 10) | ((uint32_t)(p.bm >> 3) << 17) |
